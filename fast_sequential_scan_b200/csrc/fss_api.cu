@@ -250,6 +250,13 @@ FSS_API size_t fss_workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype) {
     return workspace_total(a > c ? a : c);
 }
 
+FSS_API size_t fss_gated_backward_workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype) {
+    if (B <= 0 || T <= 0 || D <= 0) return workspace_total(0);
+    const size_t packets = lookback::workspace_bytes(B, T, D, dtype, lookback::Kind<true, true>::kTc);
+    const size_t floats = (size_t)D * 2 * sizeof(float);
+    return workspace_total(packets > floats ? packets : floats);
+}
+
 FSS_API int fss_workspace_init(void *workspace, size_t bytes, void *stream) {
     if (!workspace) return FSS_E_NULL;
     FSS_CUDA(cudaMemsetAsync(workspace, 0, bytes, (cudaStream_t)stream), "cudaMemsetAsync(workspace)");
@@ -770,4 +777,42 @@ FSS_API int fss_gates_backward(const fss_scan_ctx *ctx, int dtype, int64_t B, in
         return chunked::vector_ok<bf16>(D, {r, i, x, grad_alpha, grad_beta, grad_r, grad_i, grad_x}) ? FSS_GB(bf16, 8) : FSS_GB(bf16, 1);
     return chunked::vector_ok<float>(D, {r, i, x, grad_alpha, grad_beta, grad_r, grad_i, grad_x}) ? FSS_GB(float, 4) : FSS_GB(float, 1);
 #undef FSS_GB
+}
+
+FSS_API int fss_scan_backward_gated(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t T, int64_t D,
+                                    const fss_view *r, const fss_view *i, const fss_view *x, const float *lambda,
+                                    const fss_view *h, const fss_view *grad_out, const fss_view *grad_r,
+                                    const fss_view *grad_i, const fss_view *grad_x, float *grad_lambda) {
+    int rc;
+    if ((rc = check_ctx(ctx))) return rc;
+    if ((rc = check_shape(dtype, B, T, D))) return rc;
+    if (B == 0 || T == 0 || D == 0) return FSS_OK;
+    if (!lambda || !grad_lambda) return FSS_E_NULL;
+    const fss_view *in[] = {r, i, x, h, grad_out}, *out[] = {grad_r, grad_i, grad_x};
+    for (const fss_view *v : in)
+        if ((rc = check_view(v, B, T, D))) return rc;
+    for (const fss_view *v : out)
+        if ((rc = check_view(v, B, T, D))) return rc;
+    for (const fss_view *o : out)
+        for (const fss_view *v : in)
+            if (same_start(o, v)) return FSS_E_ALIAS;
+    if (same_start(grad_r, grad_i) || same_start(grad_r, grad_x) || same_start(grad_i, grad_x)) return FSS_E_ALIAS;
+    if (ctx->flags & FSS_FLAG_CONTINUATION) return FSS_E_ARGS;
+    // the limit of fss_gates_backward, which does this work for other layouts: alignment alone does not
+    // decide whether a problem is accepted
+    if (!gate_grid_ok(B, T)) return FSS_E_SHAPE;
+    if (ctx->algo == FSS_ALGO_CHUNKED || !aligned16(grad_lambda)) return FSS_E_LAYOUT;
+    const bool ok = dtype == FSS_DTYPE_BF16
+                        ? lookback::layout_ok<bf16>(B, T, D, {r, i, x, h, grad_out, grad_r, grad_i, grad_x})
+                        : lookback::layout_ok<float>(B, T, D, {r, i, x, h, grad_out, grad_r, grad_i, grad_x});
+    if (!ok) return FSS_E_LAYOUT;
+    if (!ctx->workspace || !aligned16(ctx->workspace) ||
+        ctx->workspace_bytes < fss_gated_backward_workspace_bytes(B, T, D, dtype))
+        return FSS_E_WORKSPACE;
+    DeviceGuard guard(ctx->device);
+    if (guard.error) return guard.error;
+    const WsPlan ws = plan_workspace(ctx->workspace, ctx->workspace_bytes);
+    return dtype == FSS_DTYPE_BF16
+               ? lookback::backward_gated<bf16>(ctx, ws, B, T, D, r, i, x, lambda, h, grad_out, grad_r, grad_i, grad_x, grad_lambda, &g_cuda_error)
+               : lookback::backward_gated<float>(ctx, ws, B, T, D, r, i, x, lambda, h, grad_out, grad_r, grad_i, grad_x, grad_lambda, &g_cuda_error);
 }

@@ -111,6 +111,33 @@ template <typename T> struct VecWidth;
 template <> struct VecWidth<bf16> { static constexpr int value = 8; };
 template <> struct VecWidth<float> { static constexpr int value = 4; };
 
+// ------------------------------------------------------------------ packed fp32 pairs
+// Two fp32 values in one 64-bit register: the packed instructions round each half exactly as the
+// scalar ones do and take one issue slot for both.
+struct Two { unsigned long long v; };
+__device__ __forceinline__ Two two(float x, float y) {
+    Two r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ Two splat(float x) { return two(x, x); }
+__device__ __forceinline__ void split(const Two &t, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(t.v)); }
+__device__ __forceinline__ Two fma2(const Two &a, const Two &b, const Two &c) {
+    Two r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Two mul2(const Two &a, const Two &b) {
+    Two r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Two add2(const Two &a, const Two &b) {
+    Two r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
 // ------------------------------------------------------------------ status word
 // Written only when a bounded wait gives up; works for device memory and for pinned host memory.
 __device__ __forceinline__ void report_status(int32_t *status, int32_t code) {

@@ -21,6 +21,13 @@ template <> struct Gate<bf16> {
         asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * z));
         return fmaf(0.5f, t, 0.5f);
     }
+    static __device__ __forceinline__ Two sigmoid(const Two &z) {      // the same roundings, two at a time
+        float x, y;
+        split(mul2(splat(0.5f), z), x, y);
+        asm("tanh.approx.f32 %0, %0;" : "+f"(x));
+        asm("tanh.approx.f32 %0, %0;" : "+f"(y));
+        return fma2(splat(0.5f), two(x, y), splat(0.5f));
+    }
     static __device__ __forceinline__ float prescale(float c) { return c * 1.4426950408889634f; }   // exp(z) = 2^(z log2 e)
     static __device__ __forceinline__ float exp_scaled(float z) {
         float r;
@@ -32,6 +39,11 @@ template <> struct Gate<bf16> {
         asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(z));
         return r;
     }
+    static __device__ __forceinline__ float rroot(float z) {
+        float r;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
+        return r;
+    }
 };
 template <> struct Gate<float> {
     // (tanh.approx, good to 2^-11, is not accurate enough for fp32 I/O)
@@ -40,6 +52,16 @@ template <> struct Gate<float> {
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * z));
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
         return r;
+    }
+    static __device__ __forceinline__ Two sigmoid(const Two &z) {      // the same roundings, two at a time
+        float x, y;
+        split(mul2(splat(-1.4426950408889634f), z), x, y);
+        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x));
+        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(y));
+        split(add2(splat(1.0f), two(x, y)), x, y);
+        asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(x));
+        asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(y));
+        return two(x, y);
     }
     static __device__ __forceinline__ float prescale(float c) { return c * 1.4426950408889634f; }
     static __device__ __forceinline__ float exp_scaled(float z) {
@@ -52,7 +74,18 @@ template <> struct Gate<float> {
         asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
         return r;
     }
+    static __device__ __forceinline__ float rroot(float z) {
+        float r;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
+        return r;
+    }
 };
+// alpha of a pair, given the pair of sigmoids, exactly as exp_scaled(scale * sigmoid) gives it
+template <typename T> __device__ __forceinline__ Two gate_alpha(const Two &scale, const Two &sigmoid) {
+    float x, y;
+    split(mul2(scale, sigmoid), x, y);
+    return two(Gate<T>::exp_scaled(x), Gate<T>::exp_scaled(y));
+}
 __device__ __forceinline__ float gate_scale(float lambda) {      // -8 * softplus(lambda)
     return -8.0f * (lambda > 20.0f ? lambda : log1pf(expf(lambda)));
 }
@@ -71,6 +104,16 @@ template <typename T>
 __global__ void prescale(const float *__restrict__ lambda, float *__restrict__ scales, int64_t D) {
     const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (d < D) scales[d] = Gate<T>::prescale(gate_scale(lambda[d]));
+}
+
+// The same for the fused backward: -8 * softplus(lambda) and its slope; dlambda starts at zero.
+__global__ void backward_tables(const float *__restrict__ lambda, float *__restrict__ scales, float *__restrict__ slopes,
+                                float *__restrict__ dlambda, int64_t D) {
+    const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= D) return;
+    scales[d] = gate_scale(lambda[d]);
+    slopes[d] = gate_scale_slope(lambda[d]);
+    dlambda[d] = 0.0f;
 }
 
 // alpha (and beta when asked) as the fused forward scan computes them, rounded to T.

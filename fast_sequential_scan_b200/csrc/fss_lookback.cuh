@@ -3,6 +3,7 @@
 //
 // Work unit: a 16 KiB tile per tensor of one batch row: 64 rows x 256 bytes of channels, or
 // 128 x 128 / 256 x 64 when the problem has too few columns to fill the GPU otherwise (kSp = 2 / 4).
+// (The gated backward, which loads five tensors, has tiles of half as many rows.)
 // Tiles are numbered row-block-major (all columns of the first row block, then the next ...; the
 // backward numbers row blocks from the end), CTA c of G takes tiles c, c+G, c+2G... so a tile only
 // ever depends on tiles with smaller numbers, which are always resident or done.
@@ -46,24 +47,39 @@ namespace fss {
 namespace lookback {
 
 constexpr int kW = 4;                         // warps per pass (pass-1 group and pass-2 group)
-constexpr int kR = 16;                        // rows per warp and tile
 constexpr int kRh = 8;                        // rows handled per register batch
-constexpr int kTc = kW * kR;                  // rows per tile
 constexpr int kRowBytes = 256;                // bytes of one tile row
 constexpr int kLaneBytes = 8;
-constexpr int kTileBytes = kTc * kRowBytes;   // 16 KiB per tensor and stage
-constexpr int kPass2Warp0 = kW;               // warps [0,kW) run pass 1, [kW,2kW) run pass 2
-constexpr int kProducerWarp = 2 * kW;
-constexpr int kSummaryWarp = 2 * kW + 1;
-constexpr int kLookbackWarp0 = 2 * kW + 2;    // first of the look-back warps
 constexpr int kLookbackWarps = 2;             // three were measured slower on every workload
 constexpr int kGens = 4;                      // generations of summary buffers: pass 1 may run this far ahead of pass 2
-constexpr int kThreads = (2 * kW + 2 + kLookbackWarps) * 32;
-constexpr int kGateWarp0 = 2 * kW + 2 + kLookbackWarps;      // gated forward only: kW more warps that evaluate the gates
-constexpr int kThreadsGated = kThreads + kW * 32;
-template <bool kGate> constexpr int threads_of() { return kGate ? kThreadsGated : kThreads; }
-constexpr int kStagesFwd = 6;                 // 6 x 32 KiB
-constexpr int kStagesBwd = 4;                 // 4 x 48 KiB
+
+// What differs between the four kinds of scan.
+template <bool kBackward, bool kGate> struct Kind {
+    // tensors a unit loads: alpha, beta | alpha, grad, h | r, x, i | r, grad, h, i, x
+    static constexpr int kIn = kGate ? (kBackward ? 5 : 3) : (kBackward ? 3 : 2);
+    // and stores: h | dalpha, dbeta | h | dr, di, dx
+    static constexpr int kOut = kBackward ? (kGate ? 3 : 2) : 1;
+    // Rows per warp and tile.  Five tensors of 16 KiB would leave room for two stages; with 8 KiB
+    // each there are five, and a tile's life (load, carry, store) overlaps with four others.
+    static constexpr int kR = kGate && kBackward ? 8 : 16;
+    static constexpr int kStages = kGate ? (kBackward ? 5 : 4) : (kBackward ? 4 : 6);
+    static constexpr int kTc = kW * kR;                       // rows per tile (times the split)
+    static constexpr int kTileBytes = kTc * kRowBytes;        // per tensor and stage
+    // Groups of kW pass-2 warps.  Two groups take units alternately where pass 2 carries the chain
+    // rule of the gates (about 45 instructions and 4 special functions per element).
+    static constexpr int kP2 = kGate && kBackward ? 2 : 1;
+    static constexpr int kGateWarps = kGate && !kBackward ? kW : 0;
+    // warps [0, kW) run pass 1, the next kP2 * kW pass 2
+    static constexpr int kPass2Warp0 = kW;
+    static constexpr int kProducerWarp = (1 + kP2) * kW;
+    static constexpr int kSummaryWarp = kProducerWarp + 1;
+    static constexpr int kLookbackWarp0 = kProducerWarp + 2;
+    static constexpr int kGateWarp0 = kLookbackWarp0 + kLookbackWarps;
+    static constexpr int kThreads = (kGateWarp0 + kGateWarps) * 32;
+};
+// rows per tile of the plain scans, before the split
+constexpr int kTc = Kind<false, false>::kTc;
+static_assert(kTc == Kind<true, false>::kTc, "both directions of a scan share their row blocks");
 constexpr uint32_t kMaxSpins = 1u << 21;      // per wait; ~a second before giving up
 
 constexpr uint32_t kStateAggregate = 1, kStateInclusive = 2;
@@ -95,7 +111,10 @@ struct Params {
     float *block_prod;       // [B, S, D]: product of alpha over the rows of each row block
     float *block_state;      // [B, S, D]: state leaving each row block
     const float *h_prev;     // backward only
-    const float *lambda;     // gated forward only: [D] exponent scales -8*softplus(lambda)*log2(e), made by gates::prescale
+    // gated scans only, [D] each: made by gates::prescale (forward: exponent scales) or
+    // gates::backward_tables (backward: -8*softplus(lambda) and its slope; dlambda zeroed)
+    const float *scales, *slopes;
+    float *dlambda;          // gated backward: accumulated
     int continuation;
     int32_t tile_rows;       // rows per tile: 64 * split
     uint32_t max_spins;      // iterations a wait may take before it gives up
@@ -237,6 +256,16 @@ template <> struct Lane<bf16> {
         __nv_bfloat162 hi = __floats2bfloat162_rn(x[2], x[3]);
         return make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
     }
+    static __device__ __forceinline__ Two unpack2(uint32_t w) { return two(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+    static __device__ __forceinline__ uint32_t pack2(const Two &t) {
+        float x, y;
+        split(t, x, y);
+        __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        return *reinterpret_cast<uint32_t *>(&v);
+    }
+    static __device__ __forceinline__ void unpack(const Raw &r, Two (&x)[2]) { x[0] = unpack2(r.x); x[1] = unpack2(r.y); }
+    static __device__ __forceinline__ Raw pack(const Two (&x)[2]) { return make_uint2(pack2(x[0]), pack2(x[1])); }
+    static __device__ __forceinline__ Two rounded(const Two &t) { return unpack2(pack2(t)); }      // as stored and read back
 };
 template <> struct Lane<float> {
     static constexpr int V = 2;
@@ -246,6 +275,13 @@ template <> struct Lane<float> {
     static __device__ __forceinline__ Raw one() { return make_float2(1.0f, 1.0f); }
     static __device__ __forceinline__ void unpack(const Raw &r, float (&x)[2]) { x[0] = r.x; x[1] = r.y; }
     static __device__ __forceinline__ Raw pack(const float (&x)[2]) { return make_float2(x[0], x[1]); }
+    static __device__ __forceinline__ void unpack(const Raw &r, Two (&x)[1]) { x[0] = two(r.x, r.y); }
+    static __device__ __forceinline__ Raw pack(const Two (&x)[1]) {
+        Raw r;
+        split(x[0], r.x, r.y);
+        return r;
+    }
+    static __device__ __forceinline__ Two rounded(const Two &t) { return t; }
 };
 
 // With 64-byte tile rows the two row groups that share a half-warp read the same 16 banks when
@@ -300,12 +336,12 @@ struct Ctl {
 };
 
 // ------------------------------------------------------------------ shared-memory plan
-template <int kTensors, int kStages> struct Smem {
+template <int kTensors, int kStages, int kTileBytes> struct Smem {
     static constexpr int kStageBytes = kTensors * kTileBytes;
     // summaries: [generation][warp][P|C][lane] as 8-byte (fp32 x2) or 16-byte (fp32 x4) entries
     static constexpr int kAggBytes = kGens * kW * 2 * 32 * 16;
     static constexpr int kSumBytes = kGens * 3 * 32 * 16;      // [generation][tile P | tile C | entering state][lane]
-    static constexpr int kBarriers = 4 * kStages + 3 * kGens;      // full, done, info, gate per stage; agg, carry, sum per generation
+    static constexpr int kBarriers = 4 * kStages + 4 * kGens;      // full, done, info, gate per stage; agg, carry, sum, lam per generation
     static constexpr int kBytes = 128 /* alignment slack */ + kStages * kStageBytes + kAggBytes + kSumBytes +
                                   kBarriers * 8 + 16 + kStages * 16 /* unit descriptors */;
 };
@@ -449,21 +485,98 @@ __device__ __forceinline__ void gate_rows(typename Lane<T>::Raw *a_t, typename L
     }
 }
 
+// TMA descriptors of a launch, in the order of Kind's lists
+template <int kIn, int kOut> struct Maps { CUtensorMap in[kIn], out[kOut]; };
+
+// Gated backward: this lane's per-channel constants of a unit, from the tables that were made once
+// per launch; fetched a unit ahead whenever the next unit is already known, so that the load's
+// latency stays off the tile's way.
+template <int V, int Dc> struct ChannelTable {
+    const float *table;
+    int64_t D;
+    int ch;                  // first channel of the lane inside a tile
+    float next[V];
+    bool ready = false;
+    __device__ __forceinline__ void load(const Unit &un, float (&out)[V]) const {
+        const int64_t dch = (int64_t)un.cg * Dc + ch;
+#pragma unroll
+        for (int v = 0; v < V; ++v) out[v] = dch + v < D ? __ldg(table + dch + v) : 0.0f;
+    }
+    template <typename C> __device__ __forceinline__ void ahead(const C &cursor) {
+        ready = cursor.next_known();
+        if (ready) load(cursor.nxt, next);
+    }
+    // the constants of the cursor's current unit; starts fetching those of its next one
+    template <typename C> __device__ __forceinline__ void take(const C &cursor, float (&out)[V]) {
+        if (!ready) load(cursor.cur, next);
+#pragma unroll
+        for (int v = 0; v < V; ++v) out[v] = next[v];
+        ahead(cursor);
+    }
+};
+
+// sum over the lane groups of a warp (lanes that differ only in q); every lane gets it
+template <int LPG> __device__ __forceinline__ float sum_over_groups(float x) {
+#pragma unroll
+    for (int d = LPG; d < 32; d <<= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    return x;
+}
+__device__ __forceinline__ void red_add(float *p, const float (&x)[4]) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
+}
+__device__ __forceinline__ void red_add(float *p, const float (&x)[2]) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x[0]), "f"(x[1]) : "memory");
+}
+
+// Two channels of one row of the gated backward: from (r, g, h_{t-1}, i, x) and the incoming u to (dr, di,
+// dx), with the running sum of d(loss)/d(scale).  The chain rule uses the unrounded gates, the
+// recurrence the alpha the forward scanned with.  `edge` (the row has no alpha): its alpha is `edge_alpha`.
+// Everything that is not a special function is packed arithmetic: the scalar form of this row was
+// limited by instruction supply (818 us for the backward at B16 T4096 D2560 bf16 against 494 us with the
+// same loop).
+template <typename T>
+__device__ __forceinline__ void gated_backward_pair(const Two &r, const Two &g, const Two &hp, const Two &i, const Two &x,
+                                                    const Two &c, const Two &scale, bool edge, float edge_alpha, Two &u, Two &acc,
+                                                    Two &o_r, Two &o_i, Two &o_x) {
+    const Two one = splat(1.0f), minus = splat(-1.0f);
+    const Two s = Gate<T>::sigmoid(r), w = Gate<T>::sigmoid(i);
+    const Two a = gate_alpha<T>(scale, s);
+    Two ar = Lane<T>::rounded(a);
+    const Two dh = add2(g, u);
+    Two da = mul2(dh, hp);
+    if (edge) { ar = splat(edge_alpha); da = splat(0.0f); }
+    u = mul2(ar, dh);
+    // q = sqrt(1 - a^2) and 1/q from one reciprocal square root; an alpha that rounds to 1 has no slope
+    const Two na = mul2(a, minus);
+    const Two q2 = fma2(na, a, one);
+    float q2x, q2y;
+    split(q2, q2x, q2y);
+    const Two rq = two(q2x <= 0.0f ? 0.0f : Gate<T>::rroot(q2x), q2y <= 0.0f ? 0.0f : Gate<T>::rroot(q2y));
+    const Two dx = mul2(mul2(dh, mul2(q2, rq)), w);
+    const Two ga = fma2(mul2(mul2(dh, rq), mul2(w, x)), na, da);      // beta depends on alpha too
+    const Two gs = mul2(mul2(ga, a), s);
+    acc = add2(acc, gs);
+    o_r = mul2(mul2(gs, c), fma2(s, minus, one));
+    o_i = mul2(mul2(dx, x), fma2(w, minus, one));
+    o_x = dx;
+}
+
 // ------------------------------------------------------------------ the kernel
 // Forward: tiles of (alpha, beta) are loaded, h is stored from beta's stage slot.
 // Backward: (alpha, grad, h shifted one row down) are loaded; dbeta is stored from grad's slot,
-// dalpha from h's slot.  Results are written in place in shared memory and leave through TMA
+// dalpha from h's slot.  Gated backward: (r, grad, h shifted, i, x); dr, di, dx are stored from the
+// slots of r, i, x.  Results are written in place in shared memory and leave through TMA
 // stores issued by the producer, so the consumer warps never stall on the global write path.
 template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false>
-__global__ void __launch_bounds__(threads_of<kGate>(), 1)
-scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant__ CUtensorMap map_x,
-            const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_out0,
-            const __grid_constant__ CUtensorMap map_out1, const Params p) {
-    static_assert(!(kGate && (kBackward || kTickets)), "the gate front-end exists for the plain forward only");
-    constexpr bool kThree = kBackward || kGate;      // tensors loaded per unit: 3, else 2
-    constexpr int kTensors = kThree ? 3 : 2;
-    constexpr int kStages = kThree ? kStagesBwd : kStagesFwd;
-    using SM = Smem<kTensors, kStages>;
+__global__ void __launch_bounds__(Kind<kBackward, kGate>::kThreads, 1)
+scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBackward, kGate>::kOut> maps, const Params p) {
+    static_assert(!(kGate && !kBackward && kTickets), "the gated forward keeps the fixed tile order");
+    using K = Kind<kBackward, kGate>;
+    constexpr int kR = K::kR, kTileBytes = K::kTileBytes, kStages = K::kStages;
+    constexpr int kPass2Warp0 = K::kPass2Warp0, kProducerWarp = K::kProducerWarp, kSummaryWarp = K::kSummaryWarp;
+    constexpr int kLookbackWarp0 = K::kLookbackWarp0, kGateWarp0 = K::kGateWarp0;
+    constexpr bool kGateBwd = kGate && kBackward;
+    using SM = Smem<K::kIn, kStages, kTileBytes>;
     constexpr int V = Cfg<T>::V;
     // Tile shape: kSp = 1: 64 rows x 256 bytes; 2: 128 x 128; 4: 256 x 64 (same 16 KiB).  A warp then
     // covers kSp row groups of kR rows at once: lane = (row group q, channel lane cl).
@@ -483,8 +596,9 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
                                                                SM::kAggBytes + SM::kSumBytes + SM::kBarriers * 8);
     Unit *units = reinterpret_cast<Unit *>(smem_raw + kStages * SM::kStageBytes + SM::kAggBytes + SM::kSumBytes +
                                            SM::kBarriers * 8 + 16);
-    auto bar_info = [&](int s) { return bars + 8u * (2 * kStages + 3 * kGens + s); };
-    auto bar_gate = [&](int s) { return bars + 8u * (3 * kStages + 3 * kGens + s); };
+    auto bar_info = [&](int s) { return bars + 8u * (2 * kStages + 4 * kGens + s); };
+    auto bar_gate = [&](int s) { return bars + 8u * (3 * kStages + 4 * kGens + s); };
+    auto bar_lam = [&](int g) { return bars + 8u * (2 * kStages + 3 * kGens + g); };
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_done = [&](int s) { return bars + 8u * (kStages + s); };
     auto bar_agg = [&](int g) { return bars + 8u * (2 * kStages + g); };
@@ -506,17 +620,16 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
     if (!p.hold_dependents) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == kProducerWarp * 32) {
         // the descriptors are kernel parameters, not data of the previous launch: fetch them now
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_alpha) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
-        if (kThree) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_h) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_out0) : "memory");
-        if (kBackward) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_out1) : "memory");
+#pragma unroll
+        for (int j = 0; j < K::kIn; ++j) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.in[j]) : "memory");
+#pragma unroll
+        for (int j = 0; j < K::kOut; ++j) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.out[j]) : "memory");
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(bar_full(s), 1); mbar_init(bar_done(s), kW); mbar_init(bar_info(s), 1); mbar_init(bar_gate(s), kW);
         }
-        for (int g = 0; g < kGens; ++g) { mbar_init(bar_agg(g), kW); mbar_init(bar_carry(g), 1); mbar_init(bar_sum(g), 1); }
+        for (int g = 0; g < kGens; ++g) { mbar_init(bar_agg(g), kW); mbar_init(bar_carry(g), 1); mbar_init(bar_sum(g), 1); mbar_init(bar_lam(g), kW); }
         *cta_abort = 0;
         asm volatile("griddepcontrol.wait;" ::: "memory");      // the previous launch and its writes are complete
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -581,10 +694,9 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
                 const uint32_t base = smem_base + st * SM::kStageBytes;
                 const int32_t c0 = nu.cg * Dc, c1 = nu.template row0<kBackward>(p), c2 = nu.b;
                 mbar_arrive_expect_tx(bar_full(st), SM::kStageBytes);
-                tma_load_3d(base, &map_alpha, bar_full(st), c0, c1, c2);
-                tma_load_3d(base + kTileBytes, &map_x, bar_full(st), c0, c1, c2);
-                if (kBackward) tma_load_3d(base + 2 * kTileBytes, &map_h, bar_full(st), c0, c1 - 1, c2);
-                if (kGate) tma_load_3d(base + 2 * kTileBytes, &map_h, bar_full(st), c0, c1, c2);      // input gate
+#pragma unroll
+                for (int j = 0; j < K::kIn; ++j)      // the backward's third tensor is h, one row up
+                    tma_load_3d(base + j * kTileBytes, &maps.in[j], bar_full(st), c0, kBackward && j == 2 ? c1 - 1 : c1, c2);
                 ++issued;
             };
             // One loop for both the initial fill (slots 0 .. kStages-1) and the steady state, in which
@@ -599,11 +711,15 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
                     const Unit u = units[st];
                     const int32_t c0 = u.cg * Dc, c1 = u.template row0<kBackward>(p), c2 = u.b;
                     if (!ctl.wait(bar_done(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
-                    if (!kBackward) {
-                        tma_store_3d(&map_out0, base + kTileBytes, c0, c1, c2);          // h
+                    if constexpr (kGateBwd) {
+                        tma_store_3d(&maps.out[0], base, c0, c1, c2);                       // dr
+                        tma_store_3d(&maps.out[1], base + 3 * kTileBytes, c0, c1, c2);      // di
+                        tma_store_3d(&maps.out[2], base + 4 * kTileBytes, c0, c1, c2);      // dx
+                    } else if constexpr (kBackward) {
+                        tma_store_3d(&maps.out[0], base + 2 * kTileBytes, c0, c1, c2);      // dalpha
+                        tma_store_3d(&maps.out[1], base + kTileBytes, c0, c1, c2);          // dbeta
                     } else {
-                        tma_store_3d(&map_out0, base + 2 * kTileBytes, c0, c1, c2);      // dalpha
-                        tma_store_3d(&map_out1, base + kTileBytes, c0, c1, c2);          // dbeta
+                        tma_store_3d(&maps.out[0], base + kTileBytes, c0, c1, c2);          // h
                     }
                     tma_commit();
                     if (nu.k >= 0) tma_wait_read_all();   // the stage may be overwritten once the store has read it
@@ -719,7 +835,7 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
                 }
             }
         }
-    } else if (kGate && warp >= kGateWarp0) {
+    } else if (kGate && !kBackward && warp >= kGateWarp0) {
         // ============================================================ gates (gated forward only)
         // The alpha slot of a stage arrives holding r, the third slot i, the beta slot x.  These
         // warps turn them into alpha and beta in place as soon as the tile has landed, one warp per
@@ -741,7 +857,7 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
         auto load_scales = [&](const Unit &un, float (&out)[V]) {
             const int64_t dch = (int64_t)un.cg * Dc + cl * V;
 #pragma unroll
-            for (int v = 0; v < V; ++v) out[v] = dch + v < p.D ? __ldg(p.lambda + dch + v) : 0.0f;
+            for (int v = 0; v < V; ++v) out[v] = dch + v < p.D ? __ldg(p.scales + dch + v) : 0.0f;
         };
         float gsc_next[V];
         load_scales(u0, gsc_next);
@@ -959,11 +1075,15 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
         const uint32_t lane_off = (uint32_t)(grp * kR) * kRowB + (uint32_t)cl * kLaneBytes;
         Cursor cursor(p, ctl, units, bar_info(0));
         cursor.init(u0, 0, 1);
+        ChannelTable<V, Dc> table{p.scales, p.D, cl * V};
+        if (kGateBwd) table.ahead(cursor);
 #pragma unroll 1
         for (int i = 0;; ++i) {
             const int st = i % kStages, g = i % kGens;
             if (!cursor.advance(i)) break;
             const Unit u = cursor.cur;
+            float c[V];
+            if (kGateBwd) table.take(cursor, c);
             const int32_t row0 = u.template row0<kBackward>(p);
             const bool head = (row0 == 0) && (grp == 0) && !p.continuation;
             // rows of this group that exist in the sequence (fewer than kR only in the last row block)
@@ -977,7 +1097,7 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
             Raw *a_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + lane_off);
             Raw *x_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + kTileBytes + lane_off);
             // gated forward: the gate warps turn the stage into (alpha, beta), edge rows included
-            if (kGate && !ctl.wait(bar_gate(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
+            if (kGate && !kBackward && !ctl.wait(bar_gate(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
             // row 0 of the whole sequence: alpha_0 is not part of the recurrence
             if (!kGate && head) a_t[0] = Lane<T>::zero();
             // rows past the end of the sequence arrive zero-filled; alpha = 1 (beta, grad = 0) makes
@@ -989,8 +1109,53 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
             float P[V], C[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) { P[v] = 1.0f; C[v] = 0.0f; }
+            if constexpr (kGateBwd) {
+                constexpr int kPairs = V / 2;
+                constexpr int kGateRows1 = 2;      // (as kGateRows2 below: 1 row 466 us, 4 rows 514 us with two in pass 2)
+                const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
+                Two scale[kPairs], P2[kPairs], C2[kPairs];
+#pragma unroll
+                for (int v = 0; v < kPairs; ++v) {
+                    scale[v] = two(Gate<T>::prescale(c[2 * v]), Gate<T>::prescale(c[2 * v + 1]));
+                    P2[v] = splat(1.0f);
+                    C2[v] = splat(0.0f);
+                }
 #pragma unroll 1
-            for (int hb = 0; hb < kR / kRh; ++hb) {
+                for (int base = kR - kGateRows1; base >= 0; base -= kGateRows1) {
+                    Raw ra[kGateRows1], rx[kGateRows1];
+#pragma unroll
+                    for (int r = 0; r < kGateRows1; ++r) {
+                        ra[r] = pair_slot<kRowStride>(a_t, base + r, dsw);
+                        rx[r] = pair_slot<kRowStride>(x_t, base + r, dsw);
+                    }
+                    pair_fix<kPairSwap>(ra, odd_grp);
+                    pair_fix<kPairSwap>(rx, odd_grp);
+#pragma unroll
+                    for (int j = 0; j < kGateRows1; ++j) {
+                        const int r = kGateRows1 - 1 - j;
+                        Two xr[kPairs], xg[kPairs];
+                        Lane<T>::unpack(ra[r], xr);
+                        Lane<T>::unpack(rx[r], xg);
+#pragma unroll
+                        for (int v = 0; v < kPairs; ++v) {      // alpha rounded as the forward rounded it
+                            Two a = Lane<T>::rounded(gate_alpha<T>(scale[v], Gate<T>::sigmoid(xr[v])));
+                            if (edge_rows) {
+                                if (head && base + r == 0) a = splat(0.0f);
+                                else if (base + r >= nvalid) a = splat(1.0f);
+                            }
+                            C2[v] = mul2(a, add2(xg[v], C2[v]));
+                            P2[v] = mul2(P2[v], a);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < kPairs; ++v) {
+                    split(P2[v], P[2 * v], P[2 * v + 1]);
+                    split(C2[v], C[2 * v], C[2 * v + 1]);
+                }
+            }
+#pragma unroll 1
+            for (int hb = 0; hb < (kGateBwd ? 0 : kR / kRh); ++hb) {
                 const int base = kBackward ? kR - kRh * (hb + 1) : kRh * hb;     // rows of this batch
                 Raw ra[kRh], rx[kRh];
 #pragma unroll
@@ -1027,7 +1192,8 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
         // Re-scans this warp's rows from the true entering state and writes the results in place.
         using Raw = typename Lane<T>::Raw;
         constexpr int kRowStride = kRowB / (int)sizeof(Raw);
-        const int w2 = warp - kPass2Warp0;
+        const int w2 = (warp - kPass2Warp0) % kW;
+        const int group2 = K::kP2 > 1 ? (warp - kPass2Warp0) / kW : 0;
         const int grp = q * kW + w2;
         constexpr bool kPairSwap = kRowB == 64;
         const bool odd_grp = kPairSwap && (q & 1);
@@ -1035,12 +1201,16 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
         const uint32_t lane_off = (uint32_t)(grp * kR) * kRowB + (uint32_t)cl * kLaneBytes;
         const int ch = cl * V;
         Cursor cursor(p, ctl, units, bar_info(0));
-        cursor.init(u0, 0, 1);
+        cursor.init(u0, group2, K::kP2);
+        ChannelTable<V, Dc> table{p.scales, p.D, ch};
+        if (kGateBwd) table.ahead(cursor);
 #pragma unroll 1
-        for (int i = 0;; ++i) {
+        for (int i = group2;; i += K::kP2) {
             const int st = i % kStages, g = i % kGens;
             if (!cursor.advance(i)) break;
             const Unit u = cursor.cur;
+            float c[V];
+            if (kGateBwd) table.take(cursor, c);
             const bool head = (u.template row0<kBackward>(p) == 0) && (grp == 0);
             const int32_t b = u.b;
             const int64_t dch = (int64_t)u.cg * Dc + ch;
@@ -1055,6 +1225,112 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
                 const VecF ep = agg_at(g, w2, 0, lane), ec = agg_at(g, w2, 1, lane), vin = sum_at(g, 2, lane);
 #pragma unroll
                 for (int v = 0; v < V; ++v) stv[v] = fmaf(vec_get(ep, v), vec_get(vin, v), vec_get(ec, v));
+            }
+            if constexpr (kGateBwd) {
+                constexpr int kPairs = V / 2;
+                // Rows per loop body.  Three heavy warps of a scheduler run different code here, and with
+                // longer bodies they wait for instructions: 4 rows 565 us, 2 rows 494 us, 1 row 456 us (c4
+                // shape, bf16).  The row pairs of 64-byte tile rows need two.
+                constexpr int kGateRows2 = kPairSwap ? 2 : 1;
+                const int64_t left = p.T - u.template row0<kBackward>(p) - (int64_t)grp * kR;
+                const int nvalid = left >= kR ? kR : (left > 0 ? (int)left : 0);
+                const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
+                Raw *r_t = const_cast<Raw *>(a_t);
+                Raw *i_t = h_t + kTileBytes / (int)sizeof(Raw), *xin_t = i_t + kTileBytes / (int)sizeof(Raw);
+                Two c2[kPairs], scale[kPairs], st2[kPairs], acc2[kPairs];
+#pragma unroll
+                for (int v = 0; v < kPairs; ++v) {
+                    c2[v] = two(c[2 * v], c[2 * v + 1]);
+                    scale[v] = two(Gate<T>::prescale(c[2 * v]), Gate<T>::prescale(c[2 * v + 1]));
+                    st2[v] = two(stv[2 * v], stv[2 * v + 1]);
+                    acc2[v] = splat(0.0f);
+                }
+#pragma unroll 1
+                for (int base = kR - kGateRows2; base >= 0; base -= kGateRows2) {
+                    Raw rr[kGateRows2], rg[kGateRows2], rh[kGateRows2], ri[kGateRows2], rx[kGateRows2];
+#pragma unroll
+                    for (int r = 0; r < kGateRows2; ++r) {
+                        rr[r] = pair_slot<kRowStride>(r_t, base + r, dsw);
+                        rg[r] = pair_slot<kRowStride>(x_t, base + r, dsw);
+                        rh[r] = pair_slot<kRowStride>(h_t, base + r, dsw);
+                        ri[r] = pair_slot<kRowStride>(i_t, base + r, dsw);
+                        rx[r] = pair_slot<kRowStride>(xin_t, base + r, dsw);
+                    }
+                    pair_fix<kPairSwap>(rr, odd_grp);
+                    pair_fix<kPairSwap>(rg, odd_grp);
+                    pair_fix<kPairSwap>(rh, odd_grp);
+                    pair_fix<kPairSwap>(ri, odd_grp);
+                    pair_fix<kPairSwap>(rx, odd_grp);
+#pragma unroll
+                    for (int j = 0; j < kGateRows2; ++j) {
+                        const int r = kGateRows2 - 1 - j;
+                        Two xr[kPairs], xg[kPairs], xh[kPairs], xi[kPairs], xx[kPairs], o_r[kPairs], o_i[kPairs], o_x[kPairs];
+                        Lane<T>::unpack(rr[r], xr);
+                        Lane<T>::unpack(rg[r], xg);
+                        Lane<T>::unpack(rh[r], xh);
+                        Lane<T>::unpack(ri[r], xi);
+                        Lane<T>::unpack(rx[r], xx);
+                        // row 0 of the sequence: alpha is not part of the recurrence; rows after the end hand u on
+                        const bool first_row = head && base + r == 0;
+                        const bool edge = edge_rows && (first_row || base + r >= nvalid);
+#pragma unroll
+                        for (int v = 0; v < kPairs; ++v)
+                            gated_backward_pair<T>(xr[v], xg[v], xh[v], xi[v], xx[v], c2[v], scale[v], edge,
+                                                   first_row ? 0.0f : 1.0f, st2[v], acc2[v], o_r[v], o_i[v], o_x[v]);
+                        rr[r] = Lane<T>::pack(o_r);
+                        ri[r] = Lane<T>::pack(o_i);
+                        rx[r] = Lane<T>::pack(o_x);
+                    }
+                    pair_fix<kPairSwap>(rr, odd_grp);
+                    pair_fix<kPairSwap>(ri, odd_grp);
+                    pair_fix<kPairSwap>(rx, odd_grp);
+#pragma unroll
+                    for (int r = 0; r < kGateRows2; ++r) {
+                        pair_slot<kRowStride>(r_t, base + r, dsw) = rr[r];
+                        pair_slot<kRowStride>(i_t, base + r, dsw) = ri[r];
+                        pair_slot<kRowStride>(xin_t, base + r, dsw) = rx[r];
+                    }
+                }
+                fence_proxy_async();
+                // d(loss)/d(lambda) of the tile: the warps leave their sums in the slots they took
+                // their prefixes from; one of them (in turn) folds the four and adds them to memory,
+                // one vector add per 32 * kSp rows and channel vector.  It reports the unit done only
+                // when it has read the slots: pass 1 may then fill them again.
+                VecF mine;
+#pragma unroll
+                for (int v = 0; v < kPairs; ++v) {
+                    float lo, hi;
+                    split(acc2[v], lo, hi);
+                    vec_set(mine, 2 * v, lo);
+                    vec_set(mine, 2 * v + 1, hi);
+                }
+                agg_at(g, w2, 0, lane) = mine;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_lam(g));
+                if (w2 == ((i / K::kP2) % kW)) {
+                    if (!ctl.wait(bar_lam(g), (uint32_t)((i / kGens) & 1), FSS_STATUS_LOOKBACK_TIMEOUT)) break;
+                    float sum[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) sum[v] = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < kW; ++w) {
+                        const VecF part = agg_at(g, w, 0, lane);
+#pragma unroll
+                        for (int v = 0; v < V; ++v) sum[v] += vec_get(part, v);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_done(st));
+#pragma unroll
+                    for (int v = 0; v < V; ++v) sum[v] = sum_over_groups<LPG>(sum[v]);
+                    if (q == 0 && dch < p.D) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v) sum[v] *= __ldg(p.slopes + dch + v);
+                        red_add(p.dlambda + dch, sum);
+                    }
+                } else if (lane == 0) {
+                    mbar_arrive(bar_done(st));
+                }
+                continue;
             }
 #pragma unroll 1
             for (int hb = 0; hb < kR / kRh; ++hb) {
@@ -1153,13 +1429,13 @@ scan_kernel(const __grid_constant__ CUtensorMap map_alpha, const __grid_constant
 // Tile shape for a problem: split s gives tiles of 64*s rows x 256/s bytes.  Narrow, tall tiles
 // multiply the number of columns; with fewer columns than about two per SM several row blocks of
 // one column are in flight at once and the carry chain between them limits the speed.
-inline int choose_split(int dtype, int64_t B, int64_t T, int64_t D) {
+inline int choose_split(int dtype, int64_t B, int64_t T, int64_t D, int tile_rows = kTc) {
     static const int env = [] { const char *e = getenv("FSS_B200_SPLIT"); return e ? atoi(e) : 0; }();
     if (env == 1 || env == 2 || env == 4) return env;
     const int64_t row_bytes = D * (dtype == FSS_DTYPE_BF16 ? 2 : 4);
     const int64_t cols = B * ceil_div(row_bytes, kRowBytes);
     int s = 1;
-    while (s < 4 && cols * s < 2 * 148 && row_bytes >= kRowBytes / s && T >= 2 * kTc * s * 2) s *= 2;
+    while (s < 4 && cols * s < 2 * 148 && row_bytes >= kRowBytes / s && T >= 2 * tile_rows * s * 2) s *= 2;
     return s;
 }
 // Tile order.  Returns how many units at the END of a CTA's share are handed out by the global
@@ -1189,12 +1465,12 @@ template <typename T> inline int64_t channel_groups(int64_t D) { return ceil_div
 template <typename T> constexpr int packets_per_tile() {
     return (PacketGroup<2 * Cfg<T>::V>::kPackets + PacketGroup<Cfg<T>::V>::kPackets) * 32;
 }
-inline size_t workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype) {
+inline size_t workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype, int tile_rows = kTc) {
     const int Dc = dtype == FSS_DTYPE_BF16 ? Cfg<bf16>::Dc : Cfg<float>::Dc;
     const int per_tile = dtype == FSS_DTYPE_BF16 ? packets_per_tile<bf16>() : packets_per_tile<float>();
     size_t worst = 0;
     for (int s = 1; s <= 4; s *= 2) {       // any tile shape the launcher may pick
-        const int64_t ntiles = B * ceil_div(D, Dc / s) * ceil_div(T, (int64_t)kTc * s);
+        const int64_t ntiles = B * ceil_div(D, Dc / s) * ceil_div(T, (int64_t)tile_rows * s);
         const size_t need = (size_t)ntiles * (per_tile / s) * 16;
         if (need > worst) worst = need;
     }
@@ -1239,17 +1515,17 @@ inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 3-D map (channels, rows, batch) with a (Dc, kTc, 1) box; out-of-range elements read as zero
+// 3-D map (channels, rows, batch) with a (Dc, tile rows, 1) box; out-of-range elements read as zero
 // and are dropped on store.
 template <typename T>
-inline bool make_map(CUtensorMap *map, const fss_view *v, int64_t B, int64_t Tn, int64_t D, int split, std::string *err) {
+inline bool make_map(CUtensorMap *map, const fss_view *v, int64_t B, int64_t Tn, int64_t D, int split, int tile_rows, std::string *err) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) { *err = "cuTensorMapEncodeTiled entry point not found"; return false; }
     const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)Tn, (cuuint64_t)B};
     const int64_t sb = B > 1 ? v->stride_b : v->stride_t * Tn;
     const cuuint64_t strides[2] = {(cuuint64_t)(v->stride_t * (int64_t)sizeof(T)),
                                    (cuuint64_t)(sb * (int64_t)sizeof(T))};
-    const cuuint32_t box[3] = {(cuuint32_t)(Cfg<T>::Dc / split), (cuuint32_t)(kTc * split), 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(Cfg<T>::Dc / split), (cuuint32_t)(tile_rows * split), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const CUresult r = fn(map, dt, 3, v->ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1273,10 +1549,10 @@ inline bool make_map(CUtensorMap *map, const fss_view *v, int64_t B, int64_t Tn,
 struct MapKey {
     const void *ptr;
     int64_t B, T, D, sb, st;
-    int32_t split, esize;
+    int32_t split, tile_rows, esize;
     bool operator==(const MapKey &o) const {
         return ptr == o.ptr && B == o.B && T == o.T && D == o.D && sb == o.sb && st == o.st && split == o.split &&
-               esize == o.esize;
+               tile_rows == o.tile_rows && esize == o.esize;
     }
 };
 struct MapCache {
@@ -1286,9 +1562,9 @@ struct MapCache {
     uint8_t next[kSets] = {};
 };
 template <typename T>
-inline const CUtensorMap *cached_map(const fss_view *v, int64_t B, int64_t Tn, int64_t D, int split, std::string *err) {
+inline const CUtensorMap *cached_map(const fss_view *v, int64_t B, int64_t Tn, int64_t D, int split, int tile_rows, std::string *err) {
     static thread_local MapCache cache;
-    const MapKey key{v->ptr, B, Tn, D, v->stride_b, v->stride_t, split, (int32_t)sizeof(T)};
+    const MapKey key{v->ptr, B, Tn, D, v->stride_b, v->stride_t, split, tile_rows, (int32_t)sizeof(T)};
     const uintptr_t a = reinterpret_cast<uintptr_t>(v->ptr);
     const int set = (int)(((a >> 9) ^ (a >> 21) ^ (uintptr_t)split) % MapCache::kSets);
     for (auto &slot : cache.slots[set])
@@ -1296,7 +1572,7 @@ inline const CUtensorMap *cached_map(const fss_view *v, int64_t B, int64_t Tn, i
     auto &slot = cache.slots[set][cache.next[set]];
     cache.next[set] = (uint8_t)((cache.next[set] + 1) % MapCache::kWays);
     slot.valid = false;
-    if (!make_map<T>(&slot.map, v, B, Tn, D, split, err)) return nullptr;
+    if (!make_map<T>(&slot.map, v, B, Tn, D, split, tile_rows, err)) return nullptr;
     slot.key = key;
     slot.valid = true;
     return &slot.map;
@@ -1314,7 +1590,7 @@ template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate> inline
         *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (*err != cudaSuccess) return 0;
         int per_sm = 0, sms = 0;
-        *err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads_of<kGate>(), smem_bytes);
+        *err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Kind<kBackward, kGate>::kThreads, smem_bytes);
         if (*err != cudaSuccess) return 0;
         *err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (*err != cudaSuccess) return 0;
@@ -1325,31 +1601,29 @@ template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate> inline
     return cached[device];
 }
 
+// `in`, `out`: the views in the order of Kind's lists
 template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false>
 inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D,
-                  const fss_view *alpha, const fss_view *x, const fss_view *h, const fss_view *out0,
-                  const fss_view *out1, Params p, int tail, std::string *err_text) {
-    constexpr int kTensors = (kBackward || kGate) ? 3 : 2;
-    constexpr int kStages = (kBackward || kGate) ? kStagesBwd : kStagesFwd;
-    constexpr int smem_bytes = Smem<kTensors, kStages>::kBytes;
+                        std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p, int tail,
+                        std::string *err_text) {
+    using K = Kind<kBackward, kGate>;
+    constexpr int kTc = K::kTc, kStages = K::kStages;
+    constexpr int smem_bytes = Smem<K::kIn, kStages, K::kTileBytes>::kBytes;
+    static_assert(smem_bytes <= 227 * 1024, "more shared memory than a CTA may have");
     constexpr int Dc = Cfg<T>::Dc / kSp;
 
-    // copies: a later look-up may evict the slot an earlier pointer refers to
-    CUtensorMap m_alpha, m_x, m_h, m_o0, m_o1;
+    Maps<K::kIn, K::kOut> maps;
     auto fetch = [&](CUtensorMap *dst, const fss_view *v) {
-        const CUtensorMap *m = cached_map<T>(v, B, Tn, D, kSp, err_text);
-        if (m) *dst = *m;
+        const CUtensorMap *m = cached_map<T>(v, B, Tn, D, kSp, kTc, err_text);
+        if (m) *dst = *m;      // a copy: a later look-up may evict the slot
         return m != nullptr;
     };
-    if (!fetch(&m_alpha, alpha) || !fetch(&m_x, x) || !fetch(&m_o0, out0)) return FSS_E_TENSORMAP;
-    if (kBackward) {
-        if (!fetch(&m_h, h) || !fetch(&m_o1, out1)) return FSS_E_TENSORMAP;
-    } else if (kGate) {
-        if (!fetch(&m_h, h)) return FSS_E_TENSORMAP;      // the input gate
-        m_o1 = m_o0;
-    } else {
-        m_h = m_alpha; m_o1 = m_o0;
-    }
+    CUtensorMap *dst = maps.in;
+    for (const fss_view *v : in)
+        if (!fetch(dst++, v)) return FSS_E_TENSORMAP;
+    dst = maps.out;
+    for (const fss_view *v : out)
+        if (!fetch(dst++, v)) return FSS_E_TENSORMAP;
 
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -1391,7 +1665,7 @@ inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, in
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads_of<kGate>());
+    cfg.blockDim = dim3(K::kThreads);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = (cudaStream_t)ctx->stream;
     cudaLaunchAttribute attr[1];
@@ -1408,22 +1682,23 @@ inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, in
     const bool use_pdl = pdl_env >= 0 ? pdl_env == 1 : (!kBackward || p.ntiles <= kPdlMaxUnits * (int64_t)grid);
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, scan_kernel<T, kBackward, kSp, kTickets, kGate>, m_alpha, m_x, m_h, m_o0, m_o1, p);
+    e = cudaLaunchKernelEx(&cfg, scan_kernel<T, kBackward, kSp, kTickets, kGate>, maps, p);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { *err_text = std::string("look-back launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     return FSS_OK;
 }
 
-template <typename T, bool kBackward>
+template <typename T, bool kBackward, bool kGate = false>
 inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D,
-                  const fss_view *alpha, const fss_view *x, const fss_view *h, const fss_view *out0,
-                  const fss_view *out1, Params p, std::string *err_text) {
+                  std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p,
+                  std::string *err_text) {
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
-    const int tail = choose_tail(dtype, kBackward, B, Tn, D);
-#define FSS_LAUNCH_SPLIT(SP)                                                                                       \
-    return tail > 0 ? launch_split<T, kBackward, SP, true>(ctx, ws, B, Tn, D, alpha, x, h, out0, out1, p, tail, err_text) \
-                    : launch_split<T, kBackward, SP, false>(ctx, ws, B, Tn, D, alpha, x, h, out0, out1, p, 0, err_text)
-    switch (choose_split(dtype, B, Tn, D)) {
+    constexpr bool kNeverTickets = kGate && !kBackward;
+    const int tail = kNeverTickets ? 0 : choose_tail(dtype, kBackward, B, Tn, D);
+#define FSS_LAUNCH_SPLIT(SP)                                                                                                    \
+    return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
+                    : launch_split<T, kBackward, SP, false, kGate>(ctx, ws, B, Tn, D, in, out, p, 0, err_text)
+    switch (choose_split(dtype, B, Tn, D, Kind<kBackward, kGate>::kTc)) {
     case 4: FSS_LAUNCH_SPLIT(4);
     case 2: FSS_LAUNCH_SPLIT(2);
     default: FSS_LAUNCH_SPLIT(1);
@@ -1508,7 +1783,7 @@ inline int forward(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t
         if (float_scratch_bytes(B, Tn, D) > ws.float_bytes) return FSS_E_WORKSPACE;
         p.block_prod = reinterpret_cast<float *>(ws.floats);
     }
-    const int rc = launch<T, false>(ctx, ws, B, Tn, D, alpha, beta, nullptr, h, nullptr, p, err_text);
+    const int rc = launch<T, false>(ctx, ws, B, Tn, D, {alpha, beta}, {h}, p, err_text);
     if (rc != FSS_OK || !prod) return rc;
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
     const int64_t S = ceil_div(Tn, block_rows(dtype, B, Tn, D));
@@ -1535,13 +1810,28 @@ inline int forward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, i
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { *err_text = std::string("gate scale launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     }
-    p.lambda = scales;
-    const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
-    switch (choose_split(dtype, B, Tn, D)) {
-    case 4: return launch_split<T, false, 4, false, true>(ctx, ws, B, Tn, D, r, x, i, h, nullptr, p, 0, err_text);
-    case 2: return launch_split<T, false, 2, false, true>(ctx, ws, B, Tn, D, r, x, i, h, nullptr, p, 0, err_text);
-    default: return launch_split<T, false, 1, false, true>(ctx, ws, B, Tn, D, r, x, i, h, nullptr, p, 0, err_text);
-    }
+    p.scales = scales;
+    return launch<T, false, true>(ctx, ws, B, Tn, D, {r, x, i}, {h}, p, err_text);
+}
+
+// Backward of the gated scan in one pass over memory: reads r, grad, h, i, x and writes dr, di, dx (8
+// tensor passes; re-creating alpha, the plain reverse scan and the gates' chain rule as launches of
+// their own take 15) and adds the gradient of lambda per tile.  Measured at B16 T4096 D2560 bf16: the three
+// launches 1,204 us (153 + 268 + 783), this one 456 us = 5.9 TB/s; fp32 at B4 T2048 D2560 107 us = 6.3 TB/s.
+template <typename T>
+inline int backward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D, const fss_view *r,
+                          const fss_view *i, const fss_view *x, const float *lambda, const fss_view *h, const fss_view *grad,
+                          const fss_view *dr, const fss_view *di, const fss_view *dx, float *dlambda, std::string *err_text) {
+    if ((size_t)D * 2 * sizeof(float) > ws.float_bytes) return FSS_E_WORKSPACE;
+    Params p{};
+    float *scales = reinterpret_cast<float *>(ws.floats), *slopes = scales + D;
+    gates::backward_tables<<<(unsigned)ceil_div(D, 256), 256, 0, (cudaStream_t)ctx->stream>>>(lambda, scales, slopes, dlambda, D);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { *err_text = std::string("gate table launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
+    p.scales = scales;
+    p.slopes = slopes;
+    p.dlambda = dlambda;
+    return launch<T, true, true>(ctx, ws, B, Tn, D, {r, grad, h, i, x}, {dr, di, dx}, p, err_text);
 }
 
 template <typename T>
@@ -1557,7 +1847,7 @@ inline int backward(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_
         p.block_state = st->block_state;
         p.h_prev = cont ? st->h_prev : nullptr;
     }
-    return launch<T, true>(ctx, ws, B, Tn, D, alpha, grad, h, dalpha, dbeta, p, err_text);
+    return launch<T, true>(ctx, ws, B, Tn, D, {alpha, grad, h}, {dalpha, dbeta}, p, err_text);
 }
 
 // fp32 state vectors are moved as 8- or 16-byte words by the single-pass kernels

@@ -85,14 +85,14 @@ def _view(t: torch.Tensor) -> _lib.View:
 _ws_bytes_cache: dict = {}
 
 
-def _workspace_for(t: torch.Tensor, dtype_id: int) -> workspace.Workspace:
-    """The calling stream's workspace on ``t``'s device, large enough for a scan of ``t``'s shape.
-    The size query is a native call; its answers are remembered per shape."""
-    key = (t.shape, dtype_id)
+def _workspace_for(t: torch.Tensor, dtype_id: int, query: str = "fss_workspace_bytes") -> workspace.Workspace:
+    """The calling stream's workspace on ``t``'s device, large enough for a scan of ``t``'s shape (``query``: the
+    native call that says how large).  The answers are remembered per shape."""
+    key = (t.shape, dtype_id, query)
     need = _ws_bytes_cache.get(key)
     if need is None:
         B, T, D = t.shape
-        need = _ws_bytes_cache[key] = _lib.lib().fss_workspace_bytes(B, T, D, dtype_id)
+        need = _ws_bytes_cache[key] = getattr(_lib.lib(), query)(B, T, D, dtype_id)
     return workspace.get(t.device, need)
 
 
@@ -277,6 +277,33 @@ def gates_backward(r, i, x, lam, grad_alpha, grad_beta):
                                        lam.data_ptr(), *[ctypes.byref(v) for v in views[3:]], dlam.data_ptr())
     _lib.check(rc, "fss_gates_backward")
     return dr, di, dx, dlam
+
+
+def scan_backward_gated(r, i, x, lam, h, grad_out):
+    """``(grad_r, grad_i, grad_x, grad_lam)`` of ``h = scan_forward_gated(r, i, x, lam)`` from the gradient of
+    ``h``: one kernel (``fss_scan_backward_gated``) where the layout allows it, else alpha again, the reverse scan
+    and the gates' chain rule as launches of their own."""
+    dtype = _check_gate_inputs(r, i, x, lam)
+    _check_tensor("h", h, r, dtype)
+    _check_tensor("grad_out", grad_out, r, dtype)
+    if r.numel():
+        B, T, D = r.shape
+        dr, di, dx = (torch.empty(r.shape, dtype=dtype, device=r.device) for _ in range(3))
+        dlam = torch.empty(D, dtype=torch.float32, device=r.device)
+        tensors = [_rowwise(t) for t in (r, i, x, h, grad_out)] + [dr, di, dx]
+        v = [_view(t) for t in tensors]
+        ws = _workspace_for(r, _DTYPES[dtype], "fss_gated_backward_workspace_bytes")
+        ctx = _ctx(r.device, ws, None)
+        rc = _lib.lib().fss_scan_backward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(v[0]),
+                                                ctypes.byref(v[1]), ctypes.byref(v[2]), lam.data_ptr(),
+                                                *[ctypes.byref(w) for w in v[3:]], dlam.data_ptr())
+        workspace.launched(ws)
+        if rc == 0:
+            return dr, di, dx, dlam
+        if rc != _lib.E_LAYOUT:
+            _lib.check(rc, "fss_scan_backward_gated")
+    alpha, _ = gates_forward(r, None, None, lam, want_beta=False)
+    return gates_backward(r, i, x, lam, *_backward(alpha, h, grad_out, dtype))
 
 
 def scan_forward_gated(r, i, x, lam) -> torch.Tensor:

@@ -218,6 +218,18 @@ int fss_gates_backward(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t T,
                        const fss_view *r, const fss_view *i, const fss_view *x, const float *lambda,
                        const fss_view *grad_alpha, const fss_view *grad_beta, const fss_view *grad_r,
                        const fss_view *grad_i, const fss_view *grad_x, float *grad_lambda);
+/* Backward of fss_scan_forward_gated in one pass over memory: re-creates alpha from r, runs the reverse
+ * scan and the chain rule of fss_gates_backward tile by tile.  Reads r, i, x, h, grad_out and writes
+ * grad_r, grad_i, grad_x: 8 tensor passes instead of the 15 of fss_gates_forward, the reverse scan and
+ * fss_gates_backward.  grad_lambda[D] (16-byte aligned, else FSS_E_LAYOUT) is overwritten; its last bits
+ * depend on the order of the additions.  Same layouts as the forward (FSS_E_LAYOUT otherwise) and the
+ * size limits of fss_gates_backward; no boundary state (FSS_FLAG_CONTINUATION: FSS_E_ARGS).  The
+ * workspace is the stream's, at least fss_gated_backward_workspace_bytes(). */
+int fss_scan_backward_gated(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t T, int64_t D,
+                            const fss_view *r, const fss_view *i, const fss_view *x, const float *lambda,
+                            const fss_view *h, const fss_view *grad_out, const fss_view *grad_r,
+                            const fss_view *grad_i, const fss_view *grad_x, float *grad_lambda);
+size_t fss_gated_backward_workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype);
 
 /* ---- sequence-parallel pieces (no counterpart in the reference, which never splits T) ---- */
 /* Rows per block of the block_prod outputs for this problem and algorithm (> 0). */

@@ -446,6 +446,33 @@ def test_gated_scan_gradients(dtype, lam_range):
     assert_same_up_to_association(h_two, h.detach(), "gate kernel + plain scan vs fused forward")
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(2, 1, 8), (1, 31, 136), (3, 33, 24), (2, 260, 136), (1, 1025, 264), (5, 97, 1000), (2, 6200, 4104)])
+def test_gated_backward_in_one_kernel_matches_the_three_kernels(shape, dtype):
+    """The fused backward at the edges of its tiles (one row; one less and more than a tile; each tile shape; the last
+    shape by tickets) on views of wider tensors, against alpha, reverse scan and chain rule as kernels of their own.
+    Bounds: the three kernels round alpha's and beta's gradients and the results to 8 bits, the fused one the results
+    only: three roundings of at most 2^-9 apart, 2^-7 in the 2-norm with room for the reverse scan's own roundings;
+    fp32 differs by a few ulp, amplified by at most 1/(1 - alpha) ~ 100 and by the sum over rows in lambda's gradient."""
+    pkg, native, _ = _mods()
+    from fast_sequential_scan_b200.workloads import Workload, make_gate_inputs
+    B, T, D = shape
+    wide = Workload("t", B, T, D + 8, "hawk", dtype)
+    r, i, x, lam = make_gate_inputs(wide, "cuda", seed=3)
+    lam = lam[8:].clone()
+    r, i, x = (t[:, :, 8:] for t in (r, i, x))
+    g = torch.randn(B, T, D, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").to(r.dtype)
+    h = native.scan_forward_gated(r, i, x, lam)
+    got = native.scan_backward_gated(r, i, x, lam, h, g)
+    alpha, _ = native.gates_forward(r, None, None, lam, want_beta=False)
+    ref = native.gates_backward(r, i, x, lam, *native._backward(alpha, h, g, r.dtype))
+    pkg.check_status()
+    for a, b, name in zip(got, ref, "r i x lam".split()):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        err = float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+        assert err <= (2.0 ** -7 if dtype == "bf16" else 1e-5), (name, err)
+
+
 def test_gated_scan_state():
     """Boundary state of the gated entry point through the C ABI."""
     pkg, native, _ = _mods()

@@ -39,10 +39,12 @@ template <> struct Gate<bf16> {
         asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(z));
         return r;
     }
-    static __device__ __forceinline__ float rroot(float z) {
+    // sqrt(z) and 1/sqrt(z), the latter 0 where there is none, from one special function
+    static __device__ __forceinline__ void roots(float z, float &root, float &inverse) {
         float r;
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
-        return r;
+        inverse = z <= 0.0f ? 0.0f : r;
+        root = z * inverse;
     }
 };
 template <> struct Gate<float> {
@@ -74,10 +76,11 @@ template <> struct Gate<float> {
         asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
         return r;
     }
-    static __device__ __forceinline__ float rroot(float z) {
-        float r;
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(z));
-        return r;
+    // as above, with a square root and a reciprocal of their own: the one-function form costs 2-3 % of the
+    // fp32 gradients' accuracy (dr 3.43e-7 against 3.35e-7 in the 2-norm), this one nothing
+    static __device__ __forceinline__ void roots(float z, float &root_, float &inverse) {
+        root_ = root(z);
+        inverse = root_ > 0.0f ? 1.0f / root_ : 0.0f;
     }
 };
 // alpha of a pair, given the pair of sigmoids, exactly as exp_scaled(scale * sigmoid) gives it

@@ -546,13 +546,14 @@ __device__ __forceinline__ void gated_backward_pair(const Two &r, const Two &g, 
     Two da = mul2(dh, hp);
     if (edge) { ar = splat(edge_alpha); da = splat(0.0f); }
     u = mul2(ar, dh);
-    // q = sqrt(1 - a^2) and 1/q from one reciprocal square root; an alpha that rounds to 1 has no slope
+    // q = sqrt(1 - a^2) and 1/q; an alpha that rounds to 1 has no slope
     const Two na = mul2(a, minus);
-    const Two q2 = fma2(na, a, one);
-    float q2x, q2y;
-    split(q2, q2x, q2y);
-    const Two rq = two(q2x <= 0.0f ? 0.0f : Gate<T>::rroot(q2x), q2y <= 0.0f ? 0.0f : Gate<T>::rroot(q2y));
-    const Two dx = mul2(mul2(dh, mul2(q2, rq)), w);
+    float zx, zy, qx, qy, rqx, rqy;
+    split(fma2(na, a, one), zx, zy);
+    Gate<T>::roots(zx, qx, rqx);
+    Gate<T>::roots(zy, qy, rqy);
+    const Two rq = two(rqx, rqy);
+    const Two dx = mul2(mul2(dh, two(qx, qy)), w);
     const Two ga = fma2(mul2(mul2(dh, rq), mul2(w, x)), na, da);      // beta depends on alpha too
     const Two gs = mul2(mul2(ga, a), s);
     acc = add2(acc, gs);

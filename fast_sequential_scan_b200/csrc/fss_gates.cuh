@@ -89,6 +89,12 @@ template <typename T> __device__ __forceinline__ Two gate_alpha(const Two &scale
     split(mul2(scale, sigmoid), x, y);
     return two(Gate<T>::exp_scaled(x), Gate<T>::exp_scaled(y));
 }
+// beta of a pair, exactly as root(fma(-a, a, 1)) * sigmoid(i) * x gives it
+template <typename T> __device__ __forceinline__ Two gate_beta(const Two &a, const Two &sigmoid, const Two &x) {
+    float p, q;
+    split(fma2(mul2(a, splat(-1.0f)), a, splat(1.0f)), p, q);
+    return mul2(mul2(two(Gate<T>::root(p), Gate<T>::root(q)), sigmoid), x);
+}
 __device__ __forceinline__ float gate_scale(float lambda) {      // -8 * softplus(lambda)
     return -8.0f * (lambda > 20.0f ? lambda : log1pf(expf(lambda)));
 }

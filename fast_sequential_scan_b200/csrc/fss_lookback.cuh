@@ -65,17 +65,16 @@ template <bool kBackward, bool kGate> struct Kind {
     static constexpr int kStages = kGate ? (kBackward ? 5 : 4) : (kBackward ? 4 : 6);
     static constexpr int kTc = kW * kR;                       // rows per tile (times the split)
     static constexpr int kTileBytes = kTc * kRowBytes;        // per tensor and stage
-    // Groups of kW pass-2 warps.  Two groups take units alternately where pass 2 carries the chain
-    // rule of the gates (about 45 instructions and 4 special functions per element).
+    // Groups of kW warps that share the units of a pass: two take them alternately in the pass that
+    // carries the gates' special functions (forward: pass 1; backward: pass 2, with the chain rule).
+    static constexpr int kP1 = kGate && !kBackward ? 2 : 1;
     static constexpr int kP2 = kGate && kBackward ? 2 : 1;
-    static constexpr int kGateWarps = kGate && !kBackward ? kW : 0;
-    // warps [0, kW) run pass 1, the next kP2 * kW pass 2
-    static constexpr int kPass2Warp0 = kW;
-    static constexpr int kProducerWarp = (1 + kP2) * kW;
+    // warps [0, kP1 * kW) run pass 1, the next kP2 * kW pass 2
+    static constexpr int kPass2Warp0 = kP1 * kW;
+    static constexpr int kProducerWarp = (kP1 + kP2) * kW;
     static constexpr int kSummaryWarp = kProducerWarp + 1;
     static constexpr int kLookbackWarp0 = kProducerWarp + 2;
-    static constexpr int kGateWarp0 = kLookbackWarp0 + kLookbackWarps;
-    static constexpr int kThreads = (kGateWarp0 + kGateWarps) * 32;
+    static constexpr int kThreads = (kLookbackWarp0 + kLookbackWarps) * 32;
 };
 // rows per tile of the plain scans, before the split
 constexpr int kTc = Kind<false, false>::kTc;
@@ -341,7 +340,7 @@ template <int kTensors, int kStages, int kTileBytes> struct Smem {
     // summaries: [generation][warp][P|C][lane] as 8-byte (fp32 x2) or 16-byte (fp32 x4) entries
     static constexpr int kAggBytes = kGens * kW * 2 * 32 * 16;
     static constexpr int kSumBytes = kGens * 3 * 32 * 16;      // [generation][tile P | tile C | entering state][lane]
-    static constexpr int kBarriers = 4 * kStages + 4 * kGens;      // full, done, info, gate per stage; agg, carry, sum, lam per generation
+    static constexpr int kBarriers = 3 * kStages + 4 * kGens;      // full, done, info per stage; agg, carry, sum, lam per generation
     static constexpr int kBytes = 128 /* alignment slack */ + kStages * kStageBytes + kAggBytes + kSumBytes +
                                   kBarriers * 8 + 16 + kStages * 16 /* unit descriptors */;
 };
@@ -437,54 +436,6 @@ template <bool kTickets, int kStages> struct UnitCursor {
     __device__ __forceinline__ bool next_known() const { return have && nxt.k >= 0; }
 };
 
-// Gated forward: turns kRh rows (from row `base` of this lane's group) of a stage from (r, x, i) into
-// (alpha, beta) in place, rounded to the I/O type as if they had come from memory.  The odd row
-// group of a 64-byte-row tile reads row r^1 in the slot of row r (see pair_slot); every value goes
-// back to the slot it came from, so nothing has to be swapped here.
-template <typename T, int kRowStride>
-__device__ __forceinline__ void gate_rows(typename Lane<T>::Raw *a_t, typename Lane<T>::Raw *x_t,
-                                          const typename Lane<T>::Raw *i_t, int base, int dsw, bool odd_grp,
-                                          const float (&gsc)[Lane<T>::V], bool head, int nvalid, bool edge_rows) {
-    constexpr int V = Lane<T>::V;
-    using Raw = typename Lane<T>::Raw;
-    Raw ra[kRh], rx[kRh], rg[kRh];
-#pragma unroll
-    for (int r = 0; r < kRh; ++r) {
-        ra[r] = pair_slot<kRowStride>(a_t, base + r, dsw);
-        rx[r] = pair_slot<kRowStride>(x_t, base + r, dsw);
-        rg[r] = pair_slot<kRowStride>(i_t, base + r, dsw);
-    }
-#pragma unroll
-    for (int r = 0; r < kRh; ++r) {
-        float rr[V], ii[V], xx[V], a[V], b[V];
-        Lane<T>::unpack(ra[r], rr);
-        Lane<T>::unpack(rg[r], ii);
-        Lane<T>::unpack(rx[r], xx);
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            a[v] = Gate<T>::exp_scaled(gsc[v] * Gate<T>::sigmoid(rr[v]));
-            b[v] = Gate<T>::root(fmaf(-a[v], a[v], 1.0f)) * Gate<T>::sigmoid(ii[v]) * xx[v];
-        }
-        if (edge_rows) {       // warp-uniform and rare: first row of the sequence, rows after its end
-            const int row = base + (odd_grp ? (r ^ 1) : r);      // the row this register holds
-            const bool first_row = head && row == 0;             // alpha_0 is not part of the recurrence
-            const bool past_end = row >= nvalid;                 // identity rows after the sequence
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                if (first_row) a[v] = 0.0f;
-                if (past_end) { a[v] = 1.0f; b[v] = 0.0f; }
-            }
-        }
-        ra[r] = Lane<T>::pack(a);
-        rx[r] = Lane<T>::pack(b);
-    }
-#pragma unroll
-    for (int r = 0; r < kRh; ++r) {
-        pair_slot<kRowStride>(a_t, base + r, dsw) = ra[r];
-        pair_slot<kRowStride>(x_t, base + r, dsw) = rx[r];
-    }
-}
-
 // TMA descriptors of a launch, in the order of Kind's lists
 template <int kIn, int kOut> struct Maps { CUtensorMap in[kIn], out[kOut]; };
 
@@ -575,7 +526,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
     using K = Kind<kBackward, kGate>;
     constexpr int kR = K::kR, kTileBytes = K::kTileBytes, kStages = K::kStages;
     constexpr int kPass2Warp0 = K::kPass2Warp0, kProducerWarp = K::kProducerWarp, kSummaryWarp = K::kSummaryWarp;
-    constexpr int kLookbackWarp0 = K::kLookbackWarp0, kGateWarp0 = K::kGateWarp0;
+    constexpr int kLookbackWarp0 = K::kLookbackWarp0;
     constexpr bool kGateBwd = kGate && kBackward;
     using SM = Smem<K::kIn, kStages, kTileBytes>;
     constexpr int V = Cfg<T>::V;
@@ -598,7 +549,6 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
     Unit *units = reinterpret_cast<Unit *>(smem_raw + kStages * SM::kStageBytes + SM::kAggBytes + SM::kSumBytes +
                                            SM::kBarriers * 8 + 16);
     auto bar_info = [&](int s) { return bars + 8u * (2 * kStages + 4 * kGens + s); };
-    auto bar_gate = [&](int s) { return bars + 8u * (3 * kStages + 4 * kGens + s); };
     auto bar_lam = [&](int g) { return bars + 8u * (2 * kStages + 3 * kGens + g); };
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_done = [&](int s) { return bars + 8u * (kStages + s); };
@@ -628,7 +578,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(bar_full(s), 1); mbar_init(bar_done(s), kW); mbar_init(bar_info(s), 1); mbar_init(bar_gate(s), kW);
+            mbar_init(bar_full(s), 1); mbar_init(bar_done(s), kW); mbar_init(bar_info(s), 1);
         }
         for (int g = 0; g < kGens; ++g) { mbar_init(bar_agg(g), kW); mbar_init(bar_carry(g), 1); mbar_init(bar_sum(g), 1); mbar_init(bar_lam(g), kW); }
         *cta_abort = 0;
@@ -836,56 +786,6 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 }
             }
         }
-    } else if (kGate && !kBackward && warp >= kGateWarp0) {
-        // ============================================================ gates (gated forward only)
-        // The alpha slot of a stage arrives holding r, the third slot i, the beta slot x.  These
-        // warps turn them into alpha and beta in place as soon as the tile has landed, one warp per
-        // row-group mapping of the pass-1 warps, so that the special-function work runs beside the
-        // scan instead of inside it.  (Measured on the c4 shape, bf16: gates inside pass 1 0.44 ms,
-        // here 0.40 ms; giving half of the rows back to the pass-1 warps 0.61 ms.)
-        using Raw = typename Lane<T>::Raw;
-        constexpr int kRowStride = kRowB / (int)sizeof(Raw);
-        const int gw = warp - kGateWarp0;
-        const int grp = q * kW + gw;
-        constexpr bool kPairSwap = kRowB == 64;
-        const bool odd_grp = kPairSwap && (q & 1);
-        const int dsw = odd_grp ? kRowStride : 0;
-        const uint32_t lane_off = (uint32_t)(grp * kR) * kRowB + (uint32_t)cl * kLaneBytes;
-        Cursor cursor(p, ctl, units, bar_info(0));
-        cursor.init(u0, 0, 1);
-        // this lane's channel scales (a table made once per launch), always fetched one unit ahead so
-        // that the load's latency never sits between a landed tile and its gates
-        auto load_scales = [&](const Unit &un, float (&out)[V]) {
-            const int64_t dch = (int64_t)un.cg * Dc + cl * V;
-#pragma unroll
-            for (int v = 0; v < V; ++v) out[v] = dch + v < p.D ? __ldg(p.scales + dch + v) : 0.0f;
-        };
-        float gsc_next[V];
-        load_scales(u0, gsc_next);
-#pragma unroll 1
-        for (int i = 0;; ++i) {
-            const int st = i % kStages;
-            if (!cursor.advance(i)) break;
-            const Unit u = cursor.cur;
-            const int32_t row0 = u.template row0<kBackward>(p);
-            const bool head = (row0 == 0) && (grp == 0) && !p.continuation;
-            const int64_t left = p.T - row0 - (int64_t)grp * kR;
-            const int nvalid = left >= kR ? kR : (left > 0 ? (int)left : 0);
-            float gsc[V];
-#pragma unroll
-            for (int v = 0; v < V; ++v) gsc[v] = gsc_next[v];
-            if (cursor.next_known()) load_scales(cursor.nxt, gsc_next);
-            if (!ctl.wait(bar_full(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
-            Raw *a_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + lane_off);
-            Raw *x_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + kTileBytes + lane_off);
-            const Raw *i_t = reinterpret_cast<const Raw *>(smem_raw + st * SM::kStageBytes + 2 * kTileBytes + lane_off);
-            const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
-#pragma unroll 1
-            for (int hb = 0; hb < kR / kRh; ++hb)
-                gate_rows<T, kRowStride>(a_t, x_t, i_t, kRh * hb, dsw, odd_grp, gsc, head, nvalid, edge_rows);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_gate(st));
-        }
     } else if (warp >= kLookbackWarp0) {
         // ============================================================ look-back
         // kLookbackWarps warps share the work units round-robin, so several carry resolutions
@@ -1069,22 +969,23 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         // and leaves (P, C); never waits for a carry, only for the summary buffers to be free.
         using Raw = typename Lane<T>::Raw;
         constexpr int kRowStride = kRowB / (int)sizeof(Raw);
-        const int grp = q * kW + warp;             // this lane's row group inside the tile
+        const int w1 = warp % kW, group1 = K::kP1 > 1 ? warp / kW : 0;
+        const int grp = q * kW + w1;               // this lane's row group inside the tile
         constexpr bool kPairSwap = kRowB == 64;
         const bool odd_grp = kPairSwap && (q & 1);
         const int dsw = odd_grp ? kRowStride : 0;
         const uint32_t lane_off = (uint32_t)(grp * kR) * kRowB + (uint32_t)cl * kLaneBytes;
         Cursor cursor(p, ctl, units, bar_info(0));
-        cursor.init(u0, 0, 1);
+        cursor.init(u0, group1, K::kP1);
         ChannelTable<V, Dc> table{p.scales, p.D, cl * V};
-        if (kGateBwd) table.ahead(cursor);
+        if (kGate) table.ahead(cursor);
 #pragma unroll 1
-        for (int i = 0;; ++i) {
+        for (int i = group1;; i += K::kP1) {
             const int st = i % kStages, g = i % kGens;
             if (!cursor.advance(i)) break;
             const Unit u = cursor.cur;
             float c[V];
-            if (kGateBwd) table.take(cursor, c);
+            if (kGate) table.take(cursor, c);
             const int32_t row0 = u.template row0<kBackward>(p);
             const bool head = (row0 == 0) && (grp == 0) && !p.continuation;
             // rows of this group that exist in the sequence (fewer than kR only in the last row block)
@@ -1097,8 +998,6 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             if (!ctl.wait(bar_full(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
             Raw *a_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + lane_off);
             Raw *x_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + kTileBytes + lane_off);
-            // gated forward: the gate warps turn the stage into (alpha, beta), edge rows included
-            if (kGate && !kBackward && !ctl.wait(bar_gate(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
             // row 0 of the whole sequence: alpha_0 is not part of the recurrence
             if (!kGate && head) a_t[0] = Lane<T>::zero();
             // rows past the end of the sequence arrive zero-filled; alpha = 1 (beta, grad = 0) makes
@@ -1110,42 +1009,78 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             float P[V], C[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) { P[v] = 1.0f; C[v] = 0.0f; }
-            if constexpr (kGateBwd) {
+            if constexpr (kGate) {
+                // The gates are part of this pass, which two groups of warps share (gates in four warps of
+                // their own, before four pass-1 warps: 300 us at B16 T4096 D2560 bf16, so 229 us = 5.9 TB/s).
+                // Forward: (r, x) of a row become (alpha, beta) in place,
+                // rounded as if they had come from memory, and are scanned; backward: alpha is made again
+                // for the summary and r stays.
                 constexpr int kPairs = V / 2;
-                constexpr int kGateRows1 = 2;      // (as kGateRows2 below: 1 row 466 us, 4 rows 514 us with two in pass 2)
+                // Rows per loop body: longer bodies wait for instructions, shorter ones for their operands.
+                // B16 T4096 D2560 bf16: forward 268 / 248 / 229 us with 1 / 2 / 4 rows, backward 466 / 456 us
+                // with 1 / 2 and 514 us with 4 (its pass 2 at one row and at two).
+                constexpr int kRows = kBackward ? 2 : 4;
+                const Raw *i_t = x_t + kTileBytes / (int)sizeof(Raw);
                 const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
                 Two scale[kPairs], P2[kPairs], C2[kPairs];
 #pragma unroll
                 for (int v = 0; v < kPairs; ++v) {
-                    scale[v] = two(Gate<T>::prescale(c[2 * v]), Gate<T>::prescale(c[2 * v + 1]));
+                    scale[v] = kBackward ? two(Gate<T>::prescale(c[2 * v]), Gate<T>::prescale(c[2 * v + 1])) : two(c[2 * v], c[2 * v + 1]);
                     P2[v] = splat(1.0f);
                     C2[v] = splat(0.0f);
                 }
 #pragma unroll 1
-                for (int base = kR - kGateRows1; base >= 0; base -= kGateRows1) {
-                    Raw ra[kGateRows1], rx[kGateRows1];
+                for (int b0 = 0; b0 < kR; b0 += kRows) {
+                    const int base = kBackward ? kR - kRows - b0 : b0;
+                    Raw ra[kRows], rx[kRows], ri[kRows];
 #pragma unroll
-                    for (int r = 0; r < kGateRows1; ++r) {
+                    for (int r = 0; r < kRows; ++r) {
                         ra[r] = pair_slot<kRowStride>(a_t, base + r, dsw);
                         rx[r] = pair_slot<kRowStride>(x_t, base + r, dsw);
+                        if (!kBackward) ri[r] = pair_slot<kRowStride>(i_t, base + r, dsw);
                     }
                     pair_fix<kPairSwap>(ra, odd_grp);
                     pair_fix<kPairSwap>(rx, odd_grp);
+                    if (!kBackward) pair_fix<kPairSwap>(ri, odd_grp);
 #pragma unroll
-                    for (int j = 0; j < kGateRows1; ++j) {
-                        const int r = kGateRows1 - 1 - j;
-                        Two xr[kPairs], xg[kPairs];
+                    for (int j = 0; j < kRows; ++j) {
+                        const int r = kBackward ? kRows - 1 - j : j;
+                        Two xr[kPairs], xx[kPairs], xi[kPairs];
                         Lane<T>::unpack(ra[r], xr);
-                        Lane<T>::unpack(rx[r], xg);
+                        Lane<T>::unpack(rx[r], xx);
+                        if (!kBackward) Lane<T>::unpack(ri[r], xi);
 #pragma unroll
-                        for (int v = 0; v < kPairs; ++v) {      // alpha rounded as the forward rounded it
-                            Two a = Lane<T>::rounded(gate_alpha<T>(scale[v], Gate<T>::sigmoid(xr[v])));
-                            if (edge_rows) {
-                                if (head && base + r == 0) a = splat(0.0f);
-                                else if (base + r >= nvalid) a = splat(1.0f);
+                        for (int v = 0; v < kPairs; ++v) {
+                            Two a = gate_alpha<T>(scale[v], Gate<T>::sigmoid(xr[v]));
+                            if constexpr (kBackward) {
+                                a = Lane<T>::rounded(a);
+                                if (edge_rows) {
+                                    if (head && base + r == 0) a = splat(0.0f);        // alpha_0 is not part of the recurrence
+                                    else if (base + r >= nvalid) a = splat(1.0f);      // identity rows after the sequence
+                                }
+                                C2[v] = mul2(a, add2(xx[v], C2[v]));
+                            } else {
+                                Two b = gate_beta<T>(a, Gate<T>::sigmoid(xi[v]), xx[v]);
+                                if (edge_rows) {
+                                    if (head && base + r == 0) a = splat(0.0f);
+                                    else if (base + r >= nvalid) { a = splat(1.0f); b = splat(0.0f); }
+                                }
+                                xr[v] = a;
+                                xx[v] = b;
+                                a = Lane<T>::rounded(a);
+                                C2[v] = fma2(a, C2[v], Lane<T>::rounded(b));
                             }
-                            C2[v] = mul2(a, add2(xg[v], C2[v]));
                             P2[v] = mul2(P2[v], a);
+                        }
+                        if (!kBackward) { ra[r] = Lane<T>::pack(xr); rx[r] = Lane<T>::pack(xx); }
+                    }
+                    if (!kBackward) {
+                        pair_fix<kPairSwap>(ra, odd_grp);
+                        pair_fix<kPairSwap>(rx, odd_grp);
+#pragma unroll
+                        for (int r = 0; r < kRows; ++r) {
+                            pair_slot<kRowStride>(a_t, base + r, dsw) = ra[r];
+                            pair_slot<kRowStride>(x_t, base + r, dsw) = rx[r];
                         }
                     }
                 }
@@ -1156,7 +1091,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 }
             }
 #pragma unroll 1
-            for (int hb = 0; hb < (kGateBwd ? 0 : kR / kRh); ++hb) {
+            for (int hb = 0; hb < (kGate ? 0 : kR / kRh); ++hb) {
                 const int base = kBackward ? kR - kRh * (hb + 1) : kRh * hb;     // rows of this batch
                 Raw ra[kRh], rx[kRh];
 #pragma unroll
@@ -1183,8 +1118,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             VecF vp, vc;
 #pragma unroll
             for (int v = 0; v < V; ++v) { vec_set(vp, v, P[v]); vec_set(vc, v, C[v]); }
-            agg_at(g, warp, 0, lane) = vp;
-            agg_at(g, warp, 1, lane) = vc;
+            agg_at(g, w1, 0, lane) = vp;
+            agg_at(g, w1, 1, lane) = vc;
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_agg(g));
         }

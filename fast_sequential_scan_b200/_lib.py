@@ -18,6 +18,7 @@ ALGO_AUTO, ALGO_CHUNKED, ALGO_LOOKBACK = 0, 1, 2
 FLAG_CONTINUATION = 1
 FLAG_DETERMINISTIC = 2
 FLAG_HOLD_DEPENDENTS = 4
+FLAG_REVERSE = 8
 E_LAYOUT = -5      # FSS_E_LAYOUT
 FLAG_TEST_SHORT_WAITS, FLAG_TEST_MUTE_FIRST_BLOCK = 0x100, 0x200
 

@@ -113,6 +113,13 @@ static int launch_check(const char *what) {
 }
 
 // ------------------------------------------------------------------ chunked path
+// The view the chunked kernels walk: for a reversed scan the same rows from the last to the first.
+template <typename T> static View<T> scan_order(const fss_scan_ctx *ctx, const fss_view *v, int64_t Tn) {
+    View<T> w = make_view<T>(v);
+    if (ctx->flags & FSS_FLAG_REVERSE) { w.ptr += (Tn - 1) * w.st; w.st = -w.st; }
+    return w;
+}
+
 template <typename T, int V>
 static int chunked_forward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64_t D,
                            const fss_view *alpha, const fss_view *beta, const fss_view *h,
@@ -125,9 +132,9 @@ static int chunked_forward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64
     const bool cont = ctx->flags & FSS_FLAG_CONTINUATION;
     if (!chunked::grid_fits(g)) return FSS_E_SHAPE;
     const unsigned blocks = (unsigned)(g.vblocks * g.S * B);
-    auto a = make_view<const T>(alpha);
-    auto b = make_view<const T>(beta);
-    auto out = make_view<T>(h);
+    auto a = scan_order<const T>(ctx, alpha, Tn);
+    auto b = scan_order<const T>(ctx, beta, Tn);
+    auto out = scan_order<T>(ctx, h, Tn);
     chunk_summary<T, V, false><<<blocks, kThreads, 0, stream>>>(g, a, b, wsP, wsC, cont);
     const int64_t cols = B * D;
     chunk_compose<false><<<(unsigned)ceil_div(cols, 128), 128, 0, stream>>>(
@@ -150,16 +157,16 @@ static int chunked_backward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int6
     const bool cont = ctx->flags & FSS_FLAG_CONTINUATION;
     if (!chunked::grid_fits(g)) return FSS_E_SHAPE;
     const unsigned blocks = (unsigned)(g.vblocks * g.S * B);
-    auto a = make_view<const T>(alpha);
-    auto hh = make_view<const T>(h);
-    auto gr = make_view<const T>(grad);
+    auto a = scan_order<const T>(ctx, alpha, Tn);
+    auto hh = scan_order<const T>(ctx, h, Tn);
+    auto gr = scan_order<const T>(ctx, grad, Tn);
     chunk_summary<T, V, true><<<blocks, kThreads, 0, stream>>>(g, a, gr, wsP, wsC, cont);
     const int64_t cols = B * D;
     chunk_compose<true><<<(unsigned)ceil_div(cols, 128), 128, 0, stream>>>(
         g, wsP, wsC, st ? st->u_in : nullptr, st ? st->u_out : nullptr, nullptr,
         st ? st->block_prod : nullptr, st ? st->block_state : nullptr);
     chunk_scan_backward<T, V><<<blocks, kThreads, 0, stream>>>(
-        g, a, hh, gr, make_view<T>(dalpha), make_view<T>(dbeta), wsC,
+        g, a, hh, gr, scan_order<T>(ctx, dalpha, Tn), scan_order<T>(ctx, dbeta, Tn), wsC,
         (st && cont) ? st->h_prev : nullptr, cont);
     return launch_check("chunked backward launch");
 }
@@ -279,6 +286,7 @@ FSS_API int fss_scan_forward_ex(const fss_scan_ctx *ctx, int dtype, int64_t B, i
     if ((rc = check_view(alpha, B, T, D)) || (rc = check_view(beta, B, T, D)) || (rc = check_view(h, B, T, D)))
         return rc;
     if (same_start(h, alpha) || same_start(h, beta)) return FSS_E_ALIAS;
+    if ((ctx->flags & FSS_FLAG_REVERSE) && state && (state->prod || state->block_prod || state->block_state)) return FSS_E_ARGS;
     if ((rc = check_chunked_grid(ctx, B, T, D))) return rc;
     if ((rc = need_workspace(ctx, B, T, D, dtype))) return rc;
     DeviceGuard guard(ctx->device);
@@ -299,7 +307,7 @@ FSS_API int fss_scan_forward_gated(const fss_scan_ctx *ctx, int dtype, int64_t B
     for (const fss_view *v : {r, i, x, h})
         if ((rc = check_view(v, B, T, D))) return rc;
     if (same_start(h, r) || same_start(h, i) || same_start(h, x)) return FSS_E_ALIAS;
-    if (state && (state->prod || state->block_prod || state->block_state)) return FSS_E_ARGS;
+    if ((ctx->flags & FSS_FLAG_REVERSE) || (state && (state->prod || state->block_prod || state->block_state))) return FSS_E_ARGS;
     if (ctx->algo == FSS_ALGO_CHUNKED) return FSS_E_LAYOUT;       // single-pass kernel only
     if (state && !lookback::state_aligned({state->h_in, state->h_last})) return FSS_E_LAYOUT;
     if ((rc = need_workspace(ctx, B, T, D, dtype))) return rc;
@@ -328,6 +336,7 @@ FSS_API int fss_scan_backward_ex(const fss_scan_ctx *ctx, int dtype, int64_t B, 
     if (same_start(grad_alpha, alpha) || same_start(grad_alpha, h) || same_start(grad_alpha, grad_out) ||
         same_start(grad_alpha, grad_beta) || same_start(grad_beta, alpha) || same_start(grad_beta, grad_out))
         return FSS_E_ALIAS;
+    if ((ctx->flags & FSS_FLAG_REVERSE) && state && (state->block_prod || state->block_state)) return FSS_E_ARGS;
     if ((rc = check_chunked_grid(ctx, B, T, D))) return rc;
     if ((rc = need_workspace(ctx, B, T, D, dtype))) return rc;
     DeviceGuard guard(ctx->device);
@@ -797,7 +806,7 @@ FSS_API int fss_scan_backward_gated(const fss_scan_ctx *ctx, int dtype, int64_t 
         for (const fss_view *v : in)
             if (same_start(o, v)) return FSS_E_ALIAS;
     if (same_start(grad_r, grad_i) || same_start(grad_r, grad_x) || same_start(grad_i, grad_x)) return FSS_E_ALIAS;
-    if (ctx->flags & FSS_FLAG_CONTINUATION) return FSS_E_ARGS;
+    if (ctx->flags & (FSS_FLAG_CONTINUATION | FSS_FLAG_REVERSE)) return FSS_E_ARGS;
     // the limit of fss_gates_backward, which does this work for other layouts: alignment alone does not
     // decide whether a problem is accepted
     if (!gate_grid_ok(B, T)) return FSS_E_SHAPE;

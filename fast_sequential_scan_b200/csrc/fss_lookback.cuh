@@ -5,7 +5,7 @@
 // 128 x 128 / 256 x 64 when the problem has too few columns to fill the GPU otherwise (kSp = 2 / 4).
 // (The gated backward, which loads five tensors, has tiles of half as many rows.)
 // Tiles are numbered row-block-major (all columns of the first row block, then the next ...; the
-// backward numbers row blocks from the end), CTA c of G takes tiles c, c+G, c+2G... so a tile only
+// scans that run from the last row number row blocks from the end), CTA c of G takes tiles c, c+G, c+2G... so a tile only
 // ever depends on tiles with smaller numbers, which are always resident or done.
 //
 // A CTA (12 warps, one per SM) runs five roles, coupled only by shared-memory mbarriers:
@@ -349,8 +349,8 @@ template <int kTensors, int kStages, int kTileBytes> struct Smem {
 // stage): tile number, row block in processing order, batch row, channel group.  k < 0 ends the CTA.
 struct Unit {
     int32_t k, s, b, cg;
-    template <bool kBackward> __device__ __forceinline__ int32_t row0(const Params &p) const {
-        return (kBackward ? ((int32_t)p.S - 1 - s) : s) * p.tile_rows;
+    template <bool kDown> __device__ __forceinline__ int32_t row0(const Params &p) const {
+        return (kDown ? ((int32_t)p.S - 1 - s) : s) * p.tile_rows;
     }
 };
 __device__ __forceinline__ Unit unit_of_tile(const Params &p, int64_t tile) {
@@ -519,10 +519,14 @@ __device__ __forceinline__ void gated_backward_pair(const Two &r, const Two &g, 
 // dalpha from h's slot.  Gated backward: (r, grad, h shifted, i, x); dr, di, dx are stored from the
 // slots of r, i, x.  Results are written in place in shared memory and leave through TMA
 // stores issued by the producer, so the consumer warps never stall on the global write path.
-template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false>
+// kReverse: the sequence runs from its last row to its first (h_t = a_t * h_{t+1} + b_t, and the
+// backward the other way), so "first row" is row T-1 and the backward pairs row t with h_{t+1}.
+template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false, bool kReverse = false>
 __global__ void __launch_bounds__(Kind<kBackward, kGate>::kThreads, 1)
 scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBackward, kGate>::kOut> maps, const Params p) {
-    static_assert(!(kGate && !kBackward && kTickets), "the gated forward keeps the fixed tile order");
+    static_assert(!((kGate || kReverse) && !kBackward && kTickets), "these forwards keep the fixed tile order");
+    static_assert(!(kGate && kReverse), "the gated scan has no reversed form");
+    constexpr bool kDown = kBackward != kReverse;      // rows are processed from the last to the first
     using K = Kind<kBackward, kGate>;
     constexpr int kR = K::kR, kTileBytes = K::kTileBytes, kStages = K::kStages;
     constexpr int kPass2Warp0 = K::kPass2Warp0, kProducerWarp = K::kProducerWarp, kSummaryWarp = K::kSummaryWarp;
@@ -643,11 +647,11 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 if (kTickets && next > p.n_fixed) mbar_arrive(bar_info(st));   // the other roles compute the first n_fixed
                 if (nu.k < 0) return;
                 const uint32_t base = smem_base + st * SM::kStageBytes;
-                const int32_t c0 = nu.cg * Dc, c1 = nu.template row0<kBackward>(p), c2 = nu.b;
+                const int32_t c0 = nu.cg * Dc, c1 = nu.template row0<kDown>(p), c2 = nu.b;
                 mbar_arrive_expect_tx(bar_full(st), SM::kStageBytes);
 #pragma unroll
-                for (int j = 0; j < K::kIn; ++j)      // the backward's third tensor is h, one row up
-                    tma_load_3d(base + j * kTileBytes, &maps.in[j], bar_full(st), c0, kBackward && j == 2 ? c1 - 1 : c1, c2);
+                for (int j = 0; j < K::kIn; ++j)      // the backward's third tensor is h, one row earlier in the scan
+                    tma_load_3d(base + j * kTileBytes, &maps.in[j], bar_full(st), c0, kBackward && j == 2 ? c1 + (kReverse ? 1 : -1) : c1, c2);
                 ++issued;
             };
             // One loop for both the initial fill (slots 0 .. kStages-1) and the steady state, in which
@@ -660,7 +664,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 prepare();                            // for slot i + kStages, which lives in this stage
                 if (i >= 0) {
                     const Unit u = units[st];
-                    const int32_t c0 = u.cg * Dc, c1 = u.template row0<kBackward>(p), c2 = u.b;
+                    const int32_t c0 = u.cg * Dc, c1 = u.template row0<kDown>(p), c2 = u.b;
                     if (!ctl.wait(bar_done(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
                     if constexpr (kGateBwd) {
                         tma_store_3d(&maps.out[0], base, c0, c1, c2);                       // dr
@@ -721,7 +725,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             for (int v = 0; v < V; ++v) { iP[v] = 1.0f; iC[v] = 0.0f; }
 #pragma unroll
             for (int ww = 0; ww < kW; ++ww) {
-                const int w = kBackward ? kW - 1 - ww : ww;
+                const int w = kDown ? kW - 1 - ww : ww;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     iC[v] = fmaf(vec_get(own_p[w], v), iC[v], vec_get(own_c[w], v));
@@ -730,8 +734,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             }
 #pragma unroll
             for (int d = 1; d < kSp; d <<= 1) {
-                const bool valid = kBackward ? (q + d < kSp) : (q >= d);
-                const int src = (kBackward ? lane + d * LPG : lane - d * LPG) & 31;
+                const bool valid = kDown ? (q + d < kSp) : (q >= d);
+                const int src = (kDown ? lane + d * LPG : lane - d * LPG) & 31;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     const float oP = __shfl_sync(0xffffffffu, iP[v], src);
@@ -741,9 +745,9 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             }
             float pc[2 * V], run[2 * V];                  // tile summary; map of the groups before this lane's
             {
-                const bool has_prev = kBackward ? (q + 1 < kSp) : (q >= 1);
-                const int prev = (kBackward ? lane + LPG : lane - LPG) & 31;
-                const int last = (kBackward ? 0 : kSp - 1) * LPG + cl;      // lane group that ends the tile
+                const bool has_prev = kDown ? (q + 1 < kSp) : (q >= 1);
+                const int prev = (kDown ? lane + LPG : lane - LPG) & 31;
+                const int last = (kDown ? 0 : kSp - 1) * LPG + cl;      // lane group that ends the tile
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     const float eP = kSp > 1 ? __shfl_sync(0xffffffffu, iP[v], prev) : 1.0f;
@@ -756,7 +760,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             }
 #pragma unroll
             for (int ww = 0; ww < kW; ++ww) {
-                const int w = kBackward ? kW - 1 - ww : ww;
+                const int w = kDown ? kW - 1 - ww : ww;
                 VecF ep, ec;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
@@ -781,7 +785,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             if (p.block_prod && q == 0) {
                 const int64_t dch = (int64_t)u.cg * Dc + cl * V;
                 if (dch < p.D) {
-                    const int64_t blk = kBackward ? (p.S - 1 - it_s) : it_s;
+                    const int64_t blk = kDown ? (p.S - 1 - it_s) : it_s;
                     *reinterpret_cast<VecF *>(p.block_prod + ((int64_t)u.b * p.S + blk) * p.D + dch) = sp;
                 }
             }
@@ -956,7 +960,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
 #pragma unroll
                 for (int v = 0; v < V; ++v) vec_set(vo, v, out[v]);
                 if (p.block_state) {
-                    const int64_t blk = kBackward ? (p.S - 1 - s) : s;
+                    const int64_t blk = kDown ? (p.S - 1 - s) : s;
                     *reinterpret_cast<VecF *>(p.block_state + ((int64_t)b * p.S + blk) * p.D + dch) = vo;
                 }
                 if (s + 1 == (int32_t)p.S && p.state_out)
@@ -986,11 +990,11 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             const Unit u = cursor.cur;
             float c[V];
             if (kGate) table.take(cursor, c);
-            const int32_t row0 = u.template row0<kBackward>(p);
-            const bool head = (row0 == 0) && (grp == 0) && !p.continuation;
+            const int32_t row0 = u.template row0<kDown>(p);
             // rows of this group that exist in the sequence (fewer than kR only in the last row block)
             const int64_t left = p.T - row0 - (int64_t)grp * kR;
             const int nvalid = left >= kR ? kR : (left > 0 ? (int)left : 0);
+            const bool head = (kReverse ? left > 0 && left <= kR : row0 == 0 && grp == 0) && !p.continuation;
             if (i >= kGens) {      // the summary buffers of this generation are free once pass 2 of unit i-kGens is done
                 const int o = i - kGens;
                 if (!ctl.wait(bar_done((int)(o % kStages)), (uint32_t)((o / kStages) & 1), FSS_STATUS_LOOKBACK_TIMEOUT)) break;
@@ -998,8 +1002,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             if (!ctl.wait(bar_full(st), (uint32_t)((i / kStages) & 1), FSS_STATUS_TMA_TIMEOUT)) break;
             Raw *a_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + lane_off);
             Raw *x_t = reinterpret_cast<Raw *>(smem_raw + st * SM::kStageBytes + kTileBytes + lane_off);
-            // row 0 of the whole sequence: alpha_0 is not part of the recurrence
-            if (!kGate && head) a_t[0] = Lane<T>::zero();
+            // first row of the whole sequence: its alpha is not part of the recurrence
+            if (!kGate && head) a_t[(kReverse ? nvalid - 1 : 0) * kRowStride] = Lane<T>::zero();
             // rows past the end of the sequence arrive zero-filled; alpha = 1 (beta, grad = 0) makes
             // them the identity for both passes, so the state after the tile is the state after
             // the last real row
@@ -1092,7 +1096,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             }
 #pragma unroll 1
             for (int hb = 0; hb < (kGate ? 0 : kR / kRh); ++hb) {
-                const int base = kBackward ? kR - kRh * (hb + 1) : kRh * hb;     // rows of this batch
+                const int base = kDown ? kR - kRh * (hb + 1) : kRh * hb;     // rows of this batch
                 Raw ra[kRh], rx[kRh];
 #pragma unroll
                 for (int r = 0; r < kRh; ++r) {
@@ -1103,7 +1107,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 pair_fix<kPairSwap>(rx, odd_grp);
 #pragma unroll
                 for (int j = 0; j < kRh; ++j) {
-                    const int r = kBackward ? kRh - 1 - j : j;
+                    const int r = kDown ? kRh - 1 - j : j;
                     float a[V], x[V];
                     Lane<T>::unpack(ra[r], a);
                     Lane<T>::unpack(rx[r], x);
@@ -1147,7 +1151,9 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             const Unit u = cursor.cur;
             float c[V];
             if (kGateBwd) table.take(cursor, c);
-            const bool head = (u.template row0<kBackward>(p) == 0) && (grp == 0);
+            const int64_t left = p.T - u.template row0<kDown>(p) - (int64_t)grp * kR;      // rows up to the sequence's end
+            const bool head = kReverse ? left > 0 && left <= kR : u.template row0<kDown>(p) == 0 && grp == 0;
+            const int head_row = kReverse ? (int)left - 1 : 0;      // the first row's place in its group
             const int32_t b = u.b;
             const int64_t dch = (int64_t)u.cg * Dc + ch;
             const Raw *a_t = reinterpret_cast<const Raw *>(smem_raw + st * SM::kStageBytes + lane_off);
@@ -1168,7 +1174,6 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 // longer bodies they wait for instructions: 4 rows 565 us, 2 rows 494 us, 1 row 456 us (c4
                 // shape, bf16).  The row pairs of 64-byte tile rows need two.
                 constexpr int kGateRows2 = kPairSwap ? 2 : 1;
-                const int64_t left = p.T - u.template row0<kBackward>(p) - (int64_t)grp * kR;
                 const int nvalid = left >= kR ? kR : (left > 0 ? (int)left : 0);
                 const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
                 Raw *r_t = const_cast<Raw *>(a_t);
@@ -1270,7 +1275,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             }
 #pragma unroll 1
             for (int hb = 0; hb < kR / kRh; ++hb) {
-                const int base = kBackward ? kR - kRh * (hb + 1) : kRh * hb;
+                const int base = kDown ? kR - kRh * (hb + 1) : kRh * hb;
                 Raw ra[kRh], rx[kRh];
 #pragma unroll
                 for (int r = 0; r < kRh; ++r) {
@@ -1281,7 +1286,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 pair_fix<kPairSwap>(rx, odd_grp);
                 if (!kBackward) {
 #pragma unroll
-                    for (int r = 0; r < kRh; ++r) {
+                    for (int j = 0; j < kRh; ++j) {
+                        const int r = kDown ? kRh - 1 - j : j;
                         float a[V], x[V];
                         Lane<T>::unpack(ra[r], a);
                         Lane<T>::unpack(rx[r], x);
@@ -1300,15 +1306,17 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
 #pragma unroll
                     for (int r = 0; r < kRh; ++r) rh[r] = pair_slot<kRowStride>(h_t, base + r, dsw);
                     pair_fix<kPairSwap>(rh, odd_grp);
-                    if (base == 0 && head && p.continuation && p.h_prev) {    // h_{-1} of a continued sequence
+                    if ((kReverse || base == 0) && head && p.continuation && p.h_prev) {    // the state before the first row
                         float hp[V];
 #pragma unroll
                         for (int v = 0; v < V; ++v) hp[v] = (dch < p.D) ? p.h_prev[(int64_t)b * p.D + dch + v] : 0.0f;
-                        rh[0] = Lane<T>::pack(hp);
+#pragma unroll
+                        for (int r = 0; r < (kReverse ? kRh : 1); ++r)
+                            if (base + r == head_row) rh[r] = Lane<T>::pack(hp);
                     }
 #pragma unroll
                     for (int j = 0; j < kRh; ++j) {
-                        const int r = kRh - 1 - j;
+                        const int r = kDown ? kRh - 1 - j : j;
                         float a[V], x[V], hp[V], da[V], dh[V];
                         Lane<T>::unpack(ra[r], a);
                         Lane<T>::unpack(rx[r], x);
@@ -1319,7 +1327,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                             da[v] = dh[v] * hp[v];
                             stv[v] = a[v] * dh[v];
                         }
-                        if (base + r == 0 && head && !p.continuation) {
+                        if (base + r == head_row && head && !p.continuation) {
 #pragma unroll
                             for (int v = 0; v < V; ++v) da[v] = 0.0f;
                         }
@@ -1515,14 +1523,14 @@ inline const CUtensorMap *cached_map(const fss_view *v, int64_t B, int64_t Tn, i
 }
 
 // CTAs that fit the device at once (one per SM with these shared-memory sizes), per device.
-template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate> inline int resident_ctas(int device, int smem_bytes, cudaError_t *err) {
+template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate, bool kReverse> inline int resident_ctas(int device, int smem_bytes, cudaError_t *err) {
     static std::mutex mu;
     static int cached[64];
     static bool have[64];
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0 || device >= 64) { *err = cudaErrorInvalidDevice; return 0; }
     if (!have[device]) {
-        auto kern = scan_kernel<T, kBackward, kSp, kTickets, kGate>;
+        auto kern = scan_kernel<T, kBackward, kSp, kTickets, kGate, kReverse>;
         *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (*err != cudaSuccess) return 0;
         int per_sm = 0, sms = 0;
@@ -1538,7 +1546,7 @@ template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate> inline
 }
 
 // `in`, `out`: the views in the order of Kind's lists
-template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false>
+template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false, bool kReverse = false>
 inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D,
                         std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p, int tail,
                         std::string *err_text) {
@@ -1564,7 +1572,7 @@ inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, in
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return FSS_E_DEVICE; }
-    const int resident = resident_ctas<T, kBackward, kSp, kTickets, kGate>(device, smem_bytes, &e);
+    const int resident = resident_ctas<T, kBackward, kSp, kTickets, kGate, kReverse>(device, smem_bytes, &e);
     if (e != cudaSuccess || resident < 1) { *err_text = cudaGetErrorString(e); return FSS_E_LAUNCH; }
 
     p.B = B; p.T = Tn; p.D = D;
@@ -1618,22 +1626,22 @@ inline int launch_split(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, in
     const bool use_pdl = pdl_env >= 0 ? pdl_env == 1 : (!kBackward || p.ntiles <= kPdlMaxUnits * (int64_t)grid);
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, scan_kernel<T, kBackward, kSp, kTickets, kGate>, maps, p);
+    e = cudaLaunchKernelEx(&cfg, scan_kernel<T, kBackward, kSp, kTickets, kGate, kReverse>, maps, p);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { *err_text = std::string("look-back launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     return FSS_OK;
 }
 
-template <typename T, bool kBackward, bool kGate = false>
+template <typename T, bool kBackward, bool kGate = false, bool kReverse = false>
 inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D,
                   std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p,
                   std::string *err_text) {
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
-    constexpr bool kNeverTickets = kGate && !kBackward;
+    constexpr bool kNeverTickets = (kGate || kReverse) && !kBackward;
     const int tail = kNeverTickets ? 0 : choose_tail(dtype, kBackward, B, Tn, D);
 #define FSS_LAUNCH_SPLIT(SP)                                                                                                    \
-    return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
-                    : launch_split<T, kBackward, SP, false, kGate>(ctx, ws, B, Tn, D, in, out, p, 0, err_text)
+    return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
+                    : launch_split<T, kBackward, SP, false, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, 0, err_text)
     switch (choose_split(dtype, B, Tn, D, Kind<kBackward, kGate>::kTc)) {
     case 4: FSS_LAUNCH_SPLIT(4);
     case 2: FSS_LAUNCH_SPLIT(2);
@@ -1719,7 +1727,9 @@ inline int forward(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t
         if (float_scratch_bytes(B, Tn, D) > ws.float_bytes) return FSS_E_WORKSPACE;
         p.block_prod = reinterpret_cast<float *>(ws.floats);
     }
-    const int rc = launch<T, false>(ctx, ws, B, Tn, D, {alpha, beta}, {h}, p, err_text);
+    const bool reverse = ctx->flags & FSS_FLAG_REVERSE;
+    const int rc = reverse ? launch<T, false, false, true>(ctx, ws, B, Tn, D, {alpha, beta}, {h}, p, err_text)
+                           : launch<T, false>(ctx, ws, B, Tn, D, {alpha, beta}, {h}, p, err_text);
     if (rc != FSS_OK || !prod) return rc;
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
     const int64_t S = ceil_div(Tn, block_rows(dtype, B, Tn, D));
@@ -1783,6 +1793,8 @@ inline int backward(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_
         p.block_state = st->block_state;
         p.h_prev = cont ? st->h_prev : nullptr;
     }
+    if (ctx->flags & FSS_FLAG_REVERSE)
+        return launch<T, true, false, true>(ctx, ws, B, Tn, D, {alpha, grad, h}, {dalpha, dbeta}, p, err_text);
     return launch<T, true>(ctx, ws, B, Tn, D, {alpha, grad, h}, {dalpha, dbeta}, p, err_text);
 }
 

@@ -32,8 +32,8 @@ sequential loop, sequential_scan/common.py:51-57, started from ``h0`` instead of
     arrives for it is added to ``dh_{T-1}``.  Feeding it to the next call as ``h0`` continues the
     sequence exactly (chunked prefill, streaming).
 ``reverse``
-    scan from the last row to the first (``h_t = alpha_t * h_{t+1} + beta_t``); done by flipping the
-    tensors around an ordinary scan, so it costs five extra tensor passes.
+    scan from the last row to the first (``h_t = alpha_t * h_{t+1} + beta_t``): the kernels walk the rows
+    in that order, at the cost of an ordinary scan.
 """
 from __future__ import annotations
 
@@ -43,7 +43,7 @@ import torch
 from torch.autograd import Function
 
 from .sequential_scan_cuda import (backward_into, forward_into, scan_backward, scan_backward_gated, scan_backward_half,
-                                   scan_forward, scan_forward_gated, scan_forward_half)
+                                   scan_forward, scan_forward_gated, scan_forward_half, tma_eligible)
 
 BACKWARD_MODES = ("saved", "inplace", "recompute")
 _default_mode = "saved"
@@ -110,6 +110,13 @@ class SequentialScanSingle(Function):
         return _backward(ctx, scan_forward, scan_backward, grad_output)
 
 
+def _addressable(t: torch.Tensor) -> torch.Tensor:
+    """A copy of ``t`` where only its placement, not its width, keeps the single-pass kernels from taking it."""
+    if t.dim() != 3 or t.shape[2] % (16 // t.element_size()) or tma_eligible(t):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
+
+
 class _StatefulScan(Function):
     """The scan with a state entering row 0 and / or the final state returned (and the reversed
     direction).  Inputs: alpha, beta, h0 (or None), flags.  Outputs: h[, h_last]."""
@@ -124,8 +131,7 @@ class _StatefulScan(Function):
         B, T, D = alpha.shape
         if T == 0:
             raise RuntimeError("a scan with boundary state needs at least one row")
-        a = alpha.flip(1) if reverse else alpha
-        b = beta.flip(1) if reverse else beta
+        a, b = (_addressable(alpha), _addressable(beta)) if reverse else (alpha, beta)
         state = None
         if h0 is not None:
             if h0.shape != (B, D) or h0.device != alpha.device:
@@ -133,25 +139,24 @@ class _StatefulScan(Function):
             state = h0.detach().float().contiguous()
         h = torch.empty(a.shape, dtype=a.dtype, device=a.device)
         h_last = torch.empty(B, D, dtype=torch.float32, device=a.device) if want_final else None
-        forward_into(a, b, h, continuation=state is not None, h_in=state, h_last=h_last)
+        forward_into(a, b, h, continuation=state is not None, h_in=state, h_last=h_last, reverse=reverse)
         ctx.reverse, ctx.has_state, ctx.want_final = reverse, state is not None, want_final
         ctx.h0_dtype = h0.dtype if h0 is not None else None
         ctx.save_for_backward(a, h, state)
-        out = h.flip(1) if reverse else h
-        return (out, h_last) if want_final else out
+        return (h, h_last) if want_final else h
 
     @staticmethod
     def backward(ctx: Any, grad_h: torch.Tensor, grad_last: Optional[torch.Tensor] = None):
         a, h, state = ctx.saved_tensors
         B, T, D = a.shape
-        g = grad_h.flip(1) if ctx.reverse else grad_h
-        g = g.to(a.dtype).contiguous()
+        g = grad_h.to(a.dtype).contiguous()
+        if ctx.reverse:
+            g = _addressable(g)
         u_in = grad_last.float().contiguous() if grad_last is not None else None
         da, db = torch.empty_like(a), torch.empty_like(a)
         u_out = torch.empty(B, D, dtype=torch.float32, device=a.device) if ctx.has_state else None
-        backward_into(a, h, g, da, db, continuation=ctx.has_state, u_in=u_in, h_prev=state, u_out=u_out)
-        if ctx.reverse:
-            da, db = da.flip(1), db.flip(1)
+        backward_into(a, h, g, da, db, continuation=ctx.has_state, u_in=u_in, h_prev=state, u_out=u_out,
+                      reverse=ctx.reverse)
         dh0 = u_out.to(ctx.h0_dtype) if ctx.has_state and ctx.needs_input_grad[2] else None
         return da, db, dh0, None, None
 

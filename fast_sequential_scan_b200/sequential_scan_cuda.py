@@ -152,9 +152,10 @@ def _launch_backward(a, hh, g, grad_alpha, grad_beta, dtype_id: int, algo, flags
 
 
 def forward_into(alpha, beta, h, *, algo=None, continuation=False, h_in=None, h_last=None,
-                 prod=None, block_prod=None, block_state=None, hold_dependents: bool = False,
+                 prod=None, block_prod=None, block_state=None, hold_dependents: bool = False, reverse: bool = False,
                  _extra_flags: int = 0) -> None:
-    """h <- scan(alpha, beta) into a caller-owned tensor, with the optional boundary state.
+    """h <- scan(alpha, beta) into a caller-owned tensor, with the optional boundary state.  ``reverse`` =
+    ``FSS_FLAG_REVERSE``: from the last row to the first.
     ``hold_dependents`` = ``FSS_FLAG_HOLD_DEPENDENTS``: the next launch on the stream is placed only when this
     scan has finished."""
     dtype = alpha.dtype
@@ -174,7 +175,8 @@ def forward_into(alpha, beta, h, *, algo=None, continuation=False, h_in=None, h_
         state = _lib.ForwardState(_vec(h_in, B, D, "h_in"), _vec(h_last, B, D, "h_last"),
                                   _vec(prod, B, D, "prod"), _blocks(block_prod, "block_prod"),
                                   _blocks(block_state, "block_state"))
-    flags = (_lib.FLAG_CONTINUATION if continuation else 0) | (_lib.FLAG_HOLD_DEPENDENTS if hold_dependents else 0)
+    flags = (_lib.FLAG_CONTINUATION if continuation else 0) | (_lib.FLAG_HOLD_DEPENDENTS if hold_dependents else 0) | \
+            (_lib.FLAG_REVERSE if reverse else 0)
     _launch_forward(a, b, h, _DTYPES[dtype], algo, flags | _extra_flags, state)
 
 
@@ -322,9 +324,9 @@ def scan_forward_gated(r, i, x, lam) -> torch.Tensor:
 
 def backward_into(alpha, h, grad_out, grad_alpha, grad_beta, *, algo=None, continuation=False,
                   u_in=None, h_prev=None, u_out=None, block_prod=None, block_state=None,
-                  hold_dependents: bool = False) -> None:
-    """Reverse scan into caller-owned gradient tensors, with the optional boundary state (``hold_dependents``:
-    see :func:`forward_into`)."""
+                  hold_dependents: bool = False, reverse: bool = False) -> None:
+    """Gradients of the scan into caller-owned tensors, with the optional boundary state (``hold_dependents``,
+    ``reverse``: see :func:`forward_into`)."""
     dtype = alpha.dtype
     if dtype not in _DTYPES:
         raise RuntimeError(f"alpha_saved: unsupported dtype {dtype} (bf16 or fp32)")
@@ -347,7 +349,7 @@ def backward_into(alpha, h, grad_out, grad_alpha, grad_beta, *, algo=None, conti
                                    _blocks(block_state, "block_state"))
     _launch_backward(a, hh, g, grad_alpha, grad_beta, _DTYPES[dtype], algo,
                      (_lib.FLAG_CONTINUATION if continuation else 0)
-                     | (_lib.FLAG_HOLD_DEPENDENTS if hold_dependents else 0), state)
+                     | (_lib.FLAG_HOLD_DEPENDENTS if hold_dependents else 0) | (_lib.FLAG_REVERSE if reverse else 0), state)
 
 
 def _forward(alpha: torch.Tensor, beta: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

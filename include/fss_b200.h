@@ -107,6 +107,13 @@ typedef struct fss_scan_ctx {
  * loads, run 5-9 microseconds faster when they are placed on an empty GPU than when their CTAs were
  * parked one by one behind the scan's last tiles; the local scans of a sequence-parallel step set it. */
 #define FSS_FLAG_HOLD_DEPENDENTS 4
+/* For fss_scan_forward_ex / fss_scan_backward_ex: the sequence runs from row T-1 to row 0,
+ *     h_{T-1} = b_{T-1} ;  h_t = a_t * h_{t+1} + b_t ;  dh_0 = g_0 ;  dh_t = g_t + a_{t-1} * dh_{t-1} ;
+ *     da_t = dh_t * h_{t+1} (t < T-1) ;  da_{T-1} = 0.
+ * "First row" then means row T-1 everywhere (FSS_FLAG_CONTINUATION, h_in, h_prev, u_out) and "last
+ * row" row 0 (h_last, u_in).  prod, block_prod and block_state must be NULL (FSS_E_ARGS); the gated
+ * scans have no reversed form (FSS_E_ARGS). */
+#define FSS_FLAG_REVERSE 8
 /* Test hooks for the bounded waits of the single-pass kernels (no effect on results otherwise):
  * SHORT_WAITS lets every wait give up after a few thousand polls instead of ~a second;
  * MUTE_FIRST_BLOCK makes the tiles of the first row block publish no descriptors, so that the

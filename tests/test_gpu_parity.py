@@ -473,6 +473,45 @@ def test_gated_backward_in_one_kernel_matches_the_three_kernels(shape, dtype):
         assert err <= (2.0 ** -7 if dtype == "bf16" else 1e-5), (name, err)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(2, 1, 8), (2, 15, 136), (3, 64, 24), (1, 65, 2056), (2, 300, 136), (5, 1000, 264), (1, 4097, 64),
+                                   (3, 77, 33), (2, 6200, 4104)])
+def test_reverse_is_the_scan_of_the_flipped_rows(shape, dtype):
+    """``reverse`` at the edges of the tiles, of each tile shape and kernel family (odd width: any-layout kernels; the
+    last shape: tickets), with and without boundary state, against the ordinary scan of flipped copies; on the flipped
+    rows the tiles fall elsewhere, so results agree up to association."""
+    _, native, _lib = _mods()
+    B, T, D = shape
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = torch.sigmoid(rnd(B, T, D)).to(dtype)
+    b, g = rnd(B, T, D).to(dtype), rnd(B, T, D).to(dtype)
+    h0, u0 = rnd(B, D), rnd(B, D)
+    for cont in (False, True):
+        out = {}
+        for reverse in (False, True):
+            x, y, z = (t if reverse else t.flip(1).contiguous() for t in (a, b, g))
+            h, da, db = (torch.full_like(x, 7.0) for _ in range(3))
+            last, u = torch.empty(B, D, device="cuda"), torch.empty(B, D, device="cuda")
+            native.forward_into(x, y, h, continuation=cont, h_in=h0 if cont else None, h_last=last, reverse=reverse)
+            native.backward_into(x, out[False][0].flip(1).contiguous() if reverse else h, z, da, db, continuation=cont, u_in=u0,
+                                 h_prev=h0 if cont else None, u_out=u, reverse=reverse)
+            out[reverse] = (h, da, db, last, u)
+        for k, name in enumerate("h da db last u".split()):
+            want, got = out[False][k], out[True][k]
+            if k < 3:
+                want = want.flip(1)
+            # association: a few ulp of the state, relative to its size (|h| <~ 5 here) where terms cancel
+            tol = 2.0 ** -7 if k < 3 and dtype == torch.bfloat16 else 2.0 ** -19
+            bound = tol * (want.float().abs() + 1.0)
+            assert bool(((want.float() - got.float()).abs() <= bound).all()), (name, cont)
+    with pytest.raises(_lib.FssError) as err:
+        native.forward_into(a, b, torch.empty_like(a), reverse=True, prod=torch.empty(B, D, device="cuda"))
+    assert err.value.code == -10
+    import fast_sequential_scan_b200 as pkg
+    pkg.check_status()
+
+
 def test_gated_scan_state():
     """Boundary state of the gated entry point through the C ABI."""
     pkg, native, _ = _mods()

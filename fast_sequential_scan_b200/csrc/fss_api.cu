@@ -9,6 +9,7 @@
 #include "fss_common.cuh"
 #include "fss_gates.cuh"
 #include "fss_lookback.cuh"
+#include "fss_ragged.cuh"
 #include "fss_seqpar.cuh"
 
 #define FSS_API extern "C" __attribute__((visibility("default")))
@@ -171,6 +172,39 @@ static int chunked_backward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int6
     return launch_check("chunked backward launch");
 }
 
+// ------------------------------------------------------------------ any-layout path
+// FSS_ALGO_AUTO takes it where TMA cannot address the tensors and 16-byte accesses do not fit either
+// (with them the chunked kernels move 8 or 4 elements per access; that is left for misaligned state
+// vectors); the callers that want block outputs get the chunked kernels, whose blocks they know.
+template <typename T> static bool ragged_ok(int64_t B, int64_t Tn, int64_t D, std::initializer_list<const fss_view *> views) {
+    return !chunked::vector_ok<T>(D, views) && ragged::fits(B, Tn, D);
+}
+template <typename T>
+static int ragged_forward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64_t D, const fss_view *alpha, const fss_view *beta,
+                          const fss_view *h, const fss_forward_state *st) {
+    ragged::Params p{};
+    p.state_in = st && (ctx->flags & FSS_FLAG_CONTINUATION) ? st->h_in : nullptr;
+    p.state_out = st ? st->h_last : nullptr;
+    const View<const T> a = scan_order<const T>(ctx, alpha, Tn);
+    const View<T> out = scan_order<T>(ctx, h, Tn);
+    return ragged::launch<T, false>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D, a,
+                                    scan_order<const T>(ctx, beta, Tn), a, out, out, p, &g_cuda_error);
+}
+template <typename T>
+static int ragged_backward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64_t D, const fss_view *alpha, const fss_view *h,
+                           const fss_view *grad, const fss_view *dalpha, const fss_view *dbeta, const fss_backward_state *st) {
+    ragged::Params p{};
+    p.state_in = st ? st->u_in : nullptr;
+    p.state_out = st ? st->u_out : nullptr;
+    p.h_prev = st && (ctx->flags & FSS_FLAG_CONTINUATION) ? st->h_prev : nullptr;
+    fss_scan_ctx back = *ctx;      // the backward visits the rows in the other order
+    back.flags ^= FSS_FLAG_REVERSE;
+    return ragged::launch<T, true>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D,
+                                   scan_order<const T>(&back, alpha, Tn), scan_order<const T>(&back, grad, Tn),
+                                   scan_order<const T>(&back, h, Tn), scan_order<T>(&back, dalpha, Tn),
+                                   scan_order<T>(&back, dbeta, Tn), p, &g_cuda_error);
+}
+
 template <typename T>
 static int forward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t Tn, int64_t D,
                          const fss_view *alpha, const fss_view *beta, const fss_view *h,
@@ -184,6 +218,9 @@ static int forward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t 
     }
     if (algo == FSS_ALGO_LOOKBACK)
         return lookback::forward<T>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D, alpha, beta, h, st, &g_cuda_error);
+    if (ctx->algo == FSS_ALGO_AUTO && !(st && (st->prod || st->block_prod || st->block_state)) &&
+        ragged_ok<T>(B, Tn, D, {alpha, beta, h}))
+        return ragged_forward<T>(ctx, B, Tn, D, alpha, beta, h, st);
     constexpr int V = VecWidth<T>::value;
     if (chunked::vector_ok<T>(D, {alpha, beta, h}))
         return chunked_forward<T, V>(ctx, B, Tn, D, alpha, beta, h, st);
@@ -213,6 +250,9 @@ static int backward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t
     if (algo == FSS_ALGO_LOOKBACK)
         return lookback::backward<T>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D, alpha, h, grad,
                                      dalpha, dbeta, st, &g_cuda_error);
+    if (ctx->algo == FSS_ALGO_AUTO && !(st && (st->block_prod || st->block_state)) &&
+        ragged_ok<T>(B, Tn, D, {alpha, h, grad, dalpha, dbeta}))
+        return ragged_backward<T>(ctx, B, Tn, D, alpha, h, grad, dalpha, dbeta, st);
     constexpr int V = VecWidth<T>::value;
     if (chunked::vector_ok<T>(D, {alpha, h, grad, dalpha, dbeta}))
         return chunked_backward<T, V>(ctx, B, Tn, D, alpha, h, grad, dalpha, dbeta, st);
@@ -253,7 +293,9 @@ FSS_API size_t fss_workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype) {
     size_t a = chunked::workspace_bytes(B, T, D);
     size_t b = lookback::workspace_bytes(B, T, D, dtype);
     size_t c = lookback::float_scratch_bytes(B, T, D);
+    size_t d = ragged::fits(B, T, D) ? ragged::workspace_bytes(B, T, D) : 0;
     if (b > a) a = b;
+    if (d > a) a = d;
     return workspace_total(a > c ? a : c);
 }
 

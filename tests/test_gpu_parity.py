@@ -512,6 +512,39 @@ def test_reverse_is_the_scan_of_the_flipped_rows(shape, dtype):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 15, 31), (3, 16, 33), (2, 17, 32), (1, 127, 65), (2, 128, 7), (2, 129, 100), (1, 3000, 45),
+                                   (4, 1000, 1001), (1, 20000, 5)])
+def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
+    """Odd widths and unaligned views at the edges of a tile (128 rows x 32 channels) and of a warp's rows, both scan
+    orders, with and without boundary state; two runs are bit-identical.  ``auto`` takes the any-layout kernel here."""
+    _, native, _ = _mods()
+    B, T, D = shape
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = (0.5 + 0.499 * torch.rand(B, T, D + 3, generator=gen, device="cuda")).to(dtype)[:, :, 1:D + 1]
+    b, g = rnd(B, T, D + 3).to(dtype)[:, :, 2:D + 2], rnd(B, T, D + 3).to(dtype)[:, :, 1:D + 1]
+    h0, u0 = rnd(B, D), rnd(B, D)
+    for cont, reverse in [(False, False), (True, False), (True, True)]:
+        runs = []
+        for algo in ("chunked", "auto", "auto"):
+            wide = [torch.full((B, T, D + 3), 7.0, dtype=dtype, device="cuda") for _ in range(3)]
+            h, da, db = (t[:, :, 1:D + 1] for t in wide)
+            last, u = torch.empty(B, D, device="cuda"), torch.empty(B, D, device="cuda")
+            native.forward_into(a, b, h, algo=_algo_id(algo), continuation=cont, h_in=h0 if cont else None, h_last=last, reverse=reverse)
+            native.backward_into(a, runs[0][0] if runs else h, g, da, db, algo=_algo_id(algo), continuation=cont, u_in=u0,
+                                 h_prev=h0 if cont else None, u_out=u, reverse=reverse)
+            assert all(bool((t[:, :, 0] == 7.0).all()) and bool((t[:, :, D + 1:] == 7.0).all()) for t in wide)
+            runs.append((h, da, db, last, u))
+        for k, name in enumerate("h da db last u".split()):
+            want, got = runs[0][k].float(), runs[1][k].float()
+            tol = 2.0 ** -7 if k < 3 and dtype == torch.bfloat16 else 2.0 ** -18       # |h| <~ 60 at these gates
+            assert bool(((want - got).abs() <= tol * (want.abs() + 4.0)).all()), (name, cont, reverse)
+            assert torch.equal(runs[1][k], runs[2][k]), name
+    import fast_sequential_scan_b200 as pkg
+    pkg.check_status()
+
+
 def test_gated_scan_state():
     """Boundary state of the gated entry point through the C ABI."""
     pkg, native, _ = _mods()

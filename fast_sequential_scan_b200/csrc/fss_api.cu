@@ -5,6 +5,7 @@
 #include <initializer_list>
 #include <string>
 
+#include "fss_brief.cuh"
 #include "fss_chunked.cuh"
 #include "fss_common.cuh"
 #include "fss_gates.cuh"
@@ -205,11 +206,28 @@ static int ragged_backward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64
                                    scan_order<T>(&back, dbeta, Tn), p, &g_cuda_error);
 }
 
+// ------------------------------------------------------------------ a few rows
+template <typename T, int V>
+static int brief_forward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64_t D, const fss_view *alpha, const fss_view *beta,
+                         const fss_view *h, const fss_forward_state *st) {
+    const bool cont = ctx->flags & FSS_FLAG_CONTINUATION;
+    brief::scan_forward<T, V><<<(unsigned)ceil_div(B * (D / V), brief::kThreads), brief::kThreads, 0, (cudaStream_t)ctx->stream>>>(
+        B, (int)Tn, D, scan_order<const T>(ctx, alpha, Tn), scan_order<const T>(ctx, beta, Tn), scan_order<T>(ctx, h, Tn),
+        st && cont ? st->h_in : nullptr, st ? st->h_last : nullptr, cont);
+    return launch_check("short forward launch");
+}
+
 template <typename T>
 static int forward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t Tn, int64_t D,
                          const fss_view *alpha, const fss_view *beta, const fss_view *h,
                          const fss_forward_state *st) {
     int algo = ctx->algo;
+    if (algo == FSS_ALGO_AUTO && Tn <= brief::kMaxRows && !(st && (st->prod || st->block_prod || st->block_state)) &&
+        ceil_div(B * D, brief::kThreads) <= 0x7fffffffLL) {
+        constexpr int V = VecWidth<T>::value;
+        const bool vec = chunked::vector_ok<T>(D, {alpha, beta, h}) && (!st || lookback::state_aligned({st->h_in, st->h_last}));
+        return vec ? brief_forward<T, V>(ctx, B, Tn, D, alpha, beta, h, st) : brief_forward<T, 1>(ctx, B, Tn, D, alpha, beta, h, st);
+    }
     if (algo != FSS_ALGO_CHUNKED) {
         const bool ok = lookback::layout_ok<T>(B, Tn, D, {alpha, beta, h}) &&
                         (!st || lookback::state_aligned({st->h_in, st->h_last, st->prod, st->block_prod, st->block_state}));

@@ -41,7 +41,8 @@ extern "C" {
 #define FSS_DTYPE_F32 1
 
 /* kernel families */
-#define FSS_ALGO_AUTO 0     /* single-pass TMA kernel when the layout allows it, else a single-pass
+#define FSS_ALGO_AUTO 0     /* forward of at most 8 rows: one thread per channel vector; else the
+                               single-pass TMA kernel when the layout allows it, else a single-pass
                                kernel for any layout, or the chunked ones (block outputs)        */
 #define FSS_ALGO_CHUNKED 1  /* three launches: chunk summaries, carry composition, chunk re-scan */
 #define FSS_ALGO_LOOKBACK 2 /* one persistent launch: TMA tiles + decoupled look-back of carries */

@@ -545,6 +545,30 @@ def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (16, 1, 2560), (3, 2, 33), (2, 7, 24), (130, 8, 520), (2, 9, 264)])
+def test_forward_of_a_few_rows_matches_the_chunked_kernels(shape, dtype):
+    """Up to 8 rows go to a kernel of their own (9: the first length that does not); aligned and odd widths, both scan
+    orders, with and without boundary state.  Its sums are the chunked kernels' sums row by row, so results are equal."""
+    _, native, _ = _mods()
+    B, T, D = shape
+    gen = torch.Generator(device="cuda").manual_seed(13)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a, b, h0 = torch.sigmoid(rnd(B, T, D)).to(dtype), rnd(B, T, D).to(dtype), rnd(B, D)
+    for cont, reverse in [(False, False), (True, False), (True, True)]:
+        runs = []
+        for algo in ("chunked", "auto"):
+            h, last = torch.full_like(a, 7.0), torch.empty(B, D, device="cuda")
+            native.forward_into(a, b, h, algo=_algo_id(algo), continuation=cont, h_in=h0 if cont else None, h_last=last, reverse=reverse)
+            runs.append((h, last))
+        if T <= 8:
+            assert torch.equal(runs[0][0], runs[1][0]), (cont, reverse)
+        assert_same_up_to_association(runs[0][0], runs[1][0], "h")
+        assert_parity(runs[1][1].cpu(), runs[0][1].cpu(), F32_TOL, "state after the last row")
+    import fast_sequential_scan_b200 as pkg
+    pkg.check_status()
+
+
 def test_gated_scan_state():
     """Boundary state of the gated entry point through the C ABI."""
     pkg, native, _ = _mods()

@@ -42,8 +42,9 @@ from typing import Any, Optional, Tuple
 import torch
 from torch.autograd import Function
 
-from .sequential_scan_cuda import (backward_into, forward_into, scan_backward, scan_backward_gated, scan_backward_half,
-                                   scan_forward, scan_forward_gated, scan_forward_half, tma_eligible)
+from . import _fss_torch, _lib
+from .sequential_scan_cuda import (backward_into, default_algo, forward_into, scan_backward, scan_backward_gated,
+                                   scan_backward_half, scan_forward, scan_forward_gated, scan_forward_half, tma_eligible)
 
 BACKWARD_MODES = ("saved", "inplace", "recompute")
 _default_mode = "saved"
@@ -161,7 +162,24 @@ class _StatefulScan(Function):
         return da, db, dh0, None, None
 
 
+_plain_types = (torch.Tensor, torch.nn.Parameter)
+
+
+def _ordinary_call(*tensors) -> bool:
+    """Plain tensors, no autocast and nothing that traces, transforms or differentiates forward: calls that the C++
+    functions may take.  All others keep to the Python classes, which torch knows how to treat there."""
+    for t in tensors:
+        if type(t) not in _plain_types:
+            return False
+    return not (torch.is_autocast_enabled("cuda") or torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
+                or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0)
+
+
 def _scan_any(plain_cls, dtype: torch.dtype, alpha, beta, backward_mode, h0, return_final_state, reverse):
+    if _resolve(backward_mode) == "saved" and (_ordinary_call(alpha, beta) if h0 is None else _ordinary_call(alpha, beta, h0)):
+        out = _fss_torch.scan(alpha, beta, h0, bool(return_final_state), bool(reverse), dtype is torch.bfloat16)
+        if out is not None:
+            return out
     if h0 is None and not return_final_state and not reverse:
         return plain_cls.apply(alpha, beta, backward_mode)
     if backward_mode not in (None, "saved"):
@@ -214,4 +232,8 @@ class GatedSequentialScan(Function):
 def scan_gated(r: torch.Tensor, i: torch.Tensor, x: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
     """Gated scan over ``[batch, seq, d_model]`` tensors ``r, i, x`` (bf16 or fp32) and the fp32
     per-channel parameter ``lam`` of ``d_model`` values; see :class:`GatedSequentialScan`."""
+    if default_algo() != _lib.ALGO_CHUNKED and _ordinary_call(r, i, x, lam):
+        out = _fss_torch.gated(r, i, x, lam)
+        if out is not None:
+            return out
     return GatedSequentialScan.apply(r, i, x, lam)

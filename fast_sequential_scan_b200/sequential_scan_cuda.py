@@ -19,7 +19,7 @@ from typing import List, Optional
 
 import torch
 
-from . import _lib, workspace
+from . import _fss_torch, _lib, workspace
 
 _DTYPES = {torch.bfloat16: _lib.DTYPE_BF16, torch.float32: _lib.DTYPE_F32}
 
@@ -107,6 +107,28 @@ def _ctx(device: torch.device, ws: workspace.Workspace, algo: Optional[int], fla
     ctx.algo = default_algo() if algo is None else algo
     ctx.flags = flags | (_lib.FLAG_DETERMINISTIC if _deterministic else 0)
     return ctx
+
+
+_torch_devices: dict = {}
+
+
+def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: int):
+    """What ``_fss_torch`` needs for one launch on the current stream: the address of its context and, once several
+    streams are in play on the device, the workspace that :func:`workspace.launched` wants to hear of afterwards."""
+    device = _torch_devices.get(index)
+    if device is None:
+        device = _torch_devices[index] = torch.device("cuda", index)
+    query = "fss_gated_backward_workspace_bytes" if gated_backward else "fss_workspace_bytes"
+    key = ((B, T, D), dtype_id, query)
+    need = _ws_bytes_cache.get(key)
+    if need is None:
+        need = _ws_bytes_cache[key] = getattr(_lib.lib(), query)(B, T, D, dtype_id)
+    ws = workspace.get(device, need)
+    ctx = _ctx(device, ws, None)
+    if ws.order.multi:
+        return ctypes.addressof(ctx), ws
+    ws.order.last = ws
+    return ctypes.addressof(ctx), None
 
 
 def _vec(t: Optional[torch.Tensor], B: int, D: int, name: str) -> Optional[int]:
@@ -350,6 +372,14 @@ def backward_into(alpha, h, grad_out, grad_alpha, grad_beta, *, algo=None, conti
     _launch_backward(a, hh, g, grad_alpha, grad_beta, _DTYPES[dtype], algo,
                      (_lib.FLAG_CONTINUATION if continuation else 0)
                      | (_lib.FLAG_HOLD_DEPENDENTS if hold_dependents else 0) | (_lib.FLAG_REVERSE if reverse else 0), state)
+
+
+def _address(name: str) -> int:
+    return ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value
+
+
+_fss_torch.bind(_address("fss_scan_forward_ex"), _address("fss_scan_backward_ex"), _address("fss_scan_forward_gated"),
+                _address("fss_scan_backward_gated"), _acquire, workspace.launched, _lib.check, scan_backward_gated)
 
 
 def _forward(alpha: torch.Tensor, beta: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

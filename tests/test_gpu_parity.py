@@ -569,6 +569,87 @@ def test_forward_of_a_few_rows_matches_the_chunked_kernels(shape, dtype):
     pkg.check_status()
 
 
+def _both_routes(monkeypatch, call, leaves, pick):
+    """Outputs and gradients of ``call`` by the C++ functions and by the Python classes."""
+    from fast_sequential_scan_b200 import scan_cuda
+    results = []
+    for native_route in (True, False):
+        if not native_route:
+            monkeypatch.setattr(scan_cuda, "_ordinary_call", lambda *a: False)
+        xs = [t.detach().requires_grad_() for t in leaves]
+        outs = call(*xs)
+        outs = list(outs) if isinstance(outs, tuple) else [outs]
+        name = type(outs[0].grad_fn).__name__
+        assert name.startswith("CppFunction") == native_route, name
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        gs = [torch.randn(o.shape, generator=gen, device="cuda").to(o.dtype) for o in outs]
+        grads = torch.autograd.grad([outs[k] for k in pick], xs, [gs[k] for k in pick], retain_graph=True)
+        again = torch.autograd.grad([outs[k] for k in pick], xs, [gs[k].mT.contiguous().mT if gs[k].dim() == 3 else gs[k] for k in pick])
+        results.append((outs, grads, again))
+    monkeypatch.undo()
+    for x, y in zip(results[0], results[1]):
+        for a, b in zip(x, y):
+            assert a.shape == b.shape and a.dtype == b.dtype
+            bound = (2.0 ** -7 if a.dtype == torch.bfloat16 else 2.0 ** -18) * (b.detach().float().abs() + 1.0)      # association
+            assert bool(((a.detach().float() - b.detach().float()).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["contiguous", "slice", "odd", "row_gap"])
+def test_cpp_functions_match_the_python_classes(form, dtype, monkeypatch):
+    """The C++ autograd functions against the Python classes over the forms that both take: strided and unaligned
+    views, boundary state in and out, both directions, one output unused, transposed gradients, saved-tensor hooks."""
+    pkg, _, _ = _mods()
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    B, T, D = 3, 70, 33 if form == "odd" else 40
+
+    def tensor(f=lambda t: t):
+        wide = f(torch.randn(B, 2 * T, D + 8, generator=gen, device="cuda")).to(dtype)
+        return {"contiguous": wide[:, :T, :D].contiguous(), "odd": wide[:, :T, :D].contiguous(), "slice": wide[:, :T, 8:],
+                "row_gap": wide[:, ::2, :D]}[form]
+    a, b, h0 = tensor(torch.sigmoid), tensor(), torch.randn(B, D, generator=gen, device="cuda")
+    scan = pkg.scan_cu if dtype == torch.bfloat16 else pkg.scan_cu_single
+    _both_routes(monkeypatch, scan, [a, b], [0])
+    _both_routes(monkeypatch, lambda x, y: scan(x, y, return_final_state=True), [a, b], [0, 1])
+    for pick in ([0, 1], [0], [1]):
+        _both_routes(monkeypatch, lambda x, y, z: scan(x, y, h0=z, return_final_state=True), [a, b, h0], pick)
+    if form == "contiguous":
+        _both_routes(monkeypatch, lambda x, y, z: scan(x, y, h0=z, return_final_state=True, reverse=True), [a, b, h0], [0, 1])
+        r, i, x, lam = (torch.randn(s, generator=gen, device="cuda").to(t) for s, t in [((B, T, D), dtype)] * 3 + [((D,), torch.float32)])
+        _both_routes(monkeypatch, pkg.scan_gated, [r, i, x, lam], [0])
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.cuda()):
+            _both_routes(monkeypatch, scan, [a, b], [0])
+            _both_routes(monkeypatch, pkg.scan_gated, [r, i, x, lam], [0])
+    pkg.check_status()
+
+
+def test_calls_that_stay_with_the_python_classes():
+    """Autocast, transforms, forward-mode tensors and everything that is refused go to the Python classes."""
+    pkg, _, _ = _mods()
+    a = torch.rand(2, 9, 16, device="cuda")
+    b = torch.randn(2, 9, 16, device="cuda")
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert pkg.scan_cu(a, b).dtype == torch.bfloat16
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: pkg.scan_cu_single(t, b).sum())(a)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda t: pkg.scan_cu_single(t, b))(a[None])
+    with pytest.raises(RuntimeError):
+        with torch.autograd.forward_ad.dual_level():
+            pkg.scan_cu_single(torch.autograd.forward_ad.make_dual(a, a), b)
+    for bad in (lambda: pkg.scan_cu(a, b), lambda: pkg.scan_cu_single(a[0], b[0]), lambda: pkg.scan_cu_single(a, b[:1]),
+                lambda: pkg.scan_cu_single(a.cpu(), b.cpu()), lambda: pkg.scan_cu_single(a, b, h0=a[:, 0, :8])):
+        with pytest.raises(RuntimeError):
+            bad()
+    with pytest.raises(TypeError):
+        pkg.scan_cu_single(a, 1.0)
+    with pytest.raises(ValueError):
+        pkg.scan_cu_single(a, b, backward_mode="other")
+    assert pkg.scan_cu_single(a[:, :0], b[:, :0]).shape == (2, 0, 16)
+    with torch.no_grad():
+        assert not pkg.scan_cu_single(a.requires_grad_(), b).requires_grad
+
+
 def test_gated_scan_state():
     """Boundary state of the gated entry point through the C ABI."""
     pkg, native, _ = _mods()

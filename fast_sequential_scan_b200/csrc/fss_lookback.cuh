@@ -47,7 +47,6 @@ namespace fss {
 namespace lookback {
 
 constexpr int kW = 4;                         // warps per pass (pass-1 group and pass-2 group)
-constexpr int kRh = 8;                        // rows handled per register batch
 constexpr int kRowBytes = 256;                // bytes of one tile row
 constexpr int kLaneBytes = 8;
 constexpr int kLookbackWarps = 2;             // three were measured slower on every workload
@@ -532,6 +531,10 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
     constexpr int kPass2Warp0 = K::kPass2Warp0, kProducerWarp = K::kProducerWarp, kSummaryWarp = K::kSummaryWarp;
     constexpr int kLookbackWarp0 = K::kLookbackWarp0;
     constexpr bool kGateBwd = kGate && kBackward;
+    // Rows per register batch.  The narrow tiles' register swaps make long loop bodies, and in the long
+    // ticketed backward the warps of a scheduler wait for instructions: 2 rows 411 us, 4 rows 418, 8 rows 428
+    // (B1 T65536 D4096 bf16; B4 T8192 D2048 108 with either).  Everywhere else 8 rows are as fast or up to 3 % faster.
+    constexpr int kRh = kTickets && kSp == 4 ? 2 : 8;
     using SM = Smem<K::kIn, kStages, kTileBytes>;
     constexpr int V = Cfg<T>::V;
     // Tile shape: kSp = 1: 64 rows x 256 bytes; 2: 128 x 128; 4: 256 x 64 (same 16 KiB).  A warp then

@@ -90,25 +90,6 @@ static int need_workspace(const fss_scan_ctx *ctx, int64_t B, int64_t T, int64_t
     return FSS_OK;
 }
 
-// Launch with the programmatic-dependent-launch attribute: the kernel may be placed while its
-// predecessor on the stream drains; it must execute griddepcontrol.wait before it touches anything
-// the predecessor wrote (the kernels launched this way do so first thing).
-template <typename... Params, typename... Args>
-static cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
-
 static int launch_check(const char *what) {
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FSS_OK : cuda_fail(e, what, FSS_E_LAUNCH);

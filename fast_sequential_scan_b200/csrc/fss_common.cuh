@@ -170,6 +170,25 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Launch with the programmatic-dependent-launch attribute: the kernel may be placed while its
+// predecessor on the stream drains; it must execute griddepcontrol.wait before it touches anything
+// the predecessor wrote (the kernels launched this way do so first thing).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // Workspace plan: [256-byte header | descriptor packets | float scratch].  The split depends only
 // on the workspace's total size, so for one allocation the packet area always sits at the same
 // place and only ever holds 16-byte packets whose fourth word is a tag: a stale float can never

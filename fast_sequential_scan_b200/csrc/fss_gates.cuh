@@ -107,10 +107,20 @@ namespace gates {
 constexpr int kThreads = 256;
 constexpr int kRowsPerCta = 32;      // rows one CTA walks (bounds the partial sums it adds to dlambda)
 
+// The tables are made by a launch of their own just before the scan's.  Both are dependent launches: this
+// one is placed while the kernel before it drains, waits for that kernel (which may still read the
+// table it will write), and lets the scan set itself up meanwhile (the scan waits for the table).
+// Gated forward of B4 T1000 D2048 bf16 in a loop: 22.8 us a call as ordinary launches, 21.3 so.
+__device__ __forceinline__ void table_prologue() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // scales[d] = -8 * softplus(lambda[d]) * log2(e): the per-channel factor of the exponent, computed once
 // per launch of the fused forward instead of once per tile
 template <typename T>
 __global__ void prescale(const float *__restrict__ lambda, float *__restrict__ scales, int64_t D) {
+    table_prologue();
     const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (d < D) scales[d] = Gate<T>::prescale(gate_scale(lambda[d]));
 }
@@ -118,6 +128,7 @@ __global__ void prescale(const float *__restrict__ lambda, float *__restrict__ s
 // The same for the fused backward: -8 * softplus(lambda) and its slope; dlambda starts at zero.
 __global__ void backward_tables(const float *__restrict__ lambda, float *__restrict__ scales, float *__restrict__ slopes,
                                 float *__restrict__ dlambda, int64_t D) {
+    table_prologue();
     const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= D) return;
     scales[d] = gate_scale(lambda[d]);

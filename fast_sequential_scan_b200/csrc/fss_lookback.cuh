@@ -1754,9 +1754,10 @@ inline int forward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, i
     // the per-channel exponent scales, once per launch, into the float scratch of the workspace
     if ((size_t)D * sizeof(float) > ws.float_bytes) return FSS_E_WORKSPACE;
     float *scales = reinterpret_cast<float *>(ws.floats);
-    gates::prescale<T><<<(unsigned)ceil_div(D, 256), 256, 0, (cudaStream_t)ctx->stream>>>(lambda, scales, D);
     {
-        const cudaError_t e = cudaGetLastError();
+        cudaError_t e = launch_dependent(gates::prescale<T>, dim3((unsigned)ceil_div(D, 256)), dim3(256), 0, (cudaStream_t)ctx->stream,
+                                         lambda, scales, D);
+        if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) { *err_text = std::string("gate scale launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     }
     p.scales = scales;
@@ -1774,8 +1775,9 @@ inline int backward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, 
     if ((size_t)D * 2 * sizeof(float) > ws.float_bytes) return FSS_E_WORKSPACE;
     Params p{};
     float *scales = reinterpret_cast<float *>(ws.floats), *slopes = scales + D;
-    gates::backward_tables<<<(unsigned)ceil_div(D, 256), 256, 0, (cudaStream_t)ctx->stream>>>(lambda, scales, slopes, dlambda, D);
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_dependent(gates::backward_tables, dim3((unsigned)ceil_div(D, 256)), dim3(256), 0, (cudaStream_t)ctx->stream,
+                                     lambda, scales, slopes, dlambda, D);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { *err_text = std::string("gate table launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     p.scales = scales;
     p.slopes = slopes;

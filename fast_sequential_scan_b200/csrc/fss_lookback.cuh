@@ -523,7 +523,7 @@ __device__ __forceinline__ void gated_backward_pair(const Two &r, const Two &g, 
 template <typename T, bool kBackward, int kSp, bool kTickets, bool kGate = false, bool kReverse = false>
 __global__ void __launch_bounds__(Kind<kBackward, kGate>::kThreads, 1)
 scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBackward, kGate>::kOut> maps, const Params p) {
-    static_assert(!((kGate || kReverse) && !kBackward && kTickets), "these forwards keep the fixed tile order");
+    static_assert(!(kTickets && (kGate || (kReverse && !kBackward))), "the gated scans and the reversed forward keep the fixed tile order");
     static_assert(!(kGate && kReverse), "the gated scan has no reversed form");
     constexpr bool kDown = kBackward != kReverse;      // rows are processed from the last to the first
     using K = Kind<kBackward, kGate>;
@@ -1024,8 +1024,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 // for the summary and r stays.
                 constexpr int kPairs = V / 2;
                 // Rows per loop body: longer bodies wait for instructions, shorter ones for their operands.
-                // B16 T4096 D2560 bf16: forward 268 / 248 / 229 us with 1 / 2 / 4 rows, backward 466 / 456 us
-                // with 1 / 2 and 514 us with 4 (its pass 2 at one row and at two).
+                // B16 T4096 D2560 bf16: forward 268 / 248 / 229 us with 1 / 2 / 4 rows; backward 449 / 439 / 440 us with
+                // 1 / 2 / 4.
                 constexpr int kRows = kBackward ? 2 : 4;
                 const Raw *i_t = x_t + kTileBytes / (int)sizeof(Raw);
                 const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
@@ -1174,8 +1174,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
             if constexpr (kGateBwd) {
                 constexpr int kPairs = V / 2;
                 // Rows per loop body.  Three heavy warps of a scheduler run different code here, and with
-                // longer bodies they wait for instructions: 4 rows 565 us, 2 rows 494 us, 1 row 456 us (c4
-                // shape, bf16).  The row pairs of 64-byte tile rows need two.
+                // longer bodies they wait for instructions: 4 rows 488 us, 1 or 2 rows 439 us (B16 T4096 D2560
+                // bf16).  The row pairs of 64-byte tile rows need two.
                 constexpr int kGateRows2 = kPairSwap ? 2 : 1;
                 const int nvalid = left >= kR ? kR : (left > 0 ? (int)left : 0);
                 const bool edge_rows = __any_sync(0xffffffffu, head || nvalid < kR);
@@ -1640,7 +1640,8 @@ inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t 
                   std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p,
                   std::string *err_text) {
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
-    constexpr bool kNeverTickets = (kGate || kReverse) && !kBackward;
+    // (the gated backward, too, is faster in the fixed order: 439 us against 475 at B16 T4096 D2560 bf16)
+    constexpr bool kNeverTickets = kGate || (kReverse && !kBackward);
     const int tail = kNeverTickets ? 0 : choose_tail(dtype, kBackward, B, Tn, D);
 #define FSS_LAUNCH_SPLIT(SP)                                                                                                    \
     return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
@@ -1767,7 +1768,7 @@ inline int forward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, i
 // Backward of the gated scan in one pass over memory: reads r, grad, h, i, x and writes dr, di, dx (8
 // tensor passes; re-creating alpha, the plain reverse scan and the gates' chain rule as launches of
 // their own take 15) and adds the gradient of lambda per tile.  Measured at B16 T4096 D2560 bf16: the three
-// launches 1,204 us (153 + 268 + 783), this one 456 us = 5.9 TB/s; fp32 at B4 T2048 D2560 107 us = 6.3 TB/s.
+// launches 1,204 us (153 + 268 + 783), this one 439 us = 6.1 TB/s; fp32 at B4 T2048 D2560 107 us = 6.3 TB/s.
 template <typename T>
 inline int backward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D, const fss_view *r,
                           const fss_view *i, const fss_view *x, const float *lambda, const fss_view *h, const fss_view *grad,

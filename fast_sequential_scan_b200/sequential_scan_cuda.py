@@ -441,7 +441,7 @@ def scan_backward_half(alpha_saved, h_saved, grad_out, inplace_grad_beta: bool =
 
 def tma_eligible(*tensors: torch.Tensor) -> bool:
     """True when the single-pass kernels can take these [B, T, D] tensors (16-byte aligned bases,
-    row and batch strides that are multiples of 16 bytes); otherwise ``auto`` uses the chunked kernels."""
+    row and batch strides that are multiples of 16 bytes); otherwise ``auto`` uses the any-layout kernels."""
     for t in tensors:
         per16 = 16 // t.element_size()
         B, T, D = t.shape

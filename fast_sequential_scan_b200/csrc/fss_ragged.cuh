@@ -14,7 +14,7 @@
 // (16 loads per tensor in flight per thread, two or three CTAs per SM).  Against the chunked kernels with
 // one element per access, which read every input twice and compose the chunks' states in one thread
 // per column (forward / backward): B4 T1000 D1001 bf16 46 / 50 -> 15 / 24 us, B8 T2048 D2049 bf16 276 / 320 ->
-// 95 / 171 us (2.1 / 2.0 TB/s), D2052 76 / 104 us, B1 T65536 D515 bf16 1687 / 1703 -> 112 / 195 us, B2 T8192 D2051 fp32
+// 87 / 161 us (2.3 / 2.1 TB/s), D2052 76 / 104 us, B1 T65536 D515 bf16 1687 / 1703 -> 112 / 195 us, B2 T8192 D2051 fp32
 // 439 / 517 -> 99 / 153 us (4.1 / 4.4 TB/s).
 #pragma once
 
@@ -88,12 +88,16 @@ __device__ __forceinline__ void store_cell(char *p, float x, uint32_t tag) {
 // us with three against 177 with two (B2 T8192 D2051), bf16 backward 207 against 171 (B8 T2048 D2049), pairs 118
 // against 104 (D2052).
 template <typename T, bool kBackward, int V> constexpr int kMinCtas = V == 2 || (kBackward && sizeof(T) == 2) ? 2 : 3;
-template <typename T, bool kBackward, int V>
+// kEarly: a first look at the tile before this one, ahead of the loads.  With more columns than a wave of
+// CTAs takes, that tile is long finished and its final state is here before this tile's rows are: B8 T2048
+// D2049 bf16 forward / backward 95 / 171 -> 87 / 160 us, B16 T512 D4093 91 / 166 -> 85 / 158.  With fewer columns it
+// finds nothing and costs 1-2 % (B4 T1000 D1001), and the fp32 kernels have no registers left for it.
+template <typename T, bool kBackward, int V, bool kEarly>
 __global__ void __launch_bounds__(kThreads, kMinCtas<T, kBackward, V>)
 scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0, View<T> out1, const Params p) {
     using L = Lot<T, V>;
     using Raw = typename L::Raw;
-    __shared__ uint32_t s_tile, s_epoch, s_abort;
+    __shared__ uint32_t s_tile, s_epoch, s_abort, s_early;
     __shared__ float sP[V][kWarps][32], sC[V][kWarps][32];
     __shared__ float wP[V][kWarps][32], wC[V][kWarps][32];      // window: summary, or final state in wC
     __shared__ int w_kind[kWarps];                               // 0 nothing yet, 1 summary, 2 final state
@@ -102,6 +106,7 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
         s_tile = atomicAdd(&p.hdr->ticket, 1u);
         s_epoch = lookback::ld_volatile(&p.hdr->epoch) + 1u;
         s_abort = 0;
+        s_early = 0;
     }
     __syncthreads();
     const uint32_t tile = s_tile, epoch = s_epoch;
@@ -111,6 +116,17 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
     const bool ch_ok = d < p.D;                                  // (V divides D)
     const int64_t i0 = s * kTileRows + warp * kRows;
     const int n = !ch_ok || i0 >= p.T ? 0 : (p.T - i0 < kRows ? (int)(p.T - i0) : kRows);      // this thread's rows
+
+    const uint32_t tag_agg = (epoch << 2) | lookback::kStateAggregate, tag_inc = (epoch << 2) | lookback::kStateInclusive;
+    auto agg_cells = [&](uint32_t k, int v) { return p.cells + (int64_t)k * (32 * V * kCellBytes) + (v * 32 + lane) * 16; };
+    auto inc_cell = [&](uint32_t k, int v) { return p.cells + (int64_t)k * (32 * V * kCellBytes) + 32 * V * 16 + (v * 32 + lane) * 8; };
+
+    const bool early_look = kEarly && warp == 0 && s > 0;
+    unsigned long long early[V];
+    if (early_look) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) early[v] = load_cell(inc_cell(tile - p.ncols, v));
+    }
 
     // ---- everything this thread will read, in flight at once
     float ones[V], zeros[V];
@@ -144,6 +160,17 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
             }
     }
 
+    if (early_look) {
+        bool ok = true;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            ok &= (uint32_t)(early[v] >> 32) == tag_inc;
+            wC[v][0][lane] = __uint_as_float((uint32_t)early[v]);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) s_early = ok;
+    }
+
     // ---- summaries: this warp's rows, the rows of the warps before it, the tile
     {
         float P[V], C[V];
@@ -164,9 +191,6 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
         for (int v = 0; v < V; ++v) { sP[v][warp][lane] = P[v]; sC[v][warp][lane] = C[v]; }
     }
     __syncthreads();
-    const uint32_t tag_agg = (epoch << 2) | lookback::kStateAggregate, tag_inc = (epoch << 2) | lookback::kStateInclusive;
-    auto agg_cells = [&](uint32_t k, int v) { return p.cells + (int64_t)k * (32 * V * kCellBytes) + (v * 32 + lane) * 16; };
-    auto inc_cell = [&](uint32_t k, int v) { return p.cells + (int64_t)k * (32 * V * kCellBytes) + 32 * V * 16 + (v * 32 + lane) * 8; };
     const bool last_block = s + 1 == p.S;
     float tP[V], tC[V];                                          // the tile's summary, in the last warp
     if (warp == kWarps - 1) {
@@ -191,7 +215,10 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
     float cin[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) cin[v] = p.state_in && ch_ok ? p.state_in[b * p.D + d + v] : 0.0f;      // ... and the scan
-    if (s > 0) {
+    if (kEarly && s > 0 && s_early) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) cin[v] = wC[v][0][lane];
+    } else if (s > 0) {
         const int64_t m = s - 1 - warp;        // row block this warp looks at; -1: the state before the first one
         uint32_t spins = 0;
         float before[V];
@@ -335,7 +362,12 @@ inline int launch_lots(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int
     p.status = ctx->status;
     p.continuation = (ctx->flags & FSS_FLAG_CONTINUATION) ? 1 : 0;
     p.max_spins = (ctx->flags & FSS_FLAG_TEST_SHORT_WAITS) ? 4096u : lookback::kMaxSpins / 4;      // (a round of the window takes several times a poll)
-    scan_kernel<T, kBackward, V><<<(unsigned)tiles(B, Tn, D, V), kThreads, 0, (cudaStream_t)ctx->stream>>>(alpha, x, h, out0, out1, p);
+    const unsigned grid = (unsigned)tiles(B, Tn, D, V);
+    const cudaStream_t stream = (cudaStream_t)ctx->stream;
+    if (sizeof(T) == 2 && p.ncols >= 2 * 148)      // (a wave: two CTAs per SM)
+        scan_kernel<T, kBackward, V, sizeof(T) == 2><<<grid, kThreads, 0, stream>>>(alpha, x, h, out0, out1, p);
+    else
+        scan_kernel<T, kBackward, V, false><<<grid, kThreads, 0, stream>>>(alpha, x, h, out0, out1, p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { *err_text = std::string("any-layout launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     return FSS_OK;

@@ -514,7 +514,7 @@ def test_reverse_is_the_scan_of_the_flipped_rows(shape, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(1, 1, 1), (2, 15, 31), (3, 16, 33), (2, 17, 32), (1, 127, 65), (2, 128, 7), (2, 129, 100), (1, 3000, 45),
-                                   (4, 1000, 1001), (1, 20000, 5)])
+                                   (4, 1000, 1001), (1, 20000, 5), (5, 400, 2003), (5, 400, 4098)])
 def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
     """Odd widths and unaligned views at the edges of a tile (128 rows x 32 channels) and of a warp's rows, both scan
     orders, with and without boundary state; two runs are bit-identical.  ``auto`` takes the any-layout kernel here."""

@@ -138,6 +138,22 @@ __device__ __forceinline__ Two add2(const Two &a, const Two &b) {
     return r;
 }
 
+// ------------------------------------------------------------------ loads of what a kernel before this one wrote
+// For kernels that are placed while the kernel before them on the stream still runs: what that kernel
+// writes is not read-only for the life of this one, so neither __ldg nor a const __restrict__ pointer
+// (which the compiler may turn into one) may read it.  These loads stay behind the dependency wait and
+// are served by L2, past whatever an earlier kernel left of the same addresses in the SM's L1.
+__device__ __forceinline__ void load_fresh(const float *p, float (&x)[1]) {
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(x[0]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void load_fresh(const float *p, float (&x)[2]) {      // p: 8-byte aligned
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(x[0]), "=f"(x[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void load_fresh(const float *p, float (&x)[4]) {      // p: 16-byte aligned
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "l"(p) : "memory");
+}
+
 // ------------------------------------------------------------------ status word
 // Written only when a bounded wait gives up; works for device memory and for pinned host memory.
 __device__ __forceinline__ void report_status(int32_t *status, int32_t code) {

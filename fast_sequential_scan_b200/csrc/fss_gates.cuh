@@ -110,6 +110,8 @@ constexpr int kRowsPerCta = 32;      // rows one CTA walks (bounds the partial s
 // The tables are made by a launch of their own just before the scan's.  Both are dependent launches: this
 // one is placed while the kernel before it drains, waits for that kernel (which may still read the
 // table it will write), and lets the scan set itself up meanwhile (the scan waits for the table).
+// Nothing of the table may therefore be read by a load that takes it for constant (load_fresh), nor
+// may lambda, which the kernel before this one may have written.
 // Gated forward of B4 T1000 D2048 bf16 in a loop: 22.8 us a call as ordinary launches, 21.3 so.
 __device__ __forceinline__ void table_prologue() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -119,20 +121,24 @@ __device__ __forceinline__ void table_prologue() {
 // scales[d] = -8 * softplus(lambda[d]) * log2(e): the per-channel factor of the exponent, computed once
 // per launch of the fused forward instead of once per tile
 template <typename T>
-__global__ void prescale(const float *__restrict__ lambda, float *__restrict__ scales, int64_t D) {
-    table_prologue();
-    const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (d < D) scales[d] = Gate<T>::prescale(gate_scale(lambda[d]));
-}
-
-// The same for the fused backward: -8 * softplus(lambda) and its slope; dlambda starts at zero.
-__global__ void backward_tables(const float *__restrict__ lambda, float *__restrict__ scales, float *__restrict__ slopes,
-                                float *__restrict__ dlambda, int64_t D) {
+__global__ void prescale(const float *lambda, float *scales, int64_t D) {
     table_prologue();
     const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= D) return;
-    scales[d] = gate_scale(lambda[d]);
-    slopes[d] = gate_scale_slope(lambda[d]);
+    float l[1];
+    load_fresh(lambda + d, l);
+    scales[d] = Gate<T>::prescale(gate_scale(l[0]));
+}
+
+// The same for the fused backward: -8 * softplus(lambda) and its slope; dlambda starts at zero.
+__global__ void backward_tables(const float *lambda, float *scales, float *slopes, float *dlambda, int64_t D) {
+    table_prologue();
+    const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= D) return;
+    float l[1];
+    load_fresh(lambda + d, l);
+    scales[d] = gate_scale(l[0]);
+    slopes[d] = gate_scale_slope(l[0]);
     dlambda[d] = 0.0f;
 }
 

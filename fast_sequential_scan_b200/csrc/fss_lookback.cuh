@@ -438,9 +438,9 @@ template <bool kTickets, int kStages> struct UnitCursor {
 // TMA descriptors of a launch, in the order of Kind's lists
 template <int kIn, int kOut> struct Maps { CUtensorMap in[kIn], out[kOut]; };
 
-// Gated backward: this lane's per-channel constants of a unit, from the tables that were made once
+// Gated scans: this lane's per-channel constants of a unit, from the tables that were made once
 // per launch; fetched a unit ahead whenever the next unit is already known, so that the load's
-// latency stays off the tile's way.
+// latency stays off the tile's way.  (The tables start at multiples of 16 bytes and V divides D.)
 template <int V, int Dc> struct ChannelTable {
     const float *table;
     int64_t D;
@@ -450,7 +450,8 @@ template <int V, int Dc> struct ChannelTable {
     __device__ __forceinline__ void load(const Unit &un, float (&out)[V]) const {
         const int64_t dch = (int64_t)un.cg * Dc + ch;
 #pragma unroll
-        for (int v = 0; v < V; ++v) out[v] = dch + v < D ? __ldg(table + dch + v) : 0.0f;
+        for (int v = 0; v < V; ++v) out[v] = 0.0f;
+        if (dch < D) load_fresh(table + dch, out);      // the kernel that writes it may end after this one starts
     }
     template <typename C> __device__ __forceinline__ void ahead(const C &cursor) {
         ready = cursor.next_known();
@@ -1252,6 +1253,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_lam(g));
                 if (w2 == ((i / K::kP2) % kW)) {
+                    float slope[V];
+                    if (q == 0 && dch < p.D) load_fresh(p.slopes + dch, slope);      // on its way while the others finish
                     if (!ctl.wait(bar_lam(g), (uint32_t)((i / kGens) & 1), FSS_STATUS_LOOKBACK_TIMEOUT)) break;
                     float sum[V];
 #pragma unroll
@@ -1268,7 +1271,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                     for (int v = 0; v < V; ++v) sum[v] = sum_over_groups<LPG>(sum[v]);
                     if (q == 0 && dch < p.D) {
 #pragma unroll
-                        for (int v = 0; v < V; ++v) sum[v] *= __ldg(p.slopes + dch + v);
+                        for (int v = 0; v < V; ++v) sum[v] *= slope[v];
                         red_add(p.dlambda + dch, sum);
                     }
                 } else if (lane == 0) {

@@ -147,3 +147,15 @@ def test_reference_arm_of_the_bench_prints_the_contract_line():
         assert key in line
     assert line["cpu_baseline"]["kind"] in ("reference", "port") and line["cpu_baseline"]["cores"] >= 1
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["e2e"]["d2h_bytes_per_step"] == 0
+
+
+def test_kernels_that_start_early_do_not_take_their_predecessors_data_for_constant():
+    """The gated scans and the kernels that make their tables are placed while the kernel before them runs.  A load that
+    is only defined for data that stay constant for the kernel's life (``__ldg``, or what the compiler makes of a
+    ``const __restrict__`` pointer) must not read what that kernel writes: the tables, lambda."""
+    csrc = ROOT / "fast_sequential_scan_b200" / "csrc"
+    lookback, gates = (re.sub(r"//[^\n]*", "", (csrc / n).read_text()) for n in ("fss_lookback.cuh", "fss_gates.cuh"))
+    assert "__ldg" not in lookback
+    for kernel in ("prescale", "backward_tables"):
+        arguments = re.search(rf"__global__ void {kernel}\((.*?)\) \{{", gates, flags=re.S).group(1)
+        assert "__restrict__" not in arguments, kernel

@@ -447,6 +447,43 @@ def test_gated_scan_gradients(dtype, lam_range):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(2, 1, 8), (2, 300, 264), (1, 1100, 2056)])
+def test_gated_scans_enqueued_back_to_back_read_their_own_tables(shape, dtype):
+    """Forwards and backwards with six different ``lam``, written to one buffer just before, enqueued alternately while
+    the stream is busy, so that every launch is placed while the one before it runs.  All use the same table addresses.
+    Each is compared with the gate kernels and the plain scan, which use no table; another ``lam``'s table is off by
+    tens of per cent.  Bounds: as for the gated backward in one kernel below."""
+    pkg, native, _ = _mods()
+    from fast_sequential_scan_b200.workloads import Workload, make_gate_inputs
+    w = Workload("t", *shape, "hawk", dtype)
+    r, i, x, _ = make_gate_inputs(w, "cuda", seed=5)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    g = torch.randn(shape, generator=gen, device="cuda").to(r.dtype)
+    lams = [torch.empty(shape[2], device="cuda").uniform_(k - 6.0, k - 5.0, generator=gen) for k in range(6)]
+    want = []
+    for lam in lams:
+        alpha, beta = native.gates_forward(r, i, x, lam)
+        h = torch.empty_like(r)
+        native.forward_into(alpha, beta, h)
+        want.append((h, *native.gates_backward(r, i, x, lam, *native._backward(alpha, h, g, r.dtype))))
+    buf, got = torch.empty_like(lams[0]), []
+    pkg.check_status()
+    torch.cuda._sleep(100_000_000)          # some 50 ms: everything below is queued meanwhile
+    for _ in range(3):
+        for lam, ref in zip(lams, want):
+            buf.copy_(lam)
+            h = native.scan_forward_gated(r, i, x, buf)
+            got.append((h, *native.scan_backward_gated(r, i, x, buf, ref[0], g)))
+    pkg.check_status()
+    for k, outs in enumerate(got):
+        ref = want[k % len(lams)]
+        assert_same_up_to_association(outs[0], ref[0], f"h of scan {k}")
+        for a, b, name in zip(outs[1:], ref[1:], "r i x lam".split()):
+            err = float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+            assert err <= (2.0 ** -7 if dtype == "bf16" else 1e-5), (k, name, err)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("shape", [(2, 1, 8), (1, 31, 136), (3, 33, 24), (2, 260, 136), (1, 1025, 264), (5, 97, 1000), (2, 6200, 4104)])
 def test_gated_backward_in_one_kernel_matches_the_three_kernels(shape, dtype):
     """The fused backward at the edges of its tiles (one row; one less and more than a tile; each tile shape; the last

@@ -7,8 +7,11 @@
 // two launches through Python classes took 129 us a step, through these 76; decoding 33 and 13 us a call.
 //
 // The library is reached through the addresses that the package's ctypes table holds, and the streams'
-// workspaces stay with workspace.py: one Python call per launch, under the GIL, returns the context.
+// workspaces stay with workspace.py: one Python call per launch, under the GIL, takes the device's lock
+// and returns what the context is made of.
 #include <torch/extension.h>
+
+#include <cstring>
 
 #include "../../include/fss_b200.h"
 
@@ -24,9 +27,9 @@ struct Library {
     decltype(&fss_scan_forward_gated) forward_gated;
     decltype(&fss_scan_backward_gated) backward_gated;
 } lib;
-// Python: acquire(device index, B, T, D, dtype id, gated backward) -> (context address, workspace or
-// None); launched(workspace); check(code, where); the gated backward for any layout.  Held for the
-// process's life.
+// Python: acquire(device index, B, T, D, dtype id, gated backward) -> (context, algo, flags, release of
+// the device's lock, workspace or None); launched(workspace); check(code, where); the gated backward for
+// any layout.  Held for the process's life.
 PyObject *py_acquire, *py_launched, *py_check, *py_gated_backward;
 
 struct Shape {
@@ -35,20 +38,36 @@ struct Shape {
     explicit Shape(const Tensor &t) : B(t.size(0)), T(t.size(1)), D(t.size(2)), dtype(t.scalar_type() == at::kBFloat16 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32) {}
 };
 
-// A launch's context; the GIL is held while it lives.
+// One launch, with a context of its own.  The device's lock (workspace.py) is held from the look-up of
+// the workspace until the launch is recorded; the GIL is held while this lives.
 struct Launch {
     fss_scan_ctx ctx;
-    py::object workspace;
+    py::object release, workspace;
     Launch(const Tensor &t, const Shape &s, int flags, bool gated_backward = false) {
-        py::tuple got = py::reinterpret_steal<py::object>(PyObject_CallFunction(py_acquire, "iLLLii", (int)t.get_device(), (long long)s.B,
-                                                                                (long long)s.T, (long long)s.D, s.dtype, (int)gated_backward));
+        const py::object got = py::reinterpret_steal<py::object>(PyObject_CallFunction(py_acquire, "iLLLii", (int)t.get_device(), (long long)s.B,
+                                                                                       (long long)s.T, (long long)s.D, s.dtype, (int)gated_backward));
         if (!got) throw py::error_already_set();
-        ctx = *reinterpret_cast<const fss_scan_ctx *>(PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(got.ptr(), 0)));
-        ctx.flags |= flags;
-        workspace = py::reinterpret_borrow<py::object>(PyTuple_GET_ITEM(got.ptr(), 1));
+        const auto item = [&](int k) { return PyTuple_GET_ITEM(got.ptr(), k); };
+        std::memcpy(&ctx, PyBytes_AS_STRING(item(0)), sizeof ctx);
+        ctx.algo = (int32_t)PyLong_AsLong(item(1));
+        ctx.flags = (int32_t)PyLong_AsLong(item(2)) | flags;
+        release = py::reinterpret_borrow<py::object>(item(3));
+        workspace = py::reinterpret_borrow<py::object>(item(4));
+    }
+    Launch(const Launch &) = delete;
+    ~Launch() {
+        if (!release) return;
+        py::error_scope keep;      // (an error that is on its way)
+        Py_XDECREF(PyObject_CallNoArgs(release.ptr()));
+    }
+    // after the call of the library
+    void done() {
+        if (!workspace.is_none()) py::reinterpret_borrow<py::object>(py_launched)(workspace);
+        py::object r = std::move(release);
+        r();
     }
     void done(int rc, const char *where) {
-        if (!workspace.is_none()) py::reinterpret_borrow<py::object>(py_launched)(workspace);
+        done();
         if (rc != FSS_OK) py::reinterpret_borrow<py::object>(py_check)(rc, where);      // raises
     }
 };
@@ -150,11 +169,12 @@ struct Gated : torch::autograd::Function<Gated> {
         Launch go(r, s, 0, true);
         const int rc = lib.backward_gated(&go.ctx, s.dtype, s.B, s.T, s.D, &vr, &vi, &vx, l.data_ptr<float>(), &vh, &vg, &v0, &v1, &v2,
                                           dlam.data_ptr<float>());
+        go.done();
         if (rc == FSS_E_LAYOUT) {      // saved-tensor hooks handed back copies that lie otherwise, say
             const py::tuple out = py::reinterpret_borrow<py::object>(py_gated_backward)(r, saved[1], saved[2], lam, saved[4], grads[0]);
             return {out[0].cast<Tensor>(), out[1].cast<Tensor>(), out[2].cast<Tensor>(), out[3].cast<Tensor>()};
         }
-        go.done(rc, "fss_scan_backward_gated");
+        if (rc != FSS_OK) py::reinterpret_borrow<py::object>(py_check)(rc, "fss_scan_backward_gated");      // raises
         return {dr, di, dx, dlam};
     }
 };

@@ -85,27 +85,38 @@ def _view(t: torch.Tensor) -> _lib.View:
 _ws_bytes_cache: dict = {}
 
 
-def _workspace_for(t: torch.Tensor, dtype_id: int, query: str = "fss_workspace_bytes") -> workspace.Workspace:
-    """The calling stream's workspace on ``t``'s device, large enough for a scan of ``t``'s shape (``query``: the
-    native call that says how large).  The answers are remembered per shape."""
-    key = (t.shape, dtype_id, query)
+def _workspace_bytes(shape, dtype_id: int, query: str = "fss_workspace_bytes") -> int:
+    """How large a workspace a scan of this shape needs (``query``: the native call that says so).  The answers are
+    remembered per shape."""
+    key = (shape, dtype_id, query)
     need = _ws_bytes_cache.get(key)
     if need is None:
-        B, T, D = t.shape
-        need = _ws_bytes_cache[key] = getattr(_lib.lib(), query)(B, T, D, dtype_id)
-    return workspace.get(t.device, need)
+        need = _ws_bytes_cache[key] = getattr(_lib.lib(), query)(*shape, dtype_id)
+    return need
+
+
+def _launch(t: torch.Tensor, dtype_id: int, query: str = "fss_workspace_bytes") -> workspace.Launch:
+    """One launch on the calling stream of ``t``'s device, with a workspace for a scan of ``t``'s shape."""
+    return workspace.Launch(t.device, _workspace_bytes(t.shape, dtype_id, query))
+
+
+def _ctx_bytes(device: torch.device, ws: workspace.Workspace) -> bytes:
+    if ws.ctx is None:      # (the workspace forgets it when its buffer is replaced)
+        ws.ctx = bytes(_lib.ScanCtx(ctypes.sizeof(_lib.ScanCtx), device.index if device.index is not None else -1,
+                                    ws.stream_handle, ws.buf.data_ptr(), ws.buf.numel(), ws.status.data_ptr(), 0, 0))
+    return ws.ctx
+
+
+def _call_flags(flags: int = 0) -> int:
+    return flags | (_lib.FLAG_DETERMINISTIC if _deterministic else 0)
 
 
 def _ctx(device: torch.device, ws: workspace.Workspace, algo: Optional[int], flags: int = 0) -> _lib.ScanCtx:
-    """The per-call context; the struct lives with the workspace and only algo / flags change per call.
-    ``device`` goes to the library, which makes it current for the launch, so no torch device
-    context is entered here."""
-    ctx = ws.ctx
-    if ctx is None or ctx.workspace != ws.buf.data_ptr():
-        ctx = ws.ctx = _lib.ScanCtx(ctypes.sizeof(_lib.ScanCtx), device.index if device.index is not None else -1,
-                                    ws.stream_handle, ws.buf.data_ptr(), ws.buf.numel(), ws.status.data_ptr(), 0, 0)
+    """The context of one call: the workspace's part, copied, with this call's algo and flags.  ``device`` goes to
+    the library, which makes it current for the launch, so no torch device context is entered here."""
+    ctx = _lib.ScanCtx.from_buffer_copy(_ctx_bytes(device, ws))
     ctx.algo = default_algo() if algo is None else algo
-    ctx.flags = flags | (_lib.FLAG_DETERMINISTIC if _deterministic else 0)
+    ctx.flags = _call_flags(flags)
     return ctx
 
 
@@ -113,22 +124,24 @@ _torch_devices: dict = {}
 
 
 def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: int):
-    """What ``_fss_torch`` needs for one launch on the current stream: the address of its context and, once several
-    streams are in play on the device, the workspace that :func:`workspace.launched` wants to hear of afterwards."""
+    """What ``_fss_torch`` needs for one launch on the current stream: the context's bytes, algo and flags; the
+    release of the device's lock, which is held from here on and which the caller calls when it has launched; and, once
+    several streams are in play on the device, the workspace that :func:`workspace.launched` wants to hear of before."""
     device = _torch_devices.get(index)
     if device is None:
         device = _torch_devices[index] = torch.device("cuda", index)
-    query = "fss_gated_backward_workspace_bytes" if gated_backward else "fss_workspace_bytes"
-    key = ((B, T, D), dtype_id, query)
-    need = _ws_bytes_cache.get(key)
-    if need is None:
-        need = _ws_bytes_cache[key] = getattr(_lib.lib(), query)(B, T, D, dtype_id)
-    ws = workspace.get(device, need)
-    ctx = _ctx(device, ws, None)
-    if ws.order.multi:
-        return ctypes.addressof(ctx), ws
-    ws.order.last = ws
-    return ctypes.addressof(ctx), None
+    need = _workspace_bytes((B, T, D), dtype_id, "fss_gated_backward_workspace_bytes" if gated_backward else "fss_workspace_bytes")
+    lock = workspace._order(device).lock
+    lock.acquire()
+    try:
+        ws = workspace._get(device, need)
+        ctx, algo, order = _ctx_bytes(device, ws), default_algo(), ws.order
+        if not order.multi:      # (stays as it is while the lock is held)
+            order.last, ws = ws, None
+        return ctx, algo, _call_flags(), lock.release, ws
+    except BaseException:
+        lock.release()
+        raise
 
 
 def _vec(t: Optional[torch.Tensor], B: int, D: int, name: str) -> Optional[int]:
@@ -150,25 +163,23 @@ def _blocks(t: Optional[torch.Tensor], name: str) -> Optional[int]:
 def _launch_forward(a, b, h, dtype_id: int, algo, flags: int, state) -> None:
     """One checked call of ``fss_scan_forward_ex`` on tensors that were validated by the caller."""
     B, T, D = a.shape
-    ws = _workspace_for(a, dtype_id)
-    ctx = _ctx(a.device, ws, algo, flags)
     va, vb, vh = _view(a), _view(b), _view(h)
-    rc = _lib.lib().fss_scan_forward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(va), ctypes.byref(vb),
-                                        ctypes.byref(vh), ctypes.byref(state) if state is not None else None)
-    workspace.launched(ws)
+    with _launch(a, dtype_id) as ws:
+        ctx = _ctx(a.device, ws, algo, flags)
+        rc = _lib.lib().fss_scan_forward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(va), ctypes.byref(vb),
+                                            ctypes.byref(vh), ctypes.byref(state) if state is not None else None)
     if rc:
         _lib.check(rc, "fss_scan_forward_ex")
 
 
 def _launch_backward(a, hh, g, grad_alpha, grad_beta, dtype_id: int, algo, flags: int, state) -> None:
     B, T, D = a.shape
-    ws = _workspace_for(a, dtype_id)
-    ctx = _ctx(a.device, ws, algo, flags)
     v0, v1, v2, v3, v4 = _view(a), _view(hh), _view(g), _view(grad_alpha), _view(grad_beta)
-    rc = _lib.lib().fss_scan_backward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(v0), ctypes.byref(v1),
-                                         ctypes.byref(v2), ctypes.byref(v3), ctypes.byref(v4),
-                                         ctypes.byref(state) if state is not None else None)
-    workspace.launched(ws)
+    with _launch(a, dtype_id) as ws:
+        ctx = _ctx(a.device, ws, algo, flags)
+        rc = _lib.lib().fss_scan_backward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(v0), ctypes.byref(v1),
+                                             ctypes.byref(v2), ctypes.byref(v3), ctypes.byref(v4),
+                                             ctypes.byref(state) if state is not None else None)
     if rc:
         _lib.check(rc, "fss_scan_backward_ex")
 
@@ -231,16 +242,15 @@ def forward_gated_into(r, i, x, lam, h, *, continuation=False, h_in=None, h_last
     rr, ii, xx = _rowwise(r), _rowwise(i), _rowwise(x)
     if _rowwise(h) is not h:
         raise RuntimeError("h: output must have unit channel stride and non-overlapping rows")
-    ws = _workspace_for(r, _DTYPES[dtype])
-    ctx = _ctx(r.device, ws, None, _lib.FLAG_CONTINUATION if continuation else 0)
     state = None
     if h_in is not None or h_last is not None:
         state = _lib.ForwardState(_vec(h_in, B, D, "h_in"), _vec(h_last, B, D, "h_last"), None, None, None)
     views = [_view(t) for t in (rr, ii, xx, h)]
-    rc = _lib.lib().fss_scan_forward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(views[0]),
-                                           ctypes.byref(views[1]), ctypes.byref(views[2]), lam.data_ptr(),
-                                           ctypes.byref(views[3]), ctypes.byref(state) if state is not None else None)
-    workspace.launched(ws)
+    with _launch(r, _DTYPES[dtype]) as ws:
+        ctx = _ctx(r.device, ws, None, _lib.FLAG_CONTINUATION if continuation else 0)
+        rc = _lib.lib().fss_scan_forward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(views[0]),
+                                               ctypes.byref(views[1]), ctypes.byref(views[2]), lam.data_ptr(),
+                                               ctypes.byref(views[3]), ctypes.byref(state) if state is not None else None)
     _lib.check(rc, "fss_scan_forward_gated")
 
 
@@ -316,12 +326,11 @@ def scan_backward_gated(r, i, x, lam, h, grad_out):
         dlam = torch.empty(D, dtype=torch.float32, device=r.device)
         tensors = [_rowwise(t) for t in (r, i, x, h, grad_out)] + [dr, di, dx]
         v = [_view(t) for t in tensors]
-        ws = _workspace_for(r, _DTYPES[dtype], "fss_gated_backward_workspace_bytes")
-        ctx = _ctx(r.device, ws, None)
-        rc = _lib.lib().fss_scan_backward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(v[0]),
-                                                ctypes.byref(v[1]), ctypes.byref(v[2]), lam.data_ptr(),
-                                                *[ctypes.byref(w) for w in v[3:]], dlam.data_ptr())
-        workspace.launched(ws)
+        with _launch(r, _DTYPES[dtype], "fss_gated_backward_workspace_bytes") as ws:
+            ctx = _ctx(r.device, ws, None)
+            rc = _lib.lib().fss_scan_backward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(v[0]),
+                                                    ctypes.byref(v[1]), ctypes.byref(v[2]), lam.data_ptr(),
+                                                    *[ctypes.byref(w) for w in v[3:]], dlam.data_ptr())
         if rc == 0:
             return dr, di, dx, dlam
         if rc != _lib.E_LAYOUT:

@@ -18,6 +18,13 @@ a device, every launch records an event and a launch on another stream first wai
 of the launch before it.  A process that only ever uses one stream per device pays nothing for
 this.  Kernels of other libraries that merely occupy SMs for a while (a collective, a GEMM on
 another stream) only delay a launch; they cannot dead-lock it.
+
+Threads
+-------
+From the look-up of its workspace until its launch is recorded, a call holds the device's lock
+(:class:`Launch`; the C++ functions hold the same lock).  A launch of another thread therefore comes
+entirely before it or entirely after it: it sees the launch and can fence it, and a workspace is never
+replaced by a larger one between the look-up and the launch.
 """
 from __future__ import annotations
 
@@ -35,9 +42,11 @@ _devices: dict[int, "_DeviceOrder"] = {}
 class _DeviceOrder:
     """Which stream launched last on a device, and -- once more than one stream is in play -- the
     event that marks the end of that launch."""
-    __slots__ = ("last", "multi", "event")
+    __slots__ = ("last", "multi", "event", "lock")
 
     def __init__(self):
+        # reentrant: a finalizer that runs inside the critical section may launch a scan itself
+        self.lock = threading.RLock()
         self.last = None        # Workspace of the most recent launch
         self.multi = False      # a second stream has been seen on this device
         self.event = None       # torch.cuda.Event recorded after the most recent launch (multi only)
@@ -48,10 +57,10 @@ class Workspace:
         self.device = device
         self.stream_handle = stream_handle
         self.buf = None
-        self.ctx = None          # the ScanCtx struct handed to the library (built by the caller)
+        self.ctx = None          # ScanCtx of this buffer as bytes: every launch makes its own copy (built by the caller)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._flag = self.status.numpy()      # same memory, read without going through torch
-        self.order = _devices.setdefault(device.index, _DeviceOrder())
+        self.order = _order(device)
         self._event = None
 
     def stream(self) -> torch.cuda.Stream:
@@ -106,8 +115,20 @@ def current_stream_handle(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def _order(device: torch.device) -> _DeviceOrder:
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    order = _devices.get(index)
+    return order if order is not None else _devices.setdefault(index, _DeviceOrder())
+
+
 def get(device: torch.device, nbytes: int) -> Workspace:
-    """Workspace of the current stream of ``device``, at least ``nbytes`` large."""
+    """Workspace of the current stream of ``device``, at least ``nbytes`` large.  For a launch that uses its
+    memory or counts as a single-pass launch, take it through :class:`Launch`."""
+    with _order(device).lock:
+        return _get(device, nbytes)
+
+
+def _get(device: torch.device, nbytes: int) -> Workspace:
     stream = current_stream_handle(device)
     key = (device.index, stream)
     ws = _cache.get(key)
@@ -128,8 +149,32 @@ def get(device: torch.device, nbytes: int) -> Workspace:
     return ws
 
 
+class Launch:
+    """``with Launch(device, nbytes) as ws``: one launch on the current stream, ordered against those of other
+    streams and threads; the body enqueues it."""
+    __slots__ = ("device", "nbytes", "lock", "ws")
+
+    def __init__(self, device: torch.device, nbytes: int):
+        self.device, self.nbytes, self.lock = device, nbytes, _order(device).lock
+
+    def __enter__(self) -> Workspace:
+        self.lock.acquire()
+        try:
+            self.ws = _get(self.device, self.nbytes)
+        except BaseException:
+            self.lock.release()
+            raise
+        return self.ws
+
+    def __exit__(self, *exc) -> None:
+        try:
+            launched(self.ws)
+        finally:
+            self.lock.release()
+
+
 def launched(ws: Workspace) -> None:
-    """Called after a launch on ``ws``'s stream."""
+    """Called after a launch on ``ws``'s stream, with the device's lock held since its workspace was looked up."""
     order = ws.order
     order.last = ws
     if order.multi and not torch.cuda.is_current_stream_capturing():
@@ -145,7 +190,8 @@ def check_status(device=None) -> None:
     with _lock:
         items = list(_cache.values())
     for ws in items:
-        ws.raise_if_flagged()
+        with ws.order.lock:
+            ws.raise_if_flagged()
 
 
 def release_all() -> None:

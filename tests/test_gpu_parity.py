@@ -1144,6 +1144,47 @@ def test_launches_on_two_streams_are_ordered_and_correct():
         assert_parity(x["da"], o_da, BF16_TOL, f"stream {k}: dalpha")
 
 
+@pytest.mark.parametrize("own_streams", [True, False])
+def test_threads_launch_on_one_device(own_streams):
+    """Two host threads, on streams of their own or on one stream, each with its own flags (forward in time; reversed
+    and continued), from the device's very first launch on: every result is what the call gives alone."""
+    import threading
+    pkg, _, _ = _mods()
+    from fast_sequential_scan_b200 import workspace
+    gen = torch.Generator(device="cuda").manual_seed(14)
+    a = torch.sigmoid(torch.randn(2, 2048, 512, generator=gen, device="cuda"))
+    b, h0, g = (torch.randn(s, generator=gen, device="cuda") for s in ((2, 2048, 512), (2, 512), (2, 2048, 512)))
+    calls = [lambda x: pkg.scan_cu_single(x, b), lambda x: pkg.scan_cu_single(x, b, h0=h0, reverse=True)]
+
+    def outputs(call):
+        x = a.detach().requires_grad_()
+        h = call(x)
+        return h.detach(), torch.autograd.grad(h, x, g)[0]
+    want = [outputs(call) for call in calls]
+    pkg.check_status()
+    workspace.release_all()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()] if own_streams else [torch.cuda.Stream()] * 2
+    start, got = threading.Barrier(2), [[], []]
+
+    def work(k):
+        start.wait(30)
+        with torch.cuda.stream(streams[k]):
+            for _ in range(30):
+                got[k].append(outputs(calls[k]))
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    pkg.check_status()
+    for k in range(2):
+        assert len(got[k]) == 30
+        for x in got[k]:
+            for u, v, name in zip(x, want[k], ("h", "dalpha")):
+                # association only: a few ulp of the state (|h| <~ 5, so |dalpha| <~ 25), relative to its size where terms cancel
+                assert bool(((u - v).abs() <= 2.0 ** -18 * (v.abs() + 5.0)).all()), (k, name)
+
+
 def test_bounded_waits_give_up_report_and_recover():
     """Failure detection without a fault: the first row block is told to publish no descriptors
     (a flag that nothing sets), waits are shortened; the tiles behind it must give up, set the

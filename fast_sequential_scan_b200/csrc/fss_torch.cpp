@@ -101,6 +101,16 @@ bool ordinary(const Tensor &t, const Tensor &first, at::ScalarType dtype) {
     return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.scalar_type() == dtype && t.dim() == 3 &&
            t.sizes() == first.sizes() && t.device() == first.device() && t.numel() > 0;
 }
+bool ordinary_vector(const Tensor &t, const Tensor &like, at::IntArrayRef sizes) {
+    return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.scalar_type() == at::kFloat && t.device() == like.device() &&
+           t.sizes() == sizes && t.is_contiguous();
+}
+// What the backward unpacks need not be what the forward saved: saved-tensor hooks may return anything.
+// The engine has checked the gradients against the outputs, so the saved tensors are checked against them.
+void check_unpacked(const Tensor &t, const Tensor &grad, const char *name) {
+    TORCH_CHECK(ordinary(t, grad, grad.scalar_type()), name, ": the saved tensor came back as ", t.toString(), t.sizes(), " on ", t.device(),
+                ", expected ", grad.toString(), grad.sizes(), " on ", grad.device());
+}
 
 struct Scan : torch::autograd::Function<Scan> {
     static variable_list forward(AutogradContext *ctx, const Tensor &alpha, const Tensor &beta, const std::optional<Tensor> &state0, bool want_final,
@@ -126,6 +136,10 @@ struct Scan : torch::autograd::Function<Scan> {
         py::gil_scoped_acquire gil;
         const variable_list saved = ctx->get_saved_variables();
         const Tensor &alpha = saved[0], &h0 = saved[2];
+        check_unpacked(alpha, grads[0], "alpha_saved");
+        check_unpacked(saved[1], grads[0], "h_saved");
+        TORCH_CHECK(!h0.defined() || ordinary_vector(h0, alpha, {alpha.size(0), alpha.size(2)}),
+                    "h_prev: expected a contiguous fp32 CUDA tensor of ", alpha.size(0), "x", alpha.size(2), " elements");
         const bool reverse = ctx->saved_data["reverse"].toBool();
         const Shape s(alpha);
         const Tensor a = rowwise(alpha), h = rowwise(saved[1]);
@@ -162,18 +176,22 @@ struct Gated : torch::autograd::Function<Gated> {
         py::gil_scoped_acquire gil;
         const variable_list saved = ctx->get_saved_variables();
         const Tensor &r = saved[0], &lam = saved[3];
+        const auto any_layout = [&] {      // or a refusal, worded there
+            const py::tuple out = py::reinterpret_borrow<py::object>(py_gated_backward)(r, saved[1], saved[2], lam, saved[4], grads[0]);
+            return variable_list{out[0].cast<Tensor>(), out[1].cast<Tensor>(), out[2].cast<Tensor>(), out[3].cast<Tensor>()};
+        };
+        for (int k : {0, 1, 2, 4})
+            if (!ordinary(saved[k], grads[0], grads[0].scalar_type())) return any_layout();
+        if (!ordinary_vector(lam, r, {r.size(2)})) return any_layout();
         const Shape s(r);
         const Tensor g = placed(grads[0].contiguous()), dr = like(r), di = like(r), dx = like(r), dlam = at::empty_like(lam);
-        const Tensor rr = rowwise(r), ri = rowwise(saved[1]), rx = rowwise(saved[2]), rh = rowwise(saved[4]), l = lam.contiguous();
+        const Tensor rr = rowwise(r), ri = rowwise(saved[1]), rx = rowwise(saved[2]), rh = rowwise(saved[4]);
         const fss_view vr = view(rr), vi = view(ri), vx = view(rx), vh = view(rh), vg = view(g), v0 = view(dr), v1 = view(di), v2 = view(dx);
         Launch go(r, s, 0, true);
-        const int rc = lib.backward_gated(&go.ctx, s.dtype, s.B, s.T, s.D, &vr, &vi, &vx, l.data_ptr<float>(), &vh, &vg, &v0, &v1, &v2,
+        const int rc = lib.backward_gated(&go.ctx, s.dtype, s.B, s.T, s.D, &vr, &vi, &vx, lam.data_ptr<float>(), &vh, &vg, &v0, &v1, &v2,
                                           dlam.data_ptr<float>());
         go.done();
-        if (rc == FSS_E_LAYOUT) {      // saved-tensor hooks handed back copies that lie otherwise, say
-            const py::tuple out = py::reinterpret_borrow<py::object>(py_gated_backward)(r, saved[1], saved[2], lam, saved[4], grads[0]);
-            return {out[0].cast<Tensor>(), out[1].cast<Tensor>(), out[2].cast<Tensor>(), out[3].cast<Tensor>()};
-        }
+        if (rc == FSS_E_LAYOUT) return any_layout();      // saved-tensor hooks handed back copies that lie otherwise, say
         if (rc != FSS_OK) py::reinterpret_borrow<py::object>(py_check)(rc, "fss_scan_backward_gated");      // raises
         return {dr, di, dx, dlam};
     }
@@ -183,9 +201,7 @@ struct Gated : torch::autograd::Function<Gated> {
 py::object scan(const Tensor &alpha, const Tensor &beta, const std::optional<Tensor> &h0, bool want_final, bool reverse, bool bf16) {
     const at::ScalarType dtype = bf16 ? at::kBFloat16 : at::kFloat;
     if (alpha.dim() != 3 || !ordinary(alpha, alpha, dtype) || !ordinary(beta, alpha, dtype)) return py::none();
-    if (h0 && !(h0->is_cuda() && h0->layout() == at::kStrided && h0->scalar_type() == at::kFloat && h0->device() == alpha.device() &&
-                h0->dim() == 2 && h0->size(0) == alpha.size(0) && h0->size(1) == alpha.size(2) && h0->is_contiguous()))
-        return py::none();
+    if (h0 && !ordinary_vector(*h0, alpha, {alpha.size(0), alpha.size(2)})) return py::none();
     if (reverse && !(addressable(alpha) && addressable(beta))) return py::none();
     variable_list out = Scan::apply(alpha, beta, h0, want_final, reverse);
     if (want_final) return py::make_tuple(out[0], out[1]);
@@ -196,9 +212,7 @@ py::object gated(const Tensor &r, const Tensor &i, const Tensor &x, const Tensor
     if (r.dim() != 3 || (r.scalar_type() != at::kBFloat16 && r.scalar_type() != at::kFloat)) return py::none();
     for (const Tensor *t : {&r, &i, &x})
         if (!ordinary(*t, r, r.scalar_type()) || !t->is_contiguous() || !addressable(*t)) return py::none();
-    if (!(lam.is_cuda() && lam.layout() == at::kStrided && lam.scalar_type() == at::kFloat && lam.device() == r.device() && lam.dim() == 1 &&
-          lam.size(0) == r.size(2) && lam.is_contiguous()))
-        return py::none();
+    if (!ordinary_vector(lam, r, {r.size(2)})) return py::none();
     return py::cast(Gated::apply(r, i, x, lam));
 }
 

@@ -660,6 +660,42 @@ def test_cpp_functions_match_the_python_classes(form, dtype, monkeypatch):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("unpack", ["other type", "fewer channels", "fewer rows", "other device", "transposed"])
+@pytest.mark.parametrize("op", ["scan", "state", "gated"])
+def test_tensors_that_hooks_unpack_are_checked(op, unpack):
+    """Saved-tensor hooks may return anything.  What the backward cannot read as what the forward saved is refused on the
+    host, as by the Python classes; the same values that only lie otherwise are taken."""
+    pkg, _, _ = _mods()
+    gen = torch.Generator(device="cuda").manual_seed(15)
+    a, b, c = (torch.sigmoid(torch.randn(2, 33, 40, generator=gen, device="cuda")) for _ in range(3))
+    h0, lam = torch.randn(2, 40, generator=gen, device="cuda"), torch.randn(40, generator=gen, device="cuda")
+    change = {"other type": lambda t: t.to(torch.bfloat16), "fewer channels": lambda t: t[..., :-8].contiguous(), "fewer rows": lambda t: t[:, :-1],
+              "other device": lambda t: t.cpu(), "transposed": lambda t: t.mT.contiguous().mT if t.dim() == 3 else t}[unpack]
+    for k in range({"scan": 2, "state": 3, "gated": 5}[op]):           # which of the saved tensors the hook changes
+        if unpack == "fewer rows" and (op, k) == ("gated", 3):
+            continue                                                    # lam has no rows
+        leaves = [t.detach().requires_grad_() for t in {"scan": (a, b), "state": (a, b, h0), "gated": (a, b, c, lam)}[op]]
+        call = {"scan": lambda x, y: pkg.scan_cu_single(x, y), "state": lambda x, y, z: pkg.scan_cu_single(x, y, h0=z),
+                "gated": lambda *t: pkg.scan_gated(*t)}[op]
+        want = torch.autograd.grad(call(*leaves).sum(), leaves)
+        seen = []
+
+        def unpacked(t):
+            seen.append(t)
+            return change(t) if len(seen) == k + 1 else t
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), unpacked):
+            h = call(*leaves)
+        g = torch.ones_like(h)
+        if unpack == "transposed":
+            for x, y in zip(torch.autograd.grad(h, leaves, g), want):
+                assert bool(((x - y).abs() <= 2.0 ** -18 * (y.abs() + 5.0)).all())
+        else:
+            with pytest.raises(RuntimeError):
+                torch.autograd.grad(h, leaves, g)
+        assert len(seen) > k
+    pkg.check_status()
+
+
 def test_calls_that_stay_with_the_python_classes():
     """Autocast, transforms, forward-mode tensors and everything that is refused go to the Python classes."""
     pkg, _, _ = _mods()

@@ -43,6 +43,7 @@ struct Params {
     const float *h_prev;      // backward only
     int continuation;
     uint32_t max_spins;
+    int mute_first_block;     // test hook: row block 0 publishes no descriptors (its successors' waits run out)
 };
 
 // P * s + c where a state of exactly zero also absorbs a product that has overflowed
@@ -262,6 +263,7 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
             if (threadIdx.x == 0 && (++spins & 15u) == 0u) {
                 if (spins >= p.max_spins) {
                     atomicExch(&p.hdr->abort, 1u);
+                    __threadfence();           // ahead of this CTA's count, so that the last CTA's reset comes after it
                     report_status(p.status, FSS_STATUS_LOOKBACK_TIMEOUT);
                 }
                 if (lookback::ld_volatile(&p.hdr->abort)) s_abort = 1;
@@ -289,8 +291,11 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             const float tile_out = apply(tP[v], cin[v], tC[v]);
-            if (!last_block) store_cell(inc_cell(tile, v), tile_out, tag_inc);
-            else if (p.state_out && ch_ok) p.state_out[b * p.D + d + v] = tile_out;
+            if (last_block) {
+                if (p.state_out && ch_ok) p.state_out[b * p.D + d + v] = tile_out;
+            } else if (s > 0 || !p.mute_first_block) {
+                store_cell(inc_cell(tile, v), tile_out, tag_inc);
+            }
         }
     }
     // counted here, so that the answer arrives while the results are written (with a fence at the CTA's end
@@ -362,6 +367,7 @@ inline int launch_lots(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int
     p.status = ctx->status;
     p.continuation = (ctx->flags & FSS_FLAG_CONTINUATION) ? 1 : 0;
     p.max_spins = (ctx->flags & FSS_FLAG_TEST_SHORT_WAITS) ? 4096u : lookback::kMaxSpins / 4;      // (a round of the window takes several times a poll)
+    p.mute_first_block = (ctx->flags & FSS_FLAG_TEST_MUTE_FIRST_BLOCK) ? 1 : 0;
     const unsigned grid = (unsigned)tiles(B, Tn, D, V);
     const cudaStream_t stream = (cudaStream_t)ctx->stream;
     if (sizeof(T) == 2 && p.ncols >= 2 * 148)      // (a wave: two CTAs per SM)

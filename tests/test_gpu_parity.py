@@ -1250,6 +1250,40 @@ def test_bounded_waits_give_up_report_and_recover():
     assert_parity(h, ref.float(), BF16_TOL, "h after recovery")
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(2, 4096, 33), (8, 1100, 1501), (4, 1100, 5002)])
+def test_bounded_waits_of_the_any_layout_kernels(shape, dtype):
+    """The same for the kernels that take odd widths, in both directions: few columns; columns enough for the look ahead
+    of the loads (bf16), by one and by two channels per lane.  The launch after it, on the same workspace, is healthy."""
+    pkg, native, _lib = _mods()
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    a = torch.sigmoid(torch.randn(shape, generator=gen, device="cuda")).to(dtype)
+    b, g = (torch.randn(shape, generator=gen, device="cuda").to(dtype) for _ in range(2))
+    test = _lib.FLAG_TEST_SHORT_WAITS | _lib.FLAG_TEST_MUTE_FIRST_BLOCK
+
+    def forward(algo=None, flags=0):
+        h = torch.empty_like(a)
+        native._launch_forward(a, b, h, native._DTYPES[dtype], algo, flags, None)
+        return (h,)
+
+    def backward(algo=None, flags=0):
+        da, db = torch.empty_like(a), torch.empty_like(a)
+        native._launch_backward(a, h_ref, g, da, db, native._DTYPES[dtype], algo, flags, None)
+        return da, db
+    h_ref, = forward(_lib.ALGO_CHUNKED)
+    for run in (forward, backward):
+        ref = run(_lib.ALGO_CHUNKED)
+        pkg.check_status()
+        run(flags=test)
+        torch.cuda.synchronize()                                      # the kernel must terminate by itself
+        with pytest.raises(RuntimeError, match="look-back timeout"):
+            pkg.check_status()
+        for _ in range(2):
+            for x, y in zip(run(), ref):
+                assert_parity(x, y.float(), BF16_TOL if dtype == torch.bfloat16 else F32_TOL, "after recovery")
+        pkg.check_status()
+
+
 def test_config5_full_length_on_one_gpu():
     """The whole 524,288-row sequence of configuration 5 (2.1 G elements, 4.3 GB per tensor) on one
     device: 64-bit offsets, 2,048 row blocks per column.  Oracle on a channel subset, all rows."""

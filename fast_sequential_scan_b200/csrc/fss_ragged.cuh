@@ -149,15 +149,17 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
     // Forward: scan row 0; backward: scan row T-1.
     const int64_t head_off = (kBackward ? p.T - 1 : 0) - i0;
     const int head = head_off >= 0 && head_off < n ? (int)head_off : -1;
+    // the state before that row (backward), in 32 bits: fp32 rows have a place for it, bf16 rows get it at their end
+    const bool has_prev = kBackward && head >= 0 && p.continuation && p.h_prev;
     if (head >= 0) {
         float prev[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) prev[v] = kBackward && p.continuation && p.h_prev ? p.h_prev[b * p.D + d + v] : 0.0f;
+        for (int v = 0; v < V; ++v) prev[v] = sizeof(T) == 4 && has_prev ? p.h_prev[b * p.D + d + v] : 0.0f;
 #pragma unroll
         for (int j = 0; j < kRows; ++j)
             if (j == head) {
                 if (!p.continuation) ra[j] = zero;
-                if (kBackward) rh[j] = L::put(prev);
+                if (kBackward && sizeof(T) == 4) rh[j] = L::put(prev);
             }
     }
 
@@ -310,6 +312,9 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
             st[v] = cin[v];
             for (int w = 0; w < warp; ++w) st[v] = apply(sP[v][w][lane], st[v], sC[v][w][lane]);
         }
+        float prev[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) prev[v] = sizeof(T) == 2 && has_prev ? p.h_prev[b * p.D + d + v] : 0.0f;
         T *p0 = out0.row(b, i0) + d, *p1 = kBackward ? out1.row(b, i0) + d : nullptr;
 #pragma unroll
         for (int j = 0; j < kRows; ++j) {
@@ -323,7 +328,7 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
                     st[v] = fmaf(a[v], st[v], y[v]);
                 } else {
                     dh[v] = y[v] + st[v];
-                    da[v] = j == head && !p.continuation ? 0.0f : dh[v] * hp[v];
+                    da[v] = j == head && !p.continuation ? 0.0f : dh[v] * (j == head && sizeof(T) == 2 ? prev[v] : hp[v]);
                     st[v] = a[v] * dh[v];
                 }
             }

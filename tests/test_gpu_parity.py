@@ -582,6 +582,27 @@ def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("shape", [(3, 1, 33), (2, 129, 100), (2, 300, 1001)])
+def test_any_layout_kernel_keeps_the_state_before_the_first_row_in_32_bits(shape, reverse):
+    """bf16 with a state whose low bits matter: the first row's dalpha is dh * h0, rounded once.  With dh = grad exactly (the
+    gradient of the last row alone in one-row scans; alpha = 0 after the first row otherwise) the product is exact in
+    64 bits, so the result is its nearest bf16 (half a unit: at most 2^-8 of the value) up to the rounding of the fp32 product
+    (2^-24): 2^-8 * (1 + 2^-14) of the value.  With h0 rounded as well it would be up to twice that."""
+    pkg, native, _ = _mods()
+    B, T, D = shape
+    gen = torch.Generator(device="cuda").manual_seed(16)
+    h0 = torch.randn(B, D, generator=gen, device="cuda")
+    a, h = torch.zeros(shape, dtype=torch.bfloat16, device="cuda"), torch.randn(shape, generator=gen, device="cuda").bfloat16()
+    g = torch.randn(shape, generator=gen, device="cuda").bfloat16()
+    da, db = torch.empty_like(a), torch.empty_like(a)
+    native.backward_into(a, h, g, da, db, continuation=True, h_prev=h0, reverse=reverse)
+    pkg.check_status()
+    first = T - 1 if reverse else 0
+    want = g[:, first].double() * h0.double()
+    assert bool(((da[:, first].double() - want).abs() <= 2.0 ** -8 * (1 + 2.0 ** -14) * want.abs()).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(1, 1, 1), (16, 1, 2560), (3, 2, 33), (2, 7, 24), (130, 8, 520), (2, 9, 264)])
 def test_forward_of_a_few_rows_matches_the_chunked_kernels(shape, dtype):

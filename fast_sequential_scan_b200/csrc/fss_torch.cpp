@@ -7,8 +7,9 @@
 // two launches through Python classes took 129 us a step, through these 76; decoding 33 and 13 us a call.
 //
 // The library is reached through the addresses that the package's ctypes table holds, and the streams'
-// workspaces stay with workspace.py: one Python call per launch, under the GIL, takes the device's lock
-// and returns what the context is made of.
+// workspaces stay with workspace.py: one Python call per launch takes the device's lock and returns what
+// the context is made of.  The GIL is held for such calls only, not for allocations, copies and launches,
+// any of which may block (memory to reclaim, a full launch queue).
 #include <torch/extension.h>
 
 #include <cstring>
@@ -38,12 +39,13 @@ struct Shape {
     explicit Shape(const Tensor &t) : B(t.size(0)), T(t.size(1)), D(t.size(2)), dtype(t.scalar_type() == at::kBFloat16 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32) {}
 };
 
-// One launch, with a context of its own.  The device's lock (workspace.py) is held from the look-up of
-// the workspace until the launch is recorded; the GIL is held while this lives.
+// One launch, with a context of its own, made without the GIL.  The device's lock (workspace.py) is held
+// from the look-up of the workspace until the launch is recorded, by the thread that makes the launch.
 struct Launch {
     fss_scan_ctx ctx;
-    py::object release, workspace;
+    PyObject *release = nullptr, *workspace = nullptr;      // owned; None: nobody wants to hear of the launch
     Launch(const Tensor &t, const Shape &s, int flags, bool gated_backward = false) {
+        py::gil_scoped_acquire gil;
         const py::object got = py::reinterpret_steal<py::object>(PyObject_CallFunction(py_acquire, "iLLLii", (int)t.get_device(), (long long)s.B,
                                                                                        (long long)s.T, (long long)s.D, s.dtype, (int)gated_backward));
         if (!got) throw py::error_already_set();
@@ -51,24 +53,30 @@ struct Launch {
         std::memcpy(&ctx, PyBytes_AS_STRING(item(0)), sizeof ctx);
         ctx.algo = (int32_t)PyLong_AsLong(item(1));
         ctx.flags = (int32_t)PyLong_AsLong(item(2)) | flags;
-        release = py::reinterpret_borrow<py::object>(item(3));
-        workspace = py::reinterpret_borrow<py::object>(item(4));
+        release = Py_NewRef(item(3));
+        workspace = Py_NewRef(item(4));
     }
     Launch(const Launch &) = delete;
     ~Launch() {
         if (!release) return;
+        py::gil_scoped_acquire gil;
         py::error_scope keep;      // (an error that is on its way)
-        Py_XDECREF(PyObject_CallNoArgs(release.ptr()));
+        give_back();
+        PyErr_Clear();
     }
     // after the call of the library
-    void done() {
-        if (!workspace.is_none()) py::reinterpret_borrow<py::object>(py_launched)(workspace);
-        py::object r = std::move(release);
-        r();
-    }
-    void done(int rc, const char *where) {
-        done();
+    void done(int rc = FSS_OK, const char *where = nullptr) {
+        py::gil_scoped_acquire gil;
+        if (workspace != Py_None) py::reinterpret_borrow<py::object>(py_launched)(py::handle(workspace));
+        give_back();
         if (rc != FSS_OK) py::reinterpret_borrow<py::object>(py_check)(rc, where);      // raises
+    }
+
+  private:
+    void give_back() {
+        Py_XDECREF(PyObject_CallNoArgs(release));
+        Py_CLEAR(release);
+        Py_CLEAR(workspace);
     }
 };
 
@@ -133,7 +141,6 @@ struct Scan : torch::autograd::Function<Scan> {
         return {h};
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        py::gil_scoped_acquire gil;
         const variable_list saved = ctx->get_saved_variables();
         const Tensor &alpha = saved[0], &h0 = saved[2];
         check_unpacked(alpha, grads[0], "alpha_saved");
@@ -173,10 +180,10 @@ struct Gated : torch::autograd::Function<Gated> {
         return h;
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        py::gil_scoped_acquire gil;
         const variable_list saved = ctx->get_saved_variables();
         const Tensor &r = saved[0], &lam = saved[3];
         const auto any_layout = [&] {      // or a refusal, worded there
+            py::gil_scoped_acquire gil;
             const py::tuple out = py::reinterpret_borrow<py::object>(py_gated_backward)(r, saved[1], saved[2], lam, saved[4], grads[0]);
             return variable_list{out[0].cast<Tensor>(), out[1].cast<Tensor>(), out[2].cast<Tensor>(), out[3].cast<Tensor>()};
         };
@@ -190,9 +197,8 @@ struct Gated : torch::autograd::Function<Gated> {
         Launch go(r, s, 0, true);
         const int rc = lib.backward_gated(&go.ctx, s.dtype, s.B, s.T, s.D, &vr, &vi, &vx, lam.data_ptr<float>(), &vh, &vg, &v0, &v1, &v2,
                                           dlam.data_ptr<float>());
-        go.done();
+        go.done(rc == FSS_E_LAYOUT ? FSS_OK : rc, "fss_scan_backward_gated");
         if (rc == FSS_E_LAYOUT) return any_layout();      // saved-tensor hooks handed back copies that lie otherwise, say
-        if (rc != FSS_OK) py::reinterpret_borrow<py::object>(py_check)(rc, "fss_scan_backward_gated");      // raises
         return {dr, di, dx, dlam};
     }
 };
@@ -203,7 +209,10 @@ py::object scan(const Tensor &alpha, const Tensor &beta, const std::optional<Ten
     if (alpha.dim() != 3 || !ordinary(alpha, alpha, dtype) || !ordinary(beta, alpha, dtype)) return py::none();
     if (h0 && !ordinary_vector(*h0, alpha, {alpha.size(0), alpha.size(2)})) return py::none();
     if (reverse && !(addressable(alpha) && addressable(beta))) return py::none();
-    variable_list out = Scan::apply(alpha, beta, h0, want_final, reverse);
+    const variable_list out = [&] {
+        py::gil_scoped_release no_gil;
+        return Scan::apply(alpha, beta, h0, want_final, reverse);
+    }();
     if (want_final) return py::make_tuple(out[0], out[1]);
     return py::cast(out[0]);
 }
@@ -213,7 +222,11 @@ py::object gated(const Tensor &r, const Tensor &i, const Tensor &x, const Tensor
     for (const Tensor *t : {&r, &i, &x})
         if (!ordinary(*t, r, r.scalar_type()) || !t->is_contiguous() || !addressable(*t)) return py::none();
     if (!ordinary_vector(lam, r, {r.size(2)})) return py::none();
-    return py::cast(Gated::apply(r, i, x, lam));
+    const Tensor h = [&] {
+        py::gil_scoped_release no_gil;
+        return Gated::apply(r, i, x, lam);
+    }();
+    return py::cast(h);
 }
 
 void bind(uintptr_t forward, uintptr_t backward, uintptr_t forward_gated, uintptr_t backward_gated, py::object acquire, py::object launched,

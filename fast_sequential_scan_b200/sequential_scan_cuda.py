@@ -121,6 +121,7 @@ def _ctx(device: torch.device, ws: workspace.Workspace, algo: Optional[int], fla
 
 
 _torch_devices: dict = {}
+_acquire_bytes: dict = {}      # workspace bytes per (B, T, D, dtype, gated backward)
 
 
 def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: int):
@@ -130,15 +131,20 @@ def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: 
     device = _torch_devices.get(index)
     if device is None:
         device = _torch_devices[index] = torch.device("cuda", index)
-    need = _workspace_bytes((B, T, D), dtype_id, "fss_gated_backward_workspace_bytes" if gated_backward else "fss_workspace_bytes")
-    lock = workspace._order(device).lock
+    # (looked up here rather than through helpers: this runs once per launch of the C++ functions)
+    key = (B, T, D, dtype_id, gated_backward)
+    need = _acquire_bytes.get(key)
+    if need is None:
+        query = _lib.lib().fss_gated_backward_workspace_bytes if gated_backward else _lib.lib().fss_workspace_bytes
+        need = _acquire_bytes[key] = query(B, T, D, dtype_id)
+    lock = (workspace._devices.get(index) or workspace._order(device)).lock
     lock.acquire()
     try:
         ws = workspace._get(device, need)
-        ctx, algo, order = _ctx_bytes(device, ws), default_algo(), ws.order
+        ctx, algo, order = ws.ctx or _ctx_bytes(device, ws), default_algo(), ws.order
         if not order.multi:      # (stays as it is while the lock is held)
             order.last, ws = ws, None
-        return ctx, algo, _call_flags(), lock.release, ws
+        return ctx, algo, _lib.FLAG_DETERMINISTIC if _deterministic else 0, lock.release, ws
     except BaseException:
         lock.release()
         raise

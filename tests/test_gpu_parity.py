@@ -717,6 +717,28 @@ def test_tensors_that_hooks_unpack_are_checked(op, unpack):
     pkg.check_status()
 
 
+def test_cpp_functions_do_not_hold_the_gil_over_a_launch():
+    """Other Python threads run while a launch blocks (a full launch queue, say).  In the library's place stands
+    ``PyGILState_Check``: 0, which is success, without the GIL; 1, an error code, with it.  No kernel is launched."""
+    import ctypes
+    pkg, native, _lib = _mods()
+    from fast_sequential_scan_b200 import _fss_torch, workspace
+    python = (native._acquire, workspace.launched, _lib.check, native.scan_backward_gated)
+    names = ("fss_scan_forward_ex", "fss_scan_backward_ex", "fss_scan_forward_gated", "fss_scan_backward_gated")
+    t = [torch.ones(2, 9, 16, device="cuda").requires_grad_() for _ in range(3)]
+    lam, g = torch.ones(16, device="cuda").requires_grad_(), torch.ones(2, 9, 16, device="cuda")
+    probe = ctypes.cast(ctypes.pythonapi.PyGILState_Check, ctypes.c_void_p).value
+    _fss_torch.bind(*[probe] * 4, *python)
+    try:
+        torch.autograd.grad(pkg.scan_cu_single(t[0], t[1]), t[:2], g)
+        torch.autograd.grad(pkg.scan_gated(*t, lam), [*t, lam], g)
+    finally:
+        _fss_torch.bind(*[native._address(n) for n in names], *python)
+    h = pkg.scan_cu_single(t[0], t[1])
+    assert bool((h[0, :, 0] == torch.arange(1.0, 10.0, device="cuda")).all())
+    pkg.check_status()
+
+
 def test_calls_that_stay_with_the_python_classes():
     """Autocast, transforms, forward-mode tensors and everything that is refused go to the Python classes."""
     pkg, _, _ = _mods()

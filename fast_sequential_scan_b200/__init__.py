@@ -3,9 +3,7 @@
 counterpart here."""
 from . import _lib
 
-_lib.lib()   # fail at import time, loudly, when the native libraries have not been built
-if not (_lib.PKG / "_fss_torch.so").is_file():
-    raise ImportError(f"{_lib.PKG / '_fss_torch.so'} is missing: build it with `python fast_sequential_scan_b200/build.py`")
+_lib.lib()   # fail at import time, loudly, when the native library has not been built
 
 from .scan_cuda import scan as scan_cu  # noqa: E402
 from .scan_cuda import scan_single as scan_cu_single  # noqa: E402

@@ -1,5 +1,7 @@
 """In-tree build of ``libfss_b200.so`` (the C-ABI CUDA library) with plain nvcc for sm_100a, and of
-``_fss_torch.so`` (the autograd side of the entry points, ``csrc/fss_torch.cpp``) with g++ against torch.
+``_fss_torch*.so`` (the autograd side of the entry points, ``csrc/fss_torch.cpp``) with g++ against torch.
+The latter carries the Python and the torch it was compiled for in its name: one for another torch is neither
+taken for up to date here nor loaded by the package.
 
 The library needs no libtorch and no pybind: its only inputs are ``csrc/*.cu[h]`` and
 ``include/fss_b200.h``.  The results sit beside this file so that they travel with the source tree.  Run as
@@ -18,7 +20,6 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libfss_b200.so"
 TORCH_SOURCE = CSRC / "fss_torch.cpp"
-TORCH_LIB = PKG / "_fss_torch.so"
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17",
@@ -47,10 +48,17 @@ def is_stale() -> bool:
     return any(s.stat().st_mtime > t for s in sources() + [Path(__file__)])
 
 
+def torch_lib() -> Path:
+    """Where ``fss_torch.cpp`` is built for the running Python and torch."""
+    import torch
+    return PKG / f"_fss_torch.{sys.implementation.cache_tag}.torch-{torch.__version__}.so"
+
+
 def build_torch(force: bool = False) -> Path:
+    lib = torch_lib()
     inputs = [TORCH_SOURCE, PKG.parent / "include" / "fss_b200.h", Path(__file__)]
-    if not force and TORCH_LIB.is_file() and TORCH_LIB.stat().st_mtime >= max(p.stat().st_mtime for p in inputs):
-        return TORCH_LIB
+    if not force and lib.is_file() and lib.stat().st_mtime >= max(p.stat().st_mtime for p in inputs):
+        return lib
     import sysconfig
 
     import torch
@@ -58,13 +66,13 @@ def build_torch(force: bool = False) -> Path:
     includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", Path(sysconfig.get_paths()["include"])]
     cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
            "-DTORCH_EXTENSION_NAME=_fss_torch", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           *[f"-I{p}" for p in includes], str(TORCH_SOURCE), "-o", str(TORCH_LIB), f"-L{root / 'lib'}",
+           *[f"-I{p}" for p in includes], str(TORCH_SOURCE), "-o", str(lib), f"-L{root / 'lib'}",
            f"-Wl,-rpath,{root / 'lib'}", "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode:
         sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("g++ failed building _fss_torch.so")
-    return TORCH_LIB
+        raise RuntimeError(f"g++ failed building {lib.name}")
+    return lib
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

@@ -42,8 +42,8 @@ from typing import Any, Optional, Tuple
 import torch
 from torch.autograd import Function
 
-from . import _fss_torch, _lib
-from .sequential_scan_cuda import (backward_into, default_algo, forward_into, scan_backward, scan_backward_gated,
+from . import _lib
+from .sequential_scan_cuda import (_fss_torch, backward_into, default_algo, forward_into, scan_backward, scan_backward_gated,
                                    scan_backward_half, scan_forward, scan_forward_gated, scan_forward_half, tma_eligible)
 
 BACKWARD_MODES = ("saved", "inplace", "recompute")
@@ -168,6 +168,8 @@ _plain_types = (torch.Tensor, torch.nn.Parameter)
 def _ordinary_call(*tensors) -> bool:
     """Plain tensors, no autocast and nothing that traces, transforms or differentiates forward: calls that the C++
     functions may take.  All others keep to the Python classes, which torch knows how to treat there."""
+    if _fss_torch is None:
+        return False
     for t in tensors:
         if type(t) not in _plain_types:
             return False

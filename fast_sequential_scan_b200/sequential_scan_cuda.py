@@ -14,12 +14,15 @@ torch's current stream; shapes, devices and layouts are validated.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import warnings
 from typing import List, Optional
 
 import torch
 
-from . import _fss_torch, _lib, workspace
+from . import _lib, workspace
+from .build import torch_lib
 
 _DTYPES = {torch.bfloat16: _lib.DTYPE_BF16, torch.float32: _lib.DTYPE_F32}
 
@@ -393,8 +396,24 @@ def _address(name: str) -> int:
     return ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value
 
 
-_fss_torch.bind(_address("fss_scan_forward_ex"), _address("fss_scan_backward_ex"), _address("fss_scan_forward_gated"),
+def _load_fss_torch():
+    """The autograd functions in C++, or None: without them the Python classes serve all calls, with more host time
+    (the kernels are the same: they are in ``libfss_b200.so``, which there is no doing without)."""
+    path = torch_lib()
+    try:
+        spec = importlib.util.spec_from_file_location(f"{__package__}._fss_torch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError as e:
+        warnings.warn(f"{path} does not load ({e}): calls take tens of microseconds more of host time; build it with "
+                      "`python fast_sequential_scan_b200/build.py`", RuntimeWarning, stacklevel=3)
+        return None
+    module.bind(_address("fss_scan_forward_ex"), _address("fss_scan_backward_ex"), _address("fss_scan_forward_gated"),
                 _address("fss_scan_backward_gated"), _acquire, workspace.launched, _lib.check, scan_backward_gated)
+    return module
+
+
+_fss_torch = _load_fss_torch()
 
 
 def _forward(alpha: torch.Tensor, beta: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

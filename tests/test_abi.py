@@ -159,3 +159,38 @@ def test_kernels_that_start_early_do_not_take_their_predecessors_data_for_consta
     for kernel in ("prescale", "backward_tables"):
         arguments = re.search(rf"__global__ void {kernel}\((.*?)\) \{{", gates, flags=re.S).group(1)
         assert "__restrict__" not in arguments, kernel
+
+
+@pytest.mark.parametrize("content", [None, b"not a shared object"])
+def test_import_without_the_cpp_autograd_functions(tmp_path, content):
+    """The Python classes serve every call by themselves: a missing ``_fss_torch`` file, or one that does not load, is a
+    warning.  A file that was built for another torch is not looked at."""
+    import shutil
+    import subprocess
+    import sys
+    package = ROOT / "fast_sequential_scan_b200"
+    copy = tmp_path / package.name
+    shutil.copytree(package, copy, ignore=shutil.ignore_patterns("*.so", "csrc", "__pycache__"))
+    (copy / "libfss_b200.so").symlink_to(package / "libfss_b200.so")
+    (copy / "_fss_torch.so").write_bytes(b"of another torch")
+    if content is not None:
+        from fast_sequential_scan_b200.build import torch_lib
+        (copy / torch_lib().name).write_bytes(content)
+    code = ("import warnings, torch\n"
+            "with warnings.catch_warnings(record=True) as seen:\n"
+            "    warnings.simplefilter('always')\n"
+            "    import fast_sequential_scan_b200 as pkg\n"
+            "    from fast_sequential_scan_b200 import scan_cuda\n"
+            "assert [w for w in seen if '_fss_torch' in str(w.message)], seen\n"
+            "assert not scan_cuda._ordinary_call(torch.ones(1, 2, 3))\n"
+            "try: pkg.scan_cu(torch.ones(1, 2, 3).bfloat16(), torch.ones(1, 2, 3).bfloat16())\n"
+            "except RuntimeError as e: assert 'CUDA tensor' in str(e)\n"
+            "else: raise AssertionError('no refusal')\n"
+            "print('imported from', pkg.__file__)\n")
+    out = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and str(tmp_path) in out.stdout, out.stdout + out.stderr
+
+
+def test_the_cpp_autograd_functions_load_here():
+    from fast_sequential_scan_b200 import scan_cuda
+    assert scan_cuda._fss_torch is not None

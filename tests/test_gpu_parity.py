@@ -722,7 +722,8 @@ def test_cpp_functions_do_not_hold_the_gil_over_a_launch():
     ``PyGILState_Check``: 0, which is success, without the GIL; 1, an error code, with it.  No kernel is launched."""
     import ctypes
     pkg, native, _lib = _mods()
-    from fast_sequential_scan_b200 import _fss_torch, workspace
+    from fast_sequential_scan_b200 import workspace
+    _fss_torch = native._fss_torch
     python = (native._acquire, workspace.launched, _lib.check, native.scan_backward_gated)
     names = ("fss_scan_forward_ex", "fss_scan_backward_ex", "fss_scan_forward_gated", "fss_scan_backward_gated")
     t = [torch.ones(2, 9, 16, device="cuda").requires_grad_() for _ in range(3)]

@@ -582,6 +582,38 @@ def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 2), (2, 15, 40), (1, 127, 66), (2, 129, 100), (3, 260, 130), (5, 400, 4098), (2, 300, 9478)])
+def test_any_layout_kernel_on_rows_that_4_byte_accesses_can_address(shape):
+    """bf16 with an even width and even strides from bases that are 4- but not 16-byte aligned: two channels per lane, the
+    last two shapes with columns enough (325 and 298) for the look ahead of the loads.  Both scan orders, with and without
+    boundary state, against the chunked kernels; bounds as for the any-layout kernel above."""
+    _, native, _ = _mods()
+    B, T, D = shape
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = (0.5 + 0.499 * torch.rand(B, T, D + 4, generator=gen, device="cuda")).bfloat16()[:, :, 2:D + 2]
+    b, g = (rnd(B, T, D + 4).bfloat16()[:, :, 2:D + 2] for _ in range(2))
+    h0, u0 = rnd(B, D), rnd(B, D)
+    for cont, reverse in [(False, False), (True, False), (False, True), (True, True)]:
+        runs = []
+        for algo in ("chunked", "auto", "auto"):
+            wide = [torch.full((B, T, D + 4), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+            h, da, db = (t[:, :, 2:D + 2] for t in wide)
+            last, u = torch.empty(B, D, device="cuda"), torch.empty(B, D, device="cuda")
+            native.forward_into(a, b, h, algo=_algo_id(algo), continuation=cont, h_in=h0 if cont else None, h_last=last, reverse=reverse)
+            native.backward_into(a, runs[0][0] if runs else h, g, da, db, algo=_algo_id(algo), continuation=cont, u_in=u0,
+                                 h_prev=h0 if cont else None, u_out=u, reverse=reverse)
+            assert all(bool((t[:, :, :2] == 7.0).all()) and bool((t[:, :, D + 2:] == 7.0).all()) for t in wide)
+            runs.append((h, da, db, last, u))
+        for k, name in enumerate("h da db last u".split()):
+            want, got = runs[0][k].float(), runs[1][k].float()
+            tol = 2.0 ** -7 if k < 3 else 2.0 ** -18       # |h| <~ 60 at these gates
+            assert bool(((want - got).abs() <= tol * (want.abs() + 4.0)).all()), (name, cont, reverse)
+            assert torch.equal(runs[1][k], runs[2][k]), name
+    import fast_sequential_scan_b200 as pkg
+    pkg.check_status()
+
+
 @pytest.mark.parametrize("reverse", [False, True])
 @pytest.mark.parametrize("shape", [(3, 1, 33), (2, 129, 100), (2, 300, 1001)])
 def test_any_layout_kernel_keeps_the_state_before_the_first_row_in_32_bits(shape, reverse):

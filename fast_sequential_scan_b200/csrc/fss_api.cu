@@ -157,9 +157,14 @@ static int chunked_backward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int6
 // ------------------------------------------------------------------ any-layout path
 // FSS_ALGO_AUTO takes it where TMA cannot address the tensors and 16-byte accesses do not fit either
 // (with them the chunked kernels move 8 or 4 elements per access; that is left for misaligned state
-// vectors); the callers that want block outputs get the chunked kernels, whose blocks they know.
-template <typename T> static bool ragged_ok(int64_t B, int64_t Tn, int64_t D, std::initializer_list<const fss_view *> views) {
-    return !chunked::vector_ok<T>(D, views) && ragged::fits(B, Tn, D);
+// vectors), and not for a few rows of many columns (ragged::rows_for_chunks); the callers that want block
+// outputs get the chunked kernels, whose blocks they know.
+template <typename T, bool kBackward>
+static bool ragged_ok(int64_t B, int64_t Tn, int64_t D, std::initializer_list<const fss_view *> views) {
+    if (chunked::vector_ok<T>(D, views) || !ragged::fits(B, Tn, D)) return false;
+    bool pairs = sizeof(T) == 2 && D % 2 == 0;
+    for (const fss_view *v : views) pairs &= ragged::pair_aligned(make_view<const bf16>(v));
+    return Tn > ragged::rows_for_chunks<T, kBackward>(B * ceil_div(D, pairs ? 64 : 32), pairs);
 }
 template <typename T>
 static int ragged_forward(const fss_scan_ctx *ctx, int64_t B, int64_t Tn, int64_t D, const fss_view *alpha, const fss_view *beta,
@@ -218,7 +223,7 @@ static int forward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t 
     if (algo == FSS_ALGO_LOOKBACK)
         return lookback::forward<T>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D, alpha, beta, h, st, &g_cuda_error);
     if (ctx->algo == FSS_ALGO_AUTO && !(st && (st->prod || st->block_prod || st->block_state)) &&
-        ragged_ok<T>(B, Tn, D, {alpha, beta, h}))
+        ragged_ok<T, false>(B, Tn, D, {alpha, beta, h}))
         return ragged_forward<T>(ctx, B, Tn, D, alpha, beta, h, st);
     constexpr int V = VecWidth<T>::value;
     if (chunked::vector_ok<T>(D, {alpha, beta, h}))
@@ -250,7 +255,7 @@ static int backward_typed(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t
         return lookback::backward<T>(ctx, plan_workspace(ctx->workspace, ctx->workspace_bytes), B, Tn, D, alpha, h, grad,
                                      dalpha, dbeta, st, &g_cuda_error);
     if (ctx->algo == FSS_ALGO_AUTO && !(st && (st->block_prod || st->block_state)) &&
-        ragged_ok<T>(B, Tn, D, {alpha, h, grad, dalpha, dbeta}))
+        ragged_ok<T, true>(B, Tn, D, {alpha, h, grad, dalpha, dbeta}))
         return ragged_backward<T>(ctx, B, Tn, D, alpha, h, grad, dalpha, dbeta, st);
     constexpr int V = VecWidth<T>::value;
     if (chunked::vector_ok<T>(D, {alpha, h, grad, dalpha, dbeta}))

@@ -349,6 +349,14 @@ scan_kernel(View<const T> alpha, View<const T> x, View<const T> h, View<T> out0,
 }
 
 // ------------------------------------------------------------------ host side
+// rows that 4-byte accesses can address
+inline bool pair_aligned(const View<const bf16> &v) { return !(reinterpret_cast<uintptr_t>(v.ptr) & 3u) && !(v.sb & 1) && !(v.st & 1); }
+inline bool pairs_ok(int64_t D, std::initializer_list<View<const bf16>> views) {
+    if (D % 2) return false;
+    for (const auto &v : views)
+        if (!pair_aligned(v)) return false;
+    return true;
+}
 inline int64_t tiles(int64_t B, int64_t T, int64_t D, int V) { return B * ceil_div(D, 32 * V) * ceil_div(T, kTileRows); }
 // tile numbers are 32-bit (checked without overflow)
 inline bool fits(int64_t B, int64_t T, int64_t D) {
@@ -357,6 +365,23 @@ inline bool fits(int64_t B, int64_t T, int64_t D) {
     return S <= lim / (B * ncg);
 }
 inline size_t workspace_bytes(int64_t B, int64_t T, int64_t D) { return (size_t)(tiles(B, T, D, 2) * 64 * kCellBytes); }
+
+// Up to how many rows the chunked kernels are faster.  A tile costs its CTA much the same whether its 128
+// rows are there or not, which nobody notices while the CTAs fit the GPU at once (some 300 of them); the
+// chunked kernels do little for few rows.  With more columns of tiles the line rises to the rows of a tile that
+// pay for its launch, look-back and stores.  Any-layout against chunked, B128 D1001 bf16 forward / backward (4,096
+// columns): 9 rows 33 / 57 us against 13 / 14, 32 rows 35 / 63 against 26 / 30, 64 rows 37 / 68 against 40 / 54, 100 rows 40 /
+// 78 against 68 / 101; fp32 32 rows 34 / 52 against 24 / 32, 64 rows 39 / 58 against 42 / 66; by pairs (B128 D5002) 32 rows
+// 134 / 176 against 116 / 144, 48 rows 137 / 183 against 196 / 231.  B16 D1001 (512 columns): backward 9 rows 9.6 against
+// 8.0, 24 rows 10.4 against 11.5.  Measured over 64 to 10,048 columns and 1 to 520 rows; near the line, and for bf16
+// backwards of 129 to 150 rows, the two lie within 7 % of each other.
+template <typename T, bool kBackward> inline int64_t rows_for_chunks(int64_t cols, bool pairs) {
+    const bool wide = sizeof(T) == 4;
+    const int64_t cap = kBackward ? (wide ? 54 : pairs ? 38 : 84) : (wide ? 50 : pairs ? 36 : 54);
+    const int64_t step = kBackward ? (wide ? 17 : 12) : (wide ? 25 : pairs ? 55 : 45);
+    const int64_t rows = (cols - 300) / step;
+    return rows < cap ? rows : cap;
+}
 
 template <typename T, bool kBackward, int V>
 inline int launch_lots(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D, const View<const T> &alpha,
@@ -382,13 +407,6 @@ inline int launch_lots(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { *err_text = std::string("any-layout launch: ") + cudaGetErrorString(e); return FSS_E_LAUNCH; }
     return FSS_OK;
-}
-// rows that 4-byte accesses can address
-inline bool pairs_ok(int64_t D, std::initializer_list<View<const bf16>> views) {
-    if (D % 2) return false;
-    for (const auto &v : views)
-        if ((reinterpret_cast<uintptr_t>(v.ptr) & 3u) || (v.sb & 1) || (v.st & 1)) return false;
-    return true;
 }
 template <typename T, bool kBackward>
 inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D, const View<const T> &alpha,

@@ -43,7 +43,8 @@ extern "C" {
 /* kernel families */
 #define FSS_ALGO_AUTO 0     /* forward of at most 8 rows: one thread per channel vector; else the
                                single-pass TMA kernel when the layout allows it, else a single-pass
-                               kernel for any layout, or the chunked ones (block outputs)        */
+                               kernel for any layout, or the chunked ones (block outputs, a few
+                               rows of many columns)                                            */
 #define FSS_ALGO_CHUNKED 1  /* three launches: chunk summaries, carry composition, chunk re-scan */
 #define FSS_ALGO_LOOKBACK 2 /* one persistent launch: TMA tiles + decoupled look-back of carries */
 

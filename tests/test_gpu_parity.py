@@ -582,6 +582,31 @@ def test_any_layout_kernel_matches_the_chunked_kernels(shape, dtype):
     pkg.check_status()
 
 
+@pytest.mark.parametrize("dtype, B, D, forward_rows, backward_rows", [
+    (torch.bfloat16, 128, 1001, 54, 84), (torch.bfloat16, 96, 1002, 22, 38), (torch.float32, 32, 1001, 28, 42), (torch.bfloat16, 16, 1001, 8, 17)])
+def test_few_rows_of_many_odd_columns_go_to_the_chunked_kernels(dtype, B, D, forward_rows, backward_rows):
+    """Where a tile of the any-layout kernel would be mostly past the end and the GPU is full of them: up to the line, auto
+    is the chunked kernels to the bit; one row further, the same up to association."""
+    _, native, _lib = _mods()
+    gen = torch.Generator(device="cuda").manual_seed(18)
+    for T in sorted({forward_rows, forward_rows + 1, backward_rows, backward_rows + 1}):
+        a = (0.5 + 0.499 * torch.rand(B, T, D, generator=gen, device="cuda")).to(dtype)
+        b, g = (torch.randn(B, T, D, generator=gen, device="cuda").to(dtype) for _ in range(2))
+        runs = []
+        for algo in (_lib.ALGO_CHUNKED, _lib.ALGO_AUTO):
+            h, da, db = (torch.full_like(a, 7.0) for _ in range(3))
+            native.forward_into(a, b, h, algo=algo)
+            native.backward_into(a, runs[0][0] if runs else h, g, da, db, algo=algo)
+            runs.append((h, da, db))
+        for x, y, name, line in zip(*runs, ("h", "da", "db"), (forward_rows, backward_rows, backward_rows)):
+            if T <= line:
+                assert torch.equal(x, y), (name, T)
+            tol = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -18       # |h| <~ 60 at these gates
+            assert bool(((x.float() - y.float()).abs() <= tol * (x.float().abs() + 4.0)).all()), (name, T)
+    import fast_sequential_scan_b200 as pkg
+    pkg.check_status()
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 2), (2, 15, 40), (1, 127, 66), (2, 129, 100), (3, 260, 130), (5, 400, 4098), (2, 300, 9478)])
 def test_any_layout_kernel_on_rows_that_4_byte_accesses_can_address(shape):
     """bf16 with an even width and even strides from bases that are 4- but not 16-byte aligned: two channels per lane, the

@@ -510,6 +510,15 @@ def test_gated_backward_in_one_kernel_matches_the_three_kernels(shape, dtype):
         assert err <= (2.0 ** -7 if dtype == "bf16" else 1e-5), (name, err)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("rows", [1, 2, 7, 8, 9, 23, 25, 40])
+@pytest.mark.parametrize("before", [0, 256])
+def test_gated_backward_visits_the_rows_that_exist(before, rows, dtype):
+    """Rows left out at the end of the sequence: within a batch of rows, whole groups of rows, whole warps; in wide tiles
+    (few rows) and in the last tile of narrow ones, whose warps hold several groups."""
+    test_gated_backward_in_one_kernel_matches_the_three_kernels((3 if before == 0 else 1, before + rows, 264), dtype)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(2, 1, 8), (2, 15, 136), (3, 64, 24), (1, 65, 2056), (2, 300, 136), (5, 1000, 264), (1, 4097, 64),
                                    (3, 77, 33), (2, 6200, 4104)])

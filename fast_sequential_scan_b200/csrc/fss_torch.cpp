@@ -12,8 +12,6 @@
 // any of which may block (memory to reclaim, a full launch queue).
 #include <torch/extension.h>
 
-#include <cstring>
-
 #include "../../include/fss_b200.h"
 
 namespace {
@@ -28,9 +26,9 @@ struct Library {
     decltype(&fss_scan_forward_gated) forward_gated;
     decltype(&fss_scan_backward_gated) backward_gated;
 } lib;
-// Python: acquire(device index, B, T, D, dtype id, gated backward) -> (context, algo, flags, release of
-// the device's lock, workspace or None); launched(workspace); check(code, where); the gated backward for
-// any layout.  Held for the process's life.
+// Python: acquire(device index, B, T, D, dtype id, gated backward) -> (context, its address, release of the
+// device's lock, workspace or None); launched(workspace); check(code, where); the gated backward for any
+// layout.  Held for the process's life.
 PyObject *py_acquire, *py_launched, *py_check, *py_gated_backward;
 
 struct Shape {
@@ -50,11 +48,10 @@ struct Launch {
                                                                                        (long long)s.T, (long long)s.D, s.dtype, (int)gated_backward));
         if (!got) throw py::error_already_set();
         const auto item = [&](int k) { return PyTuple_GET_ITEM(got.ptr(), k); };
-        std::memcpy(&ctx, PyBytes_AS_STRING(item(0)), sizeof ctx);
-        ctx.algo = (int32_t)PyLong_AsLong(item(1));
-        ctx.flags = (int32_t)PyLong_AsLong(item(2)) | flags;
-        release = Py_NewRef(item(3));
-        workspace = Py_NewRef(item(4));
+        ctx = *reinterpret_cast<const fss_scan_ctx *>(PyLong_AsUnsignedLongLong(item(1)));      // (item 0 keeps it alive)
+        ctx.flags |= flags;
+        release = Py_NewRef(item(2));
+        workspace = Py_NewRef(item(3));
     }
     Launch(const Launch &) = delete;
     ~Launch() {

@@ -178,7 +178,7 @@ def _ordinary_call(*tensors) -> bool:
 
 
 def _scan_any(plain_cls, dtype: torch.dtype, alpha, beta, backward_mode, h0, return_final_state, reverse):
-    if _resolve(backward_mode) == "saved" and (_ordinary_call(alpha, beta) if h0 is None else _ordinary_call(alpha, beta, h0)):
+    if (backward_mode or _default_mode) == "saved" and (_ordinary_call(alpha, beta) if h0 is None else _ordinary_call(alpha, beta, h0)):
         out = _fss_torch.scan(alpha, beta, h0, bool(return_final_state), bool(reverse), dtype is torch.bfloat16)
         if out is not None:
             return out

@@ -29,7 +29,10 @@ _DTYPES = {torch.bfloat16: _lib.DTYPE_BF16, torch.float32: _lib.DTYPE_F32}
 
 def default_algo() -> int:
     """Kernel family: ``FSS_B200_ALGO`` = auto | chunked | lookback (default auto)."""
-    name = os.environ.get("FSS_B200_ALGO", "auto").lower()
+    name = os.environ.get("FSS_B200_ALGO")
+    if name is None:
+        return _lib.ALGO_AUTO
+    name = name.lower()
     if name not in _lib.ALGO_BY_NAME:
         raise ValueError(f"FSS_B200_ALGO={name!r}: expected one of {sorted(_lib.ALGO_BY_NAME)}")
     return _lib.ALGO_BY_NAME[name]
@@ -98,28 +101,16 @@ def _workspace_bytes(shape, dtype_id: int, query: str = "fss_workspace_bytes") -
     return need
 
 
-def _launch(t: torch.Tensor, dtype_id: int, query: str = "fss_workspace_bytes") -> workspace.Launch:
-    """One launch on the calling stream of ``t``'s device, with a workspace for a scan of ``t``'s shape."""
-    return workspace.Launch(t.device, _workspace_bytes(t.shape, dtype_id, query))
-
-
-def _ctx_bytes(device: torch.device, ws: workspace.Workspace) -> bytes:
-    if ws.ctx is None:      # (the workspace forgets it when its buffer is replaced)
-        ws.ctx = bytes(_lib.ScanCtx(ctypes.sizeof(_lib.ScanCtx), device.index if device.index is not None else -1,
-                                    ws.stream_handle, ws.buf.data_ptr(), ws.buf.numel(), ws.status.data_ptr(), 0, 0))
-    return ws.ctx
-
-
-def _call_flags(flags: int = 0) -> int:
-    return flags | (_lib.FLAG_DETERMINISTIC if _deterministic else 0)
-
-
 def _ctx(device: torch.device, ws: workspace.Workspace, algo: Optional[int], flags: int = 0) -> _lib.ScanCtx:
-    """The context of one call: the workspace's part, copied, with this call's algo and flags.  ``device`` goes to
-    the library, which makes it current for the launch, so no torch device context is entered here."""
-    ctx = _lib.ScanCtx.from_buffer_copy(_ctx_bytes(device, ws))
-    ctx.algo = default_algo() if algo is None else algo
-    ctx.flags = _call_flags(flags)
+    """The context of a call.  One struct per algo and flags, shared by all calls that ask for the same and never
+    changed, so that no thread sees another's flags.  ``device`` goes to the library, which makes it current for the
+    launch, so no torch device context is entered here."""
+    key = (default_algo() if algo is None else algo, flags | _lib.FLAG_DETERMINISTIC if _deterministic else flags)
+    contexts = ws.contexts      # (a larger buffer comes with a new dict)
+    ctx = contexts.get(key)
+    if ctx is None:
+        ctx = contexts[key] = _lib.ScanCtx(ctypes.sizeof(_lib.ScanCtx), device.index if device.index is not None else -1,
+                                           ws.stream_handle, ws.buf.data_ptr(), ws.buf.numel(), ws.status.data_ptr(), *key)
     return ctx
 
 
@@ -128,9 +119,9 @@ _acquire_bytes: dict = {}      # workspace bytes per (B, T, D, dtype, gated back
 
 
 def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: int):
-    """What ``_fss_torch`` needs for one launch on the current stream: the context's bytes, algo and flags; the
-    release of the device's lock, which is held from here on and which the caller calls when it has launched; and, once
-    several streams are in play on the device, the workspace that :func:`workspace.launched` wants to hear of before."""
+    """What ``_fss_torch`` needs for one launch on the current stream: the context and its address, the release of the
+    device's lock, which is held from here on and which the caller calls when it has launched; and, once several streams
+    are in play on the device, the workspace that :func:`workspace.launched` wants to hear of before."""
     device = _torch_devices.get(index)
     if device is None:
         device = _torch_devices[index] = torch.device("cuda", index)
@@ -140,14 +131,14 @@ def _acquire(index: int, B: int, T: int, D: int, dtype_id: int, gated_backward: 
     if need is None:
         query = _lib.lib().fss_gated_backward_workspace_bytes if gated_backward else _lib.lib().fss_workspace_bytes
         need = _acquire_bytes[key] = query(B, T, D, dtype_id)
-    lock = (workspace._devices.get(index) or workspace._order(device)).lock
+    lock = workspace.lock(device)
     lock.acquire()
     try:
-        ws = workspace._get(device, need)
-        ctx, algo, order = ws.ctx or _ctx_bytes(device, ws), default_algo(), ws.order
+        ws = workspace.get_locked(device, need)
+        ctx, order = _ctx(device, ws, None), ws.order
         if not order.multi:      # (stays as it is while the lock is held)
             order.last, ws = ws, None
-        return ctx, algo, _lib.FLAG_DETERMINISTIC if _deterministic else 0, lock.release, ws
+        return ctx, ctypes.addressof(ctx), lock.release, ws
     except BaseException:
         lock.release()
         raise
@@ -173,10 +164,13 @@ def _launch_forward(a, b, h, dtype_id: int, algo, flags: int, state) -> None:
     """One checked call of ``fss_scan_forward_ex`` on tensors that were validated by the caller."""
     B, T, D = a.shape
     va, vb, vh = _view(a), _view(b), _view(h)
-    with _launch(a, dtype_id) as ws:
+    need = _workspace_bytes(a.shape, dtype_id)
+    with workspace.lock(a.device):
+        ws = workspace.get_locked(a.device, need)
         ctx = _ctx(a.device, ws, algo, flags)
         rc = _lib.lib().fss_scan_forward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(va), ctypes.byref(vb),
                                             ctypes.byref(vh), ctypes.byref(state) if state is not None else None)
+        workspace.launched(ws)
     if rc:
         _lib.check(rc, "fss_scan_forward_ex")
 
@@ -184,11 +178,14 @@ def _launch_forward(a, b, h, dtype_id: int, algo, flags: int, state) -> None:
 def _launch_backward(a, hh, g, grad_alpha, grad_beta, dtype_id: int, algo, flags: int, state) -> None:
     B, T, D = a.shape
     v0, v1, v2, v3, v4 = _view(a), _view(hh), _view(g), _view(grad_alpha), _view(grad_beta)
-    with _launch(a, dtype_id) as ws:
+    need = _workspace_bytes(a.shape, dtype_id)
+    with workspace.lock(a.device):
+        ws = workspace.get_locked(a.device, need)
         ctx = _ctx(a.device, ws, algo, flags)
         rc = _lib.lib().fss_scan_backward_ex(ctypes.byref(ctx), dtype_id, B, T, D, ctypes.byref(v0), ctypes.byref(v1),
                                              ctypes.byref(v2), ctypes.byref(v3), ctypes.byref(v4),
                                              ctypes.byref(state) if state is not None else None)
+        workspace.launched(ws)
     if rc:
         _lib.check(rc, "fss_scan_backward_ex")
 
@@ -255,11 +252,14 @@ def forward_gated_into(r, i, x, lam, h, *, continuation=False, h_in=None, h_last
     if h_in is not None or h_last is not None:
         state = _lib.ForwardState(_vec(h_in, B, D, "h_in"), _vec(h_last, B, D, "h_last"), None, None, None)
     views = [_view(t) for t in (rr, ii, xx, h)]
-    with _launch(r, _DTYPES[dtype]) as ws:
+    need = _workspace_bytes(r.shape, _DTYPES[dtype])
+    with workspace.lock(r.device):
+        ws = workspace.get_locked(r.device, need)
         ctx = _ctx(r.device, ws, None, _lib.FLAG_CONTINUATION if continuation else 0)
         rc = _lib.lib().fss_scan_forward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(views[0]),
                                                ctypes.byref(views[1]), ctypes.byref(views[2]), lam.data_ptr(),
                                                ctypes.byref(views[3]), ctypes.byref(state) if state is not None else None)
+        workspace.launched(ws)
     _lib.check(rc, "fss_scan_forward_gated")
 
 
@@ -335,11 +335,14 @@ def scan_backward_gated(r, i, x, lam, h, grad_out):
         dlam = torch.empty(D, dtype=torch.float32, device=r.device)
         tensors = [_rowwise(t) for t in (r, i, x, h, grad_out)] + [dr, di, dx]
         v = [_view(t) for t in tensors]
-        with _launch(r, _DTYPES[dtype], "fss_gated_backward_workspace_bytes") as ws:
+        need = _workspace_bytes(r.shape, _DTYPES[dtype], "fss_gated_backward_workspace_bytes")
+        with workspace.lock(r.device):
+            ws = workspace.get_locked(r.device, need)
             ctx = _ctx(r.device, ws, None)
             rc = _lib.lib().fss_scan_backward_gated(ctypes.byref(ctx), _DTYPES[dtype], B, T, D, ctypes.byref(v[0]),
                                                     ctypes.byref(v[1]), ctypes.byref(v[2]), lam.data_ptr(),
                                                     *[ctypes.byref(w) for w in v[3:]], dlam.data_ptr())
+            workspace.launched(ws)
         if rc == 0:
             return dr, di, dx, dlam
         if rc != _lib.E_LAYOUT:

@@ -22,9 +22,9 @@ another stream) only delay a launch; they cannot dead-lock it.
 Threads
 -------
 From the look-up of its workspace until its launch is recorded, a call holds the device's lock
-(:class:`Launch`; the C++ functions hold the same lock).  A launch of another thread therefore comes
-entirely before it or entirely after it: it sees the launch and can fence it, and a workspace is never
-replaced by a larger one between the look-up and the launch.
+(``with lock(device): ws = get(...); ...; launched(ws)``; the C++ functions hold the same lock).  A launch
+of another thread therefore comes entirely before it or entirely after it: it sees the launch and can fence
+it, and a workspace is never replaced by a larger one between the look-up and the launch.
 """
 from __future__ import annotations
 
@@ -57,7 +57,7 @@ class Workspace:
         self.device = device
         self.stream_handle = stream_handle
         self.buf = None
-        self.ctx = None          # ScanCtx of this buffer as bytes: every launch makes its own copy (built by the caller)
+        self.contexts = {}       # what the library is handed, per (algo, flags); never changed once made (by the caller)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._flag = self.status.numpy()      # same memory, read without going through torch
         self.order = _order(device)
@@ -72,7 +72,7 @@ class Workspace:
         # grow geometrically; a fresh buffer has to be zeroed before its first launch
         size = max(nbytes, 2 * (self.buf.numel() if self.buf is not None else 0), 1 << 16)
         self.buf = torch.empty(size, dtype=torch.uint8, device=self.device)
-        self.ctx = None
+        self.contexts = {}
         _lib.check(_lib.lib().fss_workspace_init(self.buf.data_ptr(), size, self.stream_handle),
                    "fss_workspace_init")
 
@@ -121,14 +121,20 @@ def _order(device: torch.device) -> _DeviceOrder:
     return order if order is not None else _devices.setdefault(index, _DeviceOrder())
 
 
+def lock(device: torch.device):
+    """The lock that orders the launches of all threads on ``device``; reentrant."""
+    return (_devices.get(device.index) or _order(device)).lock
+
+
 def get(device: torch.device, nbytes: int) -> Workspace:
-    """Workspace of the current stream of ``device``, at least ``nbytes`` large.  For a launch that uses its
-    memory or counts as a single-pass launch, take it through :class:`Launch`."""
-    with _order(device).lock:
-        return _get(device, nbytes)
+    """Workspace of the current stream of ``device``, at least ``nbytes`` large.  A launch that uses its memory or
+    counts as a single-pass launch holds the device's lock around this call too."""
+    with lock(device):
+        return get_locked(device, nbytes)
 
 
-def _get(device: torch.device, nbytes: int) -> Workspace:
+def get_locked(device: torch.device, nbytes: int) -> Workspace:
+    """:func:`get` for a caller that holds the device's lock."""
     stream = current_stream_handle(device)
     key = (device.index, stream)
     ws = _cache.get(key)
@@ -147,30 +153,6 @@ def _get(device: torch.device, nbytes: int) -> Workspace:
     if ws.order.last is not ws:
         ws.order_after_other_streams()
     return ws
-
-
-class Launch:
-    """``with Launch(device, nbytes) as ws``: one launch on the current stream, ordered against those of other
-    streams and threads; the body enqueues it."""
-    __slots__ = ("device", "nbytes", "lock", "ws")
-
-    def __init__(self, device: torch.device, nbytes: int):
-        self.device, self.nbytes, self.lock = device, nbytes, _order(device).lock
-
-    def __enter__(self) -> Workspace:
-        self.lock.acquire()
-        try:
-            self.ws = _get(self.device, self.nbytes)
-        except BaseException:
-            self.lock.release()
-            raise
-        return self.ws
-
-    def __exit__(self, *exc) -> None:
-        try:
-            launched(self.ws)
-        finally:
-            self.lock.release()
 
 
 def launched(ws: Workspace) -> None:

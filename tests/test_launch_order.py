@@ -34,7 +34,7 @@ def fake(monkeypatch):
 
     class Workspace(workspace.Workspace):
         def __init__(self, device, handle):
-            self.device, self.stream_handle, self.buf, self.ctx, self._event = device, handle, None, None, None
+            self.device, self.stream_handle, self.buf, self.contexts, self._event = device, handle, None, {}, None
             self.status, self._flag = torch.zeros(1, dtype=torch.int32), [0]
             self.order = workspace._devices.setdefault(device.index, workspace._DeviceOrder())
 
@@ -42,7 +42,7 @@ def fake(monkeypatch):
             return Stream(self.stream_handle)
 
         def ensure(self, nbytes):
-            self.buf, self.ctx = torch.zeros(nbytes, dtype=torch.uint8), None
+            self.buf, self.contexts = torch.zeros(nbytes, dtype=torch.uint8), {}
 
     def scan(ctx, *args):
         ctx = ctx._obj
@@ -105,10 +105,11 @@ def test_another_threads_stream_waits_for_the_launch_that_is_under_way(fake):
 
 def test_what_the_cpp_functions_hold_is_theirs_until_they_have_launched(fake):
     fake.thread.stream = 1
-    ctx, algo, flags, release, ws = native._acquire(0, 1, 4, 8, _lib.DTYPE_F32, 0)
+    ctx, address, release, ws = native._acquire(0, 1, 4, 8, _lib.DTYPE_F32, 0)
     other = _second_thread(lambda: _scan(fake, 2, _lib.FLAG_REVERSE))
     assert fake.log == []
-    assert _lib.ScanCtx.from_buffer_copy(ctx).stream == 1 and (algo, flags, ws) == (_lib.ALGO_AUTO, 0, None)
+    assert (ctx.stream, ctx.algo, ctx.flags, ws) == (1, _lib.ALGO_AUTO, 0, None)
+    assert bytes(_lib.ScanCtx.from_address(address)) == bytes(ctx)
     fake.log.append(("launch", 1, 0))
     release()
     other.join(LIMIT)

@@ -10,6 +10,8 @@
 namespace fss {
 namespace brief {
 
+// Rows that a thread holds in registers, two tensors at once.  Not a crossover: the first lengths past it still take the
+// look-back kernel mostly empty tiles (9 rows of B128 D2560 bf16 18 us, 8 rows 3.6).
 constexpr int kMaxRows = 8;
 constexpr int kThreads = 128;
 

@@ -207,8 +207,8 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
 
 // Workspace plan: [256-byte header | descriptor packets | float scratch].  The split depends only
 // on the workspace's total size, so for one allocation the packet area always sits at the same
-// place and only ever holds 16-byte packets whose fourth word is a tag: a stale float can never
-// pass for a tag of the current launch.
+// place and only ever holds 8-byte cells {value, tag}, whichever kernel wrote them: a stale float can
+// never pass for a tag of the current launch.
 constexpr size_t kWsHeaderBytes = 256;
 struct WsPlan {
     char *hdr, *packets, *floats;

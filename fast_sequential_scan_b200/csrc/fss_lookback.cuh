@@ -545,7 +545,10 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
     constexpr bool kGateBwd = kGate && kBackward;
     // Rows per register batch.  The narrow tiles' register swaps make long loop bodies, and in the long
     // ticketed backward the warps of a scheduler wait for instructions: 2 rows 411 us, 4 rows 418, 8 rows 428
-    // (B1 T65536 D4096 bf16; B4 T8192 D2048 108 with either).  Everywhere else 8 rows are as fast or up to 3 % faster.
+    // (B1 T65536 D4096 bf16; B4 T8192 D2048 108 with either; reversed 417 with 2, 442 with 8; B1 T262144 D1024 bf16 458 / 505,
+    // reversed 468 / 530).  fp32, half the channels a row, does not mind: 800 / 798, reversed 797 / 791 (B1 T65536 D4096), 203 /
+    // 202 (B2 T16384 D2048), 413 / 414, reversed 413 / 419 (B1 T262144 D512).  Everywhere else 8 rows are as fast or up to 3 %
+    // faster.
     constexpr int kRh = kTickets && kSp == 4 ? 2 : 8;
     using SM = Smem<K::kIn, kStages, kTileBytes>;
     constexpr int V = Cfg<T>::V;
@@ -1783,7 +1786,7 @@ inline int forward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, i
 // Backward of the gated scan in one pass over memory: reads r, grad, h, i, x and writes dr, di, dx (8
 // tensor passes; re-creating alpha, the plain reverse scan and the gates' chain rule as launches of
 // their own take 15) and adds the gradient of lambda per tile.  Measured at B16 T4096 D2560 bf16: the three
-// launches 1,204 us (153 + 268 + 783), this one 439 us = 6.1 TB/s; fp32 at B4 T2048 D2560 107 us = 6.3 TB/s.
+// launches 1,204 us (153 + 268 + 783), this one with its tables 442 us = 6.1 TB/s; fp32 at B4 T2048 D2560 118 us = 5.7 TB/s.
 template <typename T>
 inline int backward_gated(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t Tn, int64_t D, const fss_view *r,
                           const fss_view *i, const fss_view *x, const float *lambda, const fss_view *h, const fss_view *grad,

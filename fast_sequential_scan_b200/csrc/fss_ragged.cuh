@@ -14,8 +14,8 @@
 // (16 loads per tensor in flight per thread, two or three CTAs per SM).  Against the chunked kernels with
 // one element per access, which read every input twice and compose the chunks' states in one thread
 // per column (forward / backward): B4 T1000 D1001 bf16 46 / 50 -> 15 / 24 us, B8 T2048 D2049 bf16 276 / 320 ->
-// 87 / 161 us (2.3 / 2.1 TB/s), D2052 76 / 104 us, B1 T65536 D515 bf16 1687 / 1703 -> 112 / 195 us, B2 T8192 D2051 fp32
-// 439 / 517 -> 99 / 153 us (4.1 / 4.4 TB/s).
+// 87 / 161 us (2.3 / 2.1 TB/s), D2052 76 / 104 us, B1 T65536 D515 bf16 1687 / 1703 -> 113 / 196 us, B2 T8192 D2051 fp32
+// 439 / 517 -> 99 / 152 us (4.1 / 4.4 TB/s).  A few rows of many columns are the chunked kernels' (rows_for_chunks).
 #pragma once
 
 #include "fss_common.cuh"
@@ -85,13 +85,13 @@ __device__ __forceinline__ void store_cell(char *p, float x, uint32_t tag) {
 // All views are in scan order (row 0 is the first one the scan visits): the host flips those of a
 // scan that runs from the last row.  Forward: x = beta, out0 = h.  Backward: x = the gradient of h,
 // the row after the current one in scan order holds h_{t-1}; out0 = dalpha, out1 = dbeta.
-// CTAs per SM the registers are cut for.  A third one pays where it costs no spills: fp32 backward 153
+// CTAs per SM the registers are cut for.  A third one pays where it costs no spills: fp32 backward 152
 // us with three against 177 with two (B2 T8192 D2051), bf16 backward 207 against 171 (B8 T2048 D2049), pairs 118
 // against 104 (D2052).
 template <typename T, bool kBackward, int V> constexpr int kMinCtas = V == 2 || (kBackward && sizeof(T) == 2) ? 2 : 3;
 // kEarly: a first look at the tile before this one, ahead of the loads.  With more columns than a wave of
 // CTAs takes, that tile is long finished and its final state is here before this tile's rows are: B8 T2048
-// D2049 bf16 forward / backward 95 / 171 -> 87 / 160 us, B16 T512 D4093 91 / 166 -> 85 / 158.  With fewer columns it
+// D2049 bf16 forward / backward 95 / 171 -> 87 / 161 us, B16 T512 D4093 91 / 166 -> 86 / 157.  With fewer columns it
 // finds nothing and costs 1-2 % (B4 T1000 D1001), and the fp32 kernels have no registers left for it.
 template <typename T, bool kBackward, int V, bool kEarly>
 __global__ void __launch_bounds__(kThreads, kMinCtas<T, kBackward, V>)
@@ -400,7 +400,7 @@ inline int launch_lots(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int
     p.mute_first_block = (ctx->flags & FSS_FLAG_TEST_MUTE_FIRST_BLOCK) ? 1 : 0;
     const unsigned grid = (unsigned)tiles(B, Tn, D, V);
     const cudaStream_t stream = (cudaStream_t)ctx->stream;
-    if (sizeof(T) == 2 && p.ncols >= 2 * 148)      // (a wave: two CTAs per SM)
+    if (sizeof(T) == 2 && p.ncols >= 2 * 148)      // (a wave: two CTAs on each of the 148 SMs)
         scan_kernel<T, kBackward, V, sizeof(T) == 2><<<grid, kThreads, 0, stream>>>(alpha, x, h, out0, out1, p);
     else
         scan_kernel<T, kBackward, V, false><<<grid, kThreads, 0, stream>>>(alpha, x, h, out0, out1, p);

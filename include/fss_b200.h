@@ -205,8 +205,9 @@ int fss_scan_backward_ex(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t 
  * with the usual first-row rule (h_0 = beta_0 unless FSS_FLAG_CONTINUATION).  Reads r, i, x and
  * writes h: 4 tensor passes instead of the 8 of a gate kernel followed by the scan.
  * bf16 evaluates the gates with the hardware approximations (a and b are rounded to 8 bits
- * anyway), fp32 with the accurate functions.  Single-pass kernel only: layouts it cannot take,
- * and FSS_ALGO_CHUNKED, return FSS_E_LAYOUT; the caller then computes alpha and beta itself.
+ * anyway), fp32 with its exponential, reciprocal and square-root instructions (about 2^-22 each)
+ * instead of tanh.  Single-pass kernel only: layouts it cannot take, and FSS_ALGO_CHUNKED, return
+ * FSS_E_LAYOUT; the caller then computes alpha and beta itself.
  * state may carry h_in / h_last; prod, block_prod and block_state must be NULL (FSS_E_ARGS). */
 int fss_scan_forward_gated(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t T, int64_t D,
                            const fss_view *r, const fss_view *i, const fss_view *x,

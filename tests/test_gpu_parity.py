@@ -487,7 +487,7 @@ def test_gated_scans_enqueued_back_to_back_read_their_own_tables(shape, dtype):
 @pytest.mark.parametrize("shape", [(2, 1, 8), (1, 31, 136), (3, 33, 24), (2, 260, 136), (1, 1025, 264), (5, 97, 1000), (2, 6200, 4104)])
 def test_gated_backward_in_one_kernel_matches_the_three_kernels(shape, dtype):
     """The fused backward at the edges of its tiles (one row; one less and more than a tile; each tile shape; the last
-    shape by tickets) on views of wider tensors, against alpha, reverse scan and chain rule as kernels of their own.
+    shape: many tiles per CTA, in the fixed order that all gated scans keep) on views of wider tensors, against alpha, reverse scan and chain rule as kernels of their own.
     Bounds: the three kernels round alpha's and beta's gradients and the results to 8 bits, the fused one the results
     only: three roundings of at most 2^-9 apart, 2^-7 in the 2-norm with room for the reverse scan's own roundings;
     fp32 differs by a few ulp, amplified by at most 1/(1 - alpha) ~ 100 and by the sum over rows in lambda's gradient."""

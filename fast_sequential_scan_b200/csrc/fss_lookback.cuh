@@ -81,7 +81,7 @@ static_assert(kTc == Kind<true, false>::kTc, "both directions of a scan share th
 constexpr uint32_t kMaxSpins = 1u << 21;      // per wait; ~a second before giving up
 
 constexpr uint32_t kStateAggregate = 1, kStateInclusive = 2;
-constexpr int kWindow = 2;                    // predecessors inspected per look-back round trip
+constexpr int kWindow = 2;                    // predecessors inspected per look-back round trip, at least
 
 template <typename T> struct Cfg {
     static constexpr int V = kLaneBytes / (int)sizeof(T);   // channels per lane
@@ -117,7 +117,7 @@ struct Params {
     int32_t tile_rows;       // rows per tile: 64 * split
     uint32_t max_spins;      // iterations a wait may take before it gives up
     int mute_first_block;    // test hook: row block 0 publishes no descriptors (its successors' waits run out)
-    int deterministic;       // a tile only ever starts from its predecessor's inclusive state
+    int deterministic;       // a tile only ever starts from an inclusive state, carried forward tile by tile
     int hold_dependents;     // no early release of the next launch on the stream
     int64_t grid;            // CTAs of the launch
     // fixed tile order (CTA x takes tiles x, x+G, ...): ntiles = units_q * grid + units_r, so CTA x
@@ -813,7 +813,13 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         // kLookbackWarps warps share the work units round-robin, so several carry resolutions
         // (each a few L2 round trips) are in flight per CTA.
         constexpr int NI = V;                          // floats of an inclusive descriptor
-        constexpr int kWin = kWindow;
+        // Predecessors a lane reads per round trip.  In narrow tiles the lane groups, which hold the same channels, look at
+        // different ones: four in one trip at kSp = 4.  With every group at the same two the chain of carries was the
+        // bound of problems with few columns: forward / backward B1 T65536 bf16 D128 29.0 / 30.0 -> 23.7 / 25.2 us, D512 57.0 /
+        // 67.4 -> 47.1 / 64.7, D1024 89.3 / 121.9 -> 78.7 / 120.5, D4096 262 / 415 -> 247 / 414; B2 T1024 D768 7.9 / 9.8 -> 7.6 /
+        // 9.5.  More per trip costs the passes more issue slots than it saves: with eight B8 T2048 D1024
+        // forward 21.6 -> 23.0, B1 T65536 D4096 274 / 476.
+        constexpr int kLooks = kWindow > kSp ? kWindow / kSp : 1;
         using AggPk = PacketGroup<2 * V, LPG>;         // (P, C) of the tile scanned from zero
         using IncPk = PacketGroup<NI, LPG>;                 // state after the tile (and product up to it)
         constexpr int kTilePackets = (AggPk::kPackets + IncPk::kPackets) * LPG;
@@ -825,7 +831,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         auto inc_packets = [&](int64_t k) { return p.packets + k * kTilePackets + AggPk::kPackets * LPG + cl; };
 
         // The predecessor's inclusive descriptor is fetched one of this warp's units ahead of its use
-        // (as soon as the producer has described that unit) and, if it was not there yet, once more
+        // (as soon as the producer has described that unit) and, if it was not there yet, again from
         // when the unit starts.
         typename IncPk::Raw pre;
         bool have_pre = false;
@@ -866,12 +872,14 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 }
             }
             if (!ctl.wait(bar_sum(g), (uint32_t)((i / kGens) & 1), FSS_STATUS_LOOKBACK_TIMEOUT)) break;
-            if (s > 0 && !hit) {       // one more look now that the summary is in
+            // One more look now that the summary is in.  With as many columns as kSp = 1 stands for the answer is there by
+            // now more often than not (B16 T4096 D2560 bf16 forward 173 us, 178 without); a window at once saves the others
+            // a round trip.
+            if (kSp == 1 && s > 0 && !hit) {
                 typename IncPk::Raw again;
                 IncPk::load_raw(inc_packets(k - p.ncols), again);
                 hit = __all_sync(0xffffffffu, IncPk::decode(again, cur, tag_inc));
             }
-
             // the tile's summary, folded by the summary warp
             float Pt[V], Ct[V];
             {
@@ -893,56 +901,82 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
 #pragma unroll
                 for (int v = 0; v < V; ++v) cin[v] = cur[v];
             } else {
-                float Pa[V], Ca[V];          // map of the tiles between the predecessor at q and this one
+                float Pa[V], Ca[V];          // map of the tiles between the nearest one not folded yet and this one
 #pragma unroll
                 for (int v = 0; v < V; ++v) { Pa[v] = 1.0f; Ca[v] = 0.0f; }
-                int64_t q = k - p.ncols;
+                int32_t at = s - 1;          // row block of that tile
                 uint32_t spins = 0;
-                bool found = false;
-                while (!found) {
-                    // read up to kWin predecessors in one round trip
-                    float inc[kWin][NI], ag[kWin][2 * V];
-                    bool inc_ok[kWin], ag_ok[kWin];
+                for (;;) {
+                    // one round trip: lane group q reads the descriptors of row blocks at - q, at - q - kSp, ...
+                    float inc[kLooks][NI], ag[kLooks][2 * V];
+                    uint32_t inc_in[kLooks], ag_in[kLooks];
 #pragma unroll
-                    for (int j = 0; j < kWin; ++j) {
-                        const int64_t qj = q - j * p.ncols;
-                        inc_ok[j] = false; ag_ok[j] = false;
-                        if (qj >= 0) {
-                            inc_ok[j] = IncPk::load(inc_packets(qj), inc[j], tag_inc);
-                            ag_ok[j] = AggPk::load(agg_packets(qj), ag[j], tag_agg);
+                    for (int j = 0; j < kLooks; ++j) {
+                        const int32_t back = at - (j * kSp + q);
+                        bool inc_ok = false, ag_ok = false;
+                        if (back >= 0) {
+                            const int64_t kb = k - (int64_t)(s - back) * p.ncols;
+                            inc_ok = IncPk::load(inc_packets(kb), inc[j], tag_inc);
+                            ag_ok = AggPk::load(agg_packets(kb), ag[j], tag_agg);
                         }
+                        inc_in[j] = __ballot_sync(0xffffffffu, inc_ok);
+                        ag_in[j] = __ballot_sync(0xffffffffu, ag_ok);
                     }
-                    int adv = 0;          // predecessors folded in this round
-                    bool stop = false;
+                    // the nearest inclusive state with every aggregate before it in reach, or the state before block 0
+                    int from = -1, adv = 0;             // (everything here is warp-uniform)
+                    bool more = true;
 #pragma unroll
-                    for (int j = 0; j < kWin; ++j) {
-                        const int64_t qj = q - j * p.ncols;     // warp-uniform
-                        if (found || stop) {
-                            // nothing more to do in this round
-                        } else if (qj < 0) {
-                            stop = true;
-                        } else if (__all_sync(0xffffffffu, inc_ok[j])) {
+                    for (int w = 0; w < kLooks * kSp; ++w) {
+                        constexpr uint32_t kGroup = LPG == 32 ? 0xffffffffu : (1u << (LPG % 32)) - 1u;
+                        const bool inc_ok = ((inc_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
+                        const bool ag_ok = ((ag_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
+                        if (more && inc_ok) from = w;
+                        else if (more && ag_ok) adv = w + 1;
+                        if (more && !inc_ok && ag_ok && at == w) from = w + 1;
+                        more = more && !inc_ok && ag_ok && at != w;
+                    }
+                    auto of = [&](const float &x, int w) {       // what the lane group of window position w has
+                        return kSp > 1 ? __shfl_sync(0xffffffffu, x, (w % kSp) * LPG + cl) : x;
+                    };
+                    if (from >= 0) {
+                        // Carried forward tile by tile, which is how those tiles do it themselves: the bits do not
+                        // depend on which of them had got how far.
+                        float state[V];
 #pragma unroll
-                            for (int v = 0; v < V; ++v) cin[v] = fmaf(Pa[v], inc[j][v], Ca[v]);
-                            found = true;
-                        } else if (!p.deterministic && __all_sync(0xffffffffu, ag_ok[j])) {
+                        for (int v = 0; v < V; ++v) state[v] = from > at ? state0(v) : 0.0f;
+                        if (from <= at) {
+#pragma unroll
+                            for (int j = 0; j < kLooks; ++j) {
+                                if (from / kSp == j) {
+#pragma unroll
+                                    for (int v = 0; v < V; ++v) state[v] = of(inc[j][v], from);
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int w = kLooks * kSp - 1; w >= 0; --w) {
+                            if (w < from) {
+#pragma unroll
+                                for (int v = 0; v < V; ++v)
+                                    state[v] = fmaf(of(ag[w / kSp][v], w), state[v], of(ag[w / kSp][V + v], w));
+                            }
+                        }
+#pragma unroll
+                        for (int v = 0; v < V; ++v) cin[v] = at == s - 1 ? state[v] : fmaf(Pa[v], state[v], Ca[v]);
+                        break;
+                    }
+                    if (p.deterministic) adv = 0;       // summaries are not folded ahead of the state they carry
+#pragma unroll
+                    for (int w = 0; w < kLooks * kSp; ++w) {
+                        if (w < adv) {
 #pragma unroll
                             for (int v = 0; v < V; ++v) {
-                                Ca[v] = fmaf(Pa[v], ag[j][V + v], Ca[v]);
-                                Pa[v] *= ag[j][v];
+                                Ca[v] = fmaf(Pa[v], of(ag[w / kSp][V + v], w), Ca[v]);
+                                Pa[v] *= of(ag[w / kSp][v], w);
                             }
-                            adv = j + 1;
-                            if (qj - p.ncols < 0) {      // folded everything down to row block 0
-#pragma unroll
-                                for (int v = 0; v < V; ++v) cin[v] = fmaf(Pa[v], state0(v), Ca[v]);
-                                found = true;
-                            }
-                        } else {
-                            stop = true;                 // not published yet: poll again from here
                         }
                     }
-                    if (found) break;
-                    q -= (int64_t)adv * p.ncols;
+                    at -= adv;
                     if (adv == 0) {
                         ++spins;
                         if ((spins & 15u) == 0u && __any_sync(0xffffffffu, ctl.aborted())) { ok = false; break; }

@@ -43,8 +43,8 @@ _deterministic = os.environ.get("FSS_B200_DETERMINISTIC", "0") not in ("", "0")
 
 def set_deterministic(on: bool) -> bool:
     """Ask the single-pass kernels for run-to-run identical results (``FSS_FLAG_DETERMINISTIC``: every
-    tile waits for its predecessor's final state instead of taking whichever summary is published
-    first).  Slower on long sequences.  Returns the previous setting; the environment variable
+    tile waits for a near predecessor's final state instead of folding summaries that are published
+    earlier).  Slower on long sequences.  Returns the previous setting; the environment variable
     ``FSS_B200_DETERMINISTIC=1`` sets the initial one."""
     global _deterministic
     previous, _deterministic = _deterministic, bool(on)

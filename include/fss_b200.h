@@ -94,11 +94,12 @@ typedef struct fss_scan_ctx {
  * h_0 = a_0*h_in + b_0; the returned product includes a_0) instead of the h_0 = b_0 rule.      */
 #define FSS_FLAG_CONTINUATION 1
 /* Run-to-run identical results from the single-pass kernels.  By default a tile takes the state
- * that enters it from whichever is published first, its predecessor's final state or a fold of the
- * summaries of several predecessors; the two associate the same sum differently, so the last bits
- * of the fp32 state (rarely one ulp of a bf16 result) depend on timing.  With this flag a tile
- * always waits for its predecessor's final state: one fixed association, bit-identical results in
- * every run, at the price of a serial hand-over per row block (noticeable on long sequences).
+ * that enters it from whichever is published first: a near predecessor's final state, carried forward
+ * through the summaries of the tiles between, or a fold of the summaries of several predecessors; the
+ * two associate the same sum differently, so the last bits of the fp32 state (rarely one ulp of a bf16
+ * result) depend on timing.  With this flag a tile always waits for a final state it can carry
+ * forward: one fixed association, bit-identical results in every run, at the price of a slower
+ * hand-over from row block to row block (noticeable on long sequences).
  * The chunked kernels are always deterministic.  The reference's kernels are, too: one thread walks
  * a channel group from the first row to the last (csrc/include/sequential_scan_kernel_bf16.cuh:121-151). */
 #define FSS_FLAG_DETERMINISTIC 2

@@ -1417,3 +1417,28 @@ def test_config5_full_length_on_one_gpu():
                                               sub(g).float().cpu().numpy())
     assert_parity(sub(db), torch.from_numpy(db_ref), BF16_TOL, "dbeta")
     assert_parity(sub(da), torch.from_numpy(da_ref), BF16_TOL, "dalpha")
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(1, 250, 128), (1, 500, 128), (3, 511, 264), (1, 512, 136), (1, 5000, 128), (2, 20003, 72)])
+def test_carries_through_many_row_blocks_of_few_columns(shape, dtype, deterministic):
+    """Look-back windows of every tile shape (64 rows up to T = 255, 128 up to 511, then 256), whose lane groups read
+    different predecessors: fewer row blocks than a window, partial windows and long chains."""
+    pkg, _, _ = _mods()
+    dt = torch.float32 if dtype == "f32" else torch.bfloat16
+    gen = torch.Generator().manual_seed(shape[1])
+    a = (0.9 + 0.099 * torch.rand(shape, generator=gen)).to(dt).cuda()       # a state is felt hundreds of rows later
+    b, g = (torch.randn(shape, generator=gen).to(dt).cuda() for _ in range(2))
+    previous = pkg.set_deterministic(deterministic)
+    try:
+        h, da, db = run_native(a, b, g, "lookback")
+    finally:
+        pkg.set_deterministic(previous)
+    tol = F32_TOL if dtype == "f32" else BF16_TOL
+    assert_parity(h, oracle.reference_values(a, b, None)[0], tol, "h")
+    da_ref, db_ref = oracle.scan_backward_f32(a.float().cpu().numpy(), h.float().cpu().numpy(), g.float().cpu().numpy())
+    assert_parity(db, torch.from_numpy(db_ref), tol, "dbeta")
+    # dalpha_t = dh_t * h_{t-1}: what dh may be off by, tol + tol * |dh|, is multiplied with h
+    scale = 1.0 + torch.cat([torch.zeros_like(h[:, :1]), h[:, :-1]], 1).float().abs().cpu()
+    assert_parity(da.float().cpu() / scale, torch.from_numpy(da_ref) / scale, tol, "dalpha")

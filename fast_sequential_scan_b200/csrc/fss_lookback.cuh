@@ -1456,6 +1456,21 @@ inline int choose_tail(int dtype, bool backward, int64_t B, int64_t T, int64_t D
     const int64_t bytes = B * T * D * (dtype == FSS_DTYPE_BF16 ? 2 : 4);
     return bytes >= ((int64_t)96 << 20) ? kAllTickets : 0;
 }
+// Tile shape of a plain scan whose row blocks no caller asks for.  From 384 of the narrowest columns on (a wave of CTAs takes
+// 148) a row block's columns span several waves, nothing holds the CTAs together any more, and in the fixed order the
+// ones that the memory system serves slowly finish late (the CTAs of B4 T4096 D2048 fp32 ended between 59 and 72 us).  Large
+// tensors make that dearer than the second halving of the columns is worth: 128 rows x 128 bytes against 256 x 64,
+// forward: 64 MiB a tensor 37.1 -> 35.8 us (B4 T2048 D2048 fp32) and 39.4 -> 37.8 (B16 T2048 D1024 bf16), 128 MiB 76.8 -> 67.4 and
+// 81.6 -> 70.2 (twice the rows), 176 MiB 105 -> 90 (B3 T6000 D2560 fp32), 256 MiB 195 -> 138 (B32 T8192 D512
+// bf16).  Below 64 MiB or 384 columns it is the other way round: 31 MiB 20.3 / 20.2, B16 T512 D1024 bf16 13.1 / 13.8, 320
+// columns 79.4 / 81.0 (B2 T8192 D2560 fp32).  The backward gains 2 to 3 % in the fixed order (61.1 -> 59.8) and loses as much with
+// tickets, which balance the CTAs themselves (105 / 107).
+inline int choose_split_freely(int dtype, int64_t B, int64_t T, int64_t D, bool tickets) {
+    const int s = choose_split(dtype, B, T, D);
+    const int64_t esize = dtype == FSS_DTYPE_BF16 ? 2 : 4;
+    const bool wide = s == 4 && !tickets && B * T * D * esize >= ((int64_t)64 << 20) && B * ceil_div(D * esize, kRowBytes / 4) >= 384;
+    return wide ? 2 : s;
+}
 inline int64_t block_rows(int dtype, int64_t B, int64_t T, int64_t D) { return (int64_t)kTc * choose_split(dtype, B, T, D); }
 
 template <typename T> inline int64_t channel_groups(int64_t D) { return ceil_div(D, Cfg<T>::Dc); }
@@ -1698,7 +1713,8 @@ inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t 
 #define FSS_LAUNCH_SPLIT(SP)                                                                                                    \
     return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
                     : launch_split<T, kBackward, SP, false, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, 0, err_text)
-    switch (choose_split(dtype, B, Tn, D, Kind<kBackward, kGate>::kTc)) {
+    const bool blocks = p.block_prod || p.block_state;      // (whose rows block_rows() has told the caller)
+    switch (kGate || blocks ? choose_split(dtype, B, Tn, D, Kind<kBackward, kGate>::kTc) : choose_split_freely(dtype, B, Tn, D, tail > 0)) {
     case 4: FSS_LAUNCH_SPLIT(4);
     case 2: FSS_LAUNCH_SPLIT(2);
     default: FSS_LAUNCH_SPLIT(1);

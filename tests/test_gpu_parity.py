@@ -1442,3 +1442,27 @@ def test_carries_through_many_row_blocks_of_few_columns(shape, dtype, determinis
     # dalpha_t = dh_t * h_{t-1}: what dh may be off by, tol + tol * |dh|, is multiplied with h
     scale = 1.0 + torch.cat([torch.zeros_like(h[:, :1]), h[:, :-1]], 1).float().abs().cpu()
     assert_parity(da.float().cpu() / scale, torch.from_numpy(da_ref) / scale, tol, "dalpha")
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("dtype, B, T, D", [("f32", 3, 2731, 2048), ("bf16", 12, 2731, 1024), ("f32", 3, 2729, 2048), ("f32", 2, 3200, 2624)])
+def test_large_scans_of_many_narrow_columns(dtype, B, T, D, reverse):
+    """Both sides of the line (64 MiB a tensor, 384 columns of 64 bytes) from which tiles are 128 rows x 128 bytes."""
+    _, native, _lib = _mods()
+    dt = torch.float32 if dtype == "f32" else torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    a = torch.rand((B, T, D), generator=gen, device="cuda").mul_(0.5).add_(0.45).to(dt)
+    b, g = (torch.randn((B, T, D), generator=gen, device="cuda").to(dt) for _ in range(2))
+    h, da, db = (torch.empty_like(a) for _ in range(3))
+    native.forward_into(a, b, h, algo=_lib.ALGO_LOOKBACK, reverse=reverse)
+    native.backward_into(a, h, g, da, db, algo=_lib.ALGO_LOOKBACK, reverse=reverse)
+    pick = torch.cat([torch.arange(0, 24), torch.arange(D - 24, D)]).cuda()
+    turn = (lambda t: t.flip(1)) if reverse else (lambda t: t)
+    sa, sb, sg, sh, sda, sdb = (turn(t[:, :, pick]).contiguous() for t in (a, b, g, h, da, db))
+    tol = F32_TOL if dtype == "f32" else BF16_TOL
+    assert_parity(sh, oracle.reference_values(sa, sb, None)[0], tol, "h")
+    da_ref, db_ref = oracle.scan_backward_f32(sa.float().cpu().numpy(), sh.float().cpu().numpy(), sg.float().cpu().numpy())
+    assert_parity(sdb, torch.from_numpy(db_ref), tol, "dbeta")
+    # (what dh may be off by is multiplied with h)
+    scale = 1.0 + torch.cat([torch.zeros_like(sh[:, :1]), sh[:, :-1]], 1).float().abs().cpu()
+    assert_parity(sda.float().cpu() / scale, torch.from_numpy(da_ref) / scale, tol, "dalpha")

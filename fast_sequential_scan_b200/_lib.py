@@ -84,6 +84,7 @@ SIGNATURES = {
                                         c_void_p] + [_P(View)] * 5 + [c_void_p]),
     "fss_gated_backward_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "fss_block_rows": (c_int64, [c_int, c_int64, c_int64, c_int64, c_int]),
+    "fss_tile_rows": (c_int64, [c_int, c_int, c_int64, c_int64, c_int64, c_int]),
     "fss_seqpar_compose": (c_int, [_P(ScanCtx), c_int, c_int, c_int, c_int64, c_void_p, c_void_p]),
     "fss_seqpar_push": (c_int, [_P(ScanCtx), c_int, c_int, c_int, c_int64, c_void_p, c_void_p, _P(c_void_p), _P(c_void_p),
                                 c_uint32]),

@@ -322,6 +322,11 @@ FSS_API int64_t fss_block_rows(int dtype, int64_t B, int64_t T, int64_t D, int a
     return lookback::block_rows(dtype, B, T, D);
 }
 
+FSS_API int64_t fss_tile_rows(int dtype, int backward, int64_t B, int64_t T, int64_t D, int flags) {
+    if (B <= 0 || T <= 0 || D <= 0) return 1;
+    return lookback::tile_rows(dtype, backward != 0, (flags & FSS_FLAG_REVERSE) != 0, B, T, D);
+}
+
 FSS_API int fss_scan_forward_ex(const fss_scan_ctx *ctx, int dtype, int64_t B, int64_t T, int64_t D,
                                 const fss_view *alpha, const fss_view *beta, const fss_view *h,
                                 const fss_forward_state *state) {

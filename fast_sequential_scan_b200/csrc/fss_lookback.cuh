@@ -1428,9 +1428,13 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
 // Tile shape for a problem: split s gives tiles of 64*s rows x 256/s bytes.  Narrow, tall tiles
 // multiply the number of columns; with fewer columns than about two per SM several row blocks of
 // one column are in flight at once and the carry chain between them limits the speed.
-inline int choose_split(int dtype, int64_t B, int64_t T, int64_t D, int tile_rows = kTc) {
+// FSS_B200_SPLIT=1 / 2 / 4 forces s for every launch.
+inline int forced_split() {      // 0: not forced
     static const int env = [] { const char *e = getenv("FSS_B200_SPLIT"); return e ? atoi(e) : 0; }();
-    if (env == 1 || env == 2 || env == 4) return env;
+    return env == 1 || env == 2 || env == 4 ? env : 0;
+}
+inline int choose_split(int dtype, int64_t B, int64_t T, int64_t D, int tile_rows = kTc) {
+    if (forced_split()) return forced_split();
     const int64_t row_bytes = D * (dtype == FSS_DTYPE_BF16 ? 2 : 4);
     const int64_t cols = B * ceil_div(row_bytes, kRowBytes);
     int s = 1;
@@ -1456,6 +1460,12 @@ inline int choose_tail(int dtype, bool backward, int64_t B, int64_t T, int64_t D
     const int64_t bytes = B * T * D * (dtype == FSS_DTYPE_BF16 ? 2 : 4);
     return bytes >= ((int64_t)96 << 20) ? kAllTickets : 0;
 }
+// Units of a CTA's share that the launch hands out by ticket.  Gated scans and reversed forward scans never take tickets
+// (the gated backward, too, is faster in the fixed order: 439 us against 475 at B16 T4096 D2560 bf16).
+constexpr bool never_tickets(bool backward, bool gated, bool reverse) { return gated || (reverse && !backward); }
+inline int launch_tail(int dtype, bool backward, bool gated, bool reverse, int64_t B, int64_t T, int64_t D) {
+    return never_tickets(backward, gated, reverse) ? 0 : choose_tail(dtype, backward, B, T, D);
+}
 // Tile shape of a plain scan whose row blocks no caller asks for.  From 384 of the narrowest columns on (a wave of CTAs takes
 // 148) a row block's columns span several waves, nothing holds the CTAs together any more, and in the fixed order the
 // ones that the memory system serves slowly finish late (the CTAs of B4 T4096 D2048 fp32 ended between 59 and 72 us).  Large
@@ -1468,8 +1478,12 @@ inline int choose_tail(int dtype, bool backward, int64_t B, int64_t T, int64_t D
 inline int choose_split_freely(int dtype, int64_t B, int64_t T, int64_t D, bool tickets) {
     const int s = choose_split(dtype, B, T, D);
     const int64_t esize = dtype == FSS_DTYPE_BF16 ? 2 : 4;
-    const bool wide = s == 4 && !tickets && B * T * D * esize >= ((int64_t)64 << 20) && B * ceil_div(D * esize, kRowBytes / 4) >= 384;
+    const bool wide = s == 4 && !forced_split() && !tickets && B * T * D * esize >= ((int64_t)64 << 20) && B * ceil_div(D * esize, kRowBytes / 4) >= 384;
     return wide ? 2 : s;
+}
+// rows per tile of a plain scan that leaves no block outputs
+inline int64_t tile_rows(int dtype, bool backward, bool reverse, int64_t B, int64_t T, int64_t D) {
+    return (int64_t)kTc * choose_split_freely(dtype, B, T, D, launch_tail(dtype, backward, false, reverse, B, T, D) > 0);
 }
 inline int64_t block_rows(int dtype, int64_t B, int64_t T, int64_t D) { return (int64_t)kTc * choose_split(dtype, B, T, D); }
 
@@ -1707,9 +1721,8 @@ inline int launch(const fss_scan_ctx *ctx, const WsPlan &ws, int64_t B, int64_t 
                   std::initializer_list<const fss_view *> in, std::initializer_list<const fss_view *> out, Params p,
                   std::string *err_text) {
     const int dtype = sizeof(T) == 2 ? FSS_DTYPE_BF16 : FSS_DTYPE_F32;
-    // (the gated backward, too, is faster in the fixed order: 439 us against 475 at B16 T4096 D2560 bf16)
-    constexpr bool kNeverTickets = kGate || (kReverse && !kBackward);
-    const int tail = kNeverTickets ? 0 : choose_tail(dtype, kBackward, B, Tn, D);
+    constexpr bool kNeverTickets = never_tickets(kBackward, kGate, kReverse);
+    const int tail = launch_tail(dtype, kBackward, kGate, kReverse, B, Tn, D);
 #define FSS_LAUNCH_SPLIT(SP)                                                                                                    \
     return tail > 0 ? launch_split<T, kBackward, SP, !kNeverTickets, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, tail, err_text)      \
                     : launch_split<T, kBackward, SP, false, kGate, kReverse>(ctx, ws, B, Tn, D, in, out, p, 0, err_text)

@@ -243,6 +243,11 @@ int fss_scan_backward_gated(const fss_scan_ctx *ctx, int dtype, int64_t B, int64
                             const fss_view *grad_i, const fss_view *grad_x, float *grad_lambda);
 size_t fss_gated_backward_workspace_bytes(int64_t B, int64_t T, int64_t D, int dtype);
 
+/* Rows per tile of the single-pass kernels (64, 128 or 256) for an ungated scan of this problem without block outputs:
+ * the tile shape that its launch takes.  backward: 0 / 1; flags: FSS_FLAG_REVERSE counts.  The environment variable
+ * FSS_B200_SPLIT = 1 / 2 / 4 (read once) forces 64 / 128 / 256. */
+int64_t fss_tile_rows(int dtype, int backward, int64_t B, int64_t T, int64_t D, int flags);
+
 /* ---- sequence-parallel pieces (no counterpart in the reference, which never splits T) ---- */
 /* Rows per block of the block_prod outputs for this problem and algorithm (> 0). */
 int64_t fss_block_rows(int dtype, int64_t B, int64_t T, int64_t D, int algo);

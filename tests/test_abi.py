@@ -1,7 +1,10 @@
 """CPU-side checks of the boundary: the library loads, exports every symbol the header
 declares, and rejects bad arguments before touching a device."""
 import ctypes
+import os
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -87,6 +90,37 @@ def test_error_strings_and_argument_checks_need_no_device():
     assert L.fss_workspace_bytes(8, 2048, 1024, 0) > 256
     assert L.fss_workspace_bytes(0, 0, 0, 0) >= 256
     assert L.fss_block_rows(0, 1, 65536, 4096, 1) >= 1
+
+
+# dtype, B, T, D of single-pass problems: both sides of 64 MiB a tensor and 384 columns of 64 bytes, wide ones, short ones
+TILE_SHAPES = [("f32", 4, 4096, 2048), ("f32", 4, 2048, 1024), ("f32", 2, 8192, 2560), ("bf16", 16, 2048, 1024), ("bf16", 4, 4096, 2048),
+               ("bf16", 16, 4096, 2560), ("f32", 16, 4096, 2560), ("bf16", 2, 300, 768), ("bf16", 1, 40, 512)]
+
+
+def _tile_rows(forced):
+    """Rows per tile of forward, reversed forward and backward launches, in a process of its own (the switch is read once)."""
+    code = ("import ctypes, sys; L = ctypes.CDLL(sys.argv[1]); L.fss_tile_rows.restype = ctypes.c_int64\n"
+            "for a in sys.argv[2:]:\n"
+            "    dt, B, T, D = a.split(',')\n"
+            "    print(*[L.fss_tile_rows(int(dt == 'f32'), bwd, *map(ctypes.c_int64, (int(B), int(T), int(D))), flags)"
+            " for bwd, flags in ((0, 0), (0, 8), (1, 0), (1, 8))])")
+    from fast_sequential_scan_b200 import _lib
+    env = {k: v for k, v in os.environ.items() if k not in ("FSS_B200_SPLIT", "FSS_B200_TAIL", "FSS_B200_TICKETS")}
+    if forced:
+        env["FSS_B200_SPLIT"] = str(forced)
+    out = subprocess.run([sys.executable, "-c", code, str(_lib.LIB_PATH), *[",".join(map(str, c)) for c in TILE_SHAPES]],
+                         capture_output=True, text=True, check=True, env=env).stdout
+    return [tuple(map(int, line.split())) for line in out.splitlines()]
+
+
+@pytest.mark.parametrize("forced", [1, 2, 4])
+def test_forced_tile_shape_holds_for_every_problem(forced):
+    assert _tile_rows(forced) == [(64 * forced,) * 4] * len(TILE_SHAPES)
+
+
+def test_tile_shapes_chosen_by_default():
+    rows = _tile_rows(None)
+    assert rows == [(128, 128, 256, 256), (256,) * 4, (256,) * 4, (128,) * 4, (256,) * 4, (64,) * 4, (64,) * 4, (128,) * 4, (64,) * 4]
 
 
 def test_package_has_no_fallback_when_library_is_missing(monkeypatch, tmp_path):

@@ -1466,3 +1466,48 @@ def test_large_scans_of_many_narrow_columns(dtype, B, T, D, reverse):
     # (what dh may be off by is multiplied with h)
     scale = 1.0 + torch.cat([torch.zeros_like(sh[:, :1]), sh[:, :-1]], 1).float().abs().cpu()
     assert_parity(sda.float().cpu() / scale, torch.from_numpy(da_ref) / scale, tol, "dalpha")
+
+
+def _worst(x, y, tol, scale=1.0):
+    """max |x - y| / (tol + tol |y|) over all elements, on the GPU, of both divided by ``scale``"""
+    x, y = x.float() / scale, y.float() / scale
+    return float(((x - y).abs() / (tol + tol * y.abs())).max())
+
+
+def _every_channel(dtype, B, T, D, reverse=False):
+    """Single-pass kernels, with entering and returned states, against the chunked kernels, which share no code with them.  Both
+    hold the state in fp32 and round a result once: they differ by one rounding to bf16 (2^-8 of the value; the bound is 1e-2)
+    or by the order of fp32 sums (1e-5)."""
+    pkg, native, _lib = _mods()
+    dt, tol = (torch.float32, F32_TOL) if dtype == "f32" else (torch.bfloat16, BF16_TOL)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    a = torch.rand((B, T, D), generator=gen, device="cuda").mul_(0.5).add_(0.45).to(dt)
+    b, g = (torch.randn((B, T, D), generator=gen, device="cuda").to(dt) for _ in range(2))
+    h0, u0 = (torch.randn((B, D), generator=gen, device="cuda") for _ in range(2))
+
+    def run(algo, saved=None):
+        h, da, db = (torch.full_like(a, float("nan")) for _ in range(3))
+        h_last, u_out = (torch.full_like(h0, float("nan")) for _ in range(2))
+        native.forward_into(a, b, h, algo=algo, continuation=True, h_in=h0, h_last=h_last, reverse=reverse)
+        saved = h if saved is None else saved
+        native.backward_into(a, saved, g, da, db, algo=algo, continuation=True, u_in=u0, h_prev=h0, u_out=u_out, reverse=reverse)
+        pkg.check_status()
+        return h, h_last, da, db, u_out
+
+    ref = run(_lib.ALGO_CHUNKED)
+    got = run(_lib.ALGO_LOOKBACK, ref[0])
+    scale = 1.0 + ref[0].float().abs().roll(-1 if reverse else 1, 1)      # dalpha_t = dh_t * h_{t-1}
+    scale[:, -1 if reverse else 0] = 1.0 + h0.abs()
+    for x, y, t, what in zip(got, ref, (tol, F32_TOL, tol, tol, F32_TOL), ("h", "h_last", "dalpha", "dbeta", "u_out")):
+        worst = _worst(x, y, t, scale if what == "dalpha" else 1.0)
+        assert worst <= 1.0, f"{what}: {worst:.3f} of the bound"
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("dtype, B, T, D, rows", [
+    ("f32", 1, 5000, 56, 64), ("bf16", 3, 5000, 120, 64)])      # one column of full-width tiles, long chains
+def test_carries_in_every_channel(dtype, B, T, D, rows, reverse):
+    """Look-back where the chain of carries is long."""
+    _, _, _lib = _mods()
+    assert _lib.lib().fss_tile_rows(int(dtype == "f32"), 0, B, T, D, _lib.FLAG_REVERSE if reverse else 0) == rows
+    _every_channel(dtype, B, T, D, reverse)

@@ -820,6 +820,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         // 9.5.  More per trip costs the passes more issue slots than it saves: with eight B8 T2048 D1024
         // forward 21.6 -> 23.0, B1 T65536 D4096 274 / 476.
         constexpr int kLooks = kWindow > kSp ? kWindow / kSp : 1;
+        constexpr int kTrip = kLooks * kSp;            // predecessors the warp reads per round trip
         using AggPk = PacketGroup<2 * V, LPG>;         // (P, C) of the tile scanned from zero
         using IncPk = PacketGroup<NI, LPG>;                 // state after the tile (and product up to it)
         constexpr int kTilePackets = (AggPk::kPackets + IncPk::kPackets) * LPG;
@@ -843,6 +844,14 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         };
         first_look();
         const int64_t step = p.ncols * kTilePackets;      // from a tile's descriptors to its predecessor's
+        // One more look at the predecessor once the summary is in, before a whole window is read: where the columns span
+        // more than a wave of CTAs the predecessor is of an earlier wave and has mostly just published.  Forward with /
+        // without: kSp = 1 B16 T4096 D2560 bf16 173 / 178 us, kSp = 2 B1 T7084 D9472 fp32 151 / 154, kSp = 4 B1 T1024 D3584 fp32
+        // 11.8 / 12.0.  From 12 tiles per CTA on it gains nothing at kSp = 4 and loses on large tensors (B1 T10951 D6128 fp32
+        // 149 / 143), and with fewer columns, where the chain of carries is the bound, it is a round trip lost (B1 T65536
+        // D64 bf16 36.3 / 35.9).  Narrow backward scans are indifferent (B4 T4096 D2048 bf16 60.7 / 61.0).
+        const bool look_again =
+            p.ncols >= p.grid && (kSp == 1 || (!kBackward && (kSp == 2 || p.ntiles <= 12 * p.grid)));
 
 #pragma unroll 1
         for (int i = lb;; i += kLookbackWarps) {
@@ -873,10 +882,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 }
             }
             if (!ctl.wait(bar_sum(g), (uint32_t)((i / kGens) & 1), FSS_STATUS_LOOKBACK_TIMEOUT)) break;
-            // One more look now that the summary is in.  With as many columns as kSp = 1 stands for the answer is there by
-            // now more often than not (B16 T4096 D2560 bf16 forward 173 us, 178 without); a window at once saves the others
-            // a round trip.
-            if (kSp == 1 && s > 0 && !hit) {
+            if (look_again && s > 0 && !hit) {
                 typename IncPk::Raw again;
                 IncPk::load_raw(inc_packets(k - p.ncols), again);
                 hit = __all_sync(0xffffffffu, IncPk::decode(again, cur, tag_inc));
@@ -913,34 +919,50 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                 for (;;) {
                     // one round trip: lane group q reads the descriptors of row blocks at - q, at - q - kSp, ...
                     float inc[kLooks][NI], ag[kLooks][2 * V];
+                    bool inc_ok[kLooks], ag_ok[kLooks];
+#pragma unroll
+                    for (int j = 0; j < kLooks; ++j) {
+                        inc_ok[j] = ag_ok[j] = false;
+                        if (at >= j * kSp + q) {
+                            const uint4 *pk = near_packets - (int64_t)(j * kSp + q) * step;
+                            inc_ok[j] = IncPk::load(pk + AggPk::kPackets * LPG, inc[j], tag_inc);
+                            ag_ok[j] = AggPk::load(pk, ag[j], tag_agg);
+                        }
+                    }
+                    auto of = [&](const float &x, int w) {       // what the lane group of window position w has
+                        return kSp > 1 ? __shfl_sync(0xffffffffu, x, (w % kSp) * LPG + cl) : x;
+                    };
+                    // The nearest tile's own state, usually the predecessor's, before anything else is asked: the tiles
+                    // behind wait for it.  Votes follow the loads of all looks, which are not moved over one.  Forward B1
+                    // T65536 D56 fp32 34.8 -> 27.0 us, B1 T1024 D3584 fp32 12.3 -> 11.8 (with the second look), B4 T4096
+                    // D2048 bf16 37.6 -> 36.8.
+                    if (__all_sync(0xffffffffu, q != 0 || inc_ok[0])) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            const float state = of(inc[0][v], 0);
+                            cin[v] = at == s - 1 ? state : fmaf(Pa[v], state, Ca[v]);
+                        }
+                        break;
+                    }
                     uint32_t inc_in[kLooks], ag_in[kLooks];
 #pragma unroll
                     for (int j = 0; j < kLooks; ++j) {
-                        bool inc_ok = false, ag_ok = false;
-                        if (at >= j * kSp + q) {
-                            const uint4 *pk = near_packets - (int64_t)(j * kSp + q) * step;
-                            inc_ok = IncPk::load(pk + AggPk::kPackets * LPG, inc[j], tag_inc);
-                            ag_ok = AggPk::load(pk, ag[j], tag_agg);
-                        }
-                        inc_in[j] = __ballot_sync(0xffffffffu, inc_ok);
-                        ag_in[j] = __ballot_sync(0xffffffffu, ag_ok);
+                        inc_in[j] = __ballot_sync(0xffffffffu, inc_ok[j]);
+                        ag_in[j] = __ballot_sync(0xffffffffu, ag_ok[j]);
                     }
                     // the nearest inclusive state with every aggregate before it in reach, or the state before block 0
                     int from = -1, adv = 0;             // (everything here is warp-uniform)
                     bool more = true;
 #pragma unroll
-                    for (int w = 0; w < kLooks * kSp; ++w) {
+                    for (int w = 0; w < kTrip; ++w) {
                         constexpr uint32_t kGroup = LPG == 32 ? 0xffffffffu : (1u << (LPG % 32)) - 1u;
-                        const bool inc_ok = ((inc_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
-                        const bool ag_ok = ((ag_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
-                        if (more && inc_ok) from = w;
-                        else if (more && ag_ok) adv = w + 1;
-                        if (more && !inc_ok && ag_ok && at == w) from = w + 1;
-                        more = more && !inc_ok && ag_ok && at != w;
+                        const bool has_inc = ((inc_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
+                        const bool has_ag = ((ag_in[w / kSp] >> ((w % kSp) * LPG)) & kGroup) == kGroup;
+                        if (more && has_inc) from = w;
+                        else if (more && has_ag) adv = w + 1;
+                        if (more && !has_inc && has_ag && at == w) from = w + 1;
+                        more = more && !has_inc && has_ag && at != w;
                     }
-                    auto of = [&](const float &x, int w) {       // what the lane group of window position w has
-                        return kSp > 1 ? __shfl_sync(0xffffffffu, x, (w % kSp) * LPG + cl) : x;
-                    };
                     if (from >= 0) {
                         // Carried forward tile by tile, which is how those tiles do it themselves: the bits do not
                         // depend on which of them had got how far.
@@ -957,7 +979,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                             }
                         }
 #pragma unroll
-                        for (int w = kLooks * kSp - 1; w >= 0; --w) {
+                        for (int w = kTrip - 1; w >= 0; --w) {
                             if (w < from) {
 #pragma unroll
                                 for (int v = 0; v < V; ++v)
@@ -970,7 +992,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                     }
                     if (p.deterministic) adv = 0;       // summaries are not folded ahead of the state they carry
 #pragma unroll
-                    for (int w = 0; w < kLooks * kSp; ++w) {
+                    for (int w = 0; w < kTrip; ++w) {
                         if (w < adv) {
 #pragma unroll
                             for (int v = 0; v < V; ++v) {

@@ -1505,9 +1505,13 @@ def _every_channel(dtype, B, T, D, reverse=False):
 
 @pytest.mark.parametrize("reverse", [False, True])
 @pytest.mark.parametrize("dtype, B, T, D, rows", [
-    ("f32", 1, 5000, 56, 64), ("bf16", 3, 5000, 120, 64)])      # one column of full-width tiles, long chains
+    ("f32", 1, 5000, 56, 64), ("bf16", 3, 5000, 120, 64),      # one column of full-width tiles, long chains
+    ("bf16", 1, 1030, 5120, 256), ("f32", 1, 2816, 2560, 256), ("f32", 1, 2817, 2560, 256),      # 160 columns: 5, 11, 12 row blocks
+    ("f32", 1, 1100, 2368, 256), ("f32", 1, 1100, 2352, 256),      # 148 columns, as many as CTAs, and 147
+    ("bf16", 1, 700, 18944, 128), ("f32", 3, 400, 4100, 128), ("f32", 5, 400, 4100, 64)])
 def test_carries_in_every_channel(dtype, B, T, D, rows, reverse):
-    """Look-back where the chain of carries is long."""
+    """Look-back where the chain of carries is long, and on both sides of the lines (columns against CTAs, 12 tiles per
+    CTA) that decide about the second look at the predecessor."""
     _, _, _lib = _mods()
     assert _lib.lib().fss_tile_rows(int(dtype == "f32"), 0, B, T, D, _lib.FLAG_REVERSE if reverse else 0) == rows
     _every_channel(dtype, B, T, D, reverse)

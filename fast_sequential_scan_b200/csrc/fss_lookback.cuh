@@ -815,12 +815,15 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         constexpr int NI = V;                          // floats of an inclusive descriptor
         // Predecessors a lane reads per round trip.  In narrow tiles the lane groups, which hold the same channels, look at
         // different ones: four in one trip at kSp = 4.  With every group at the same two the chain of carries was the
-        // bound of problems with few columns: forward / backward B1 T65536 bf16 D128 29.0 / 30.0 -> 23.7 / 25.2 us, D512 57.0 /
-        // 67.4 -> 47.1 / 64.7, D1024 89.3 / 121.9 -> 78.7 / 120.5, D4096 262 / 415 -> 247 / 414; B2 T1024 D768 7.9 / 9.8 -> 7.6 /
-        // 9.5.  More per trip costs the passes more issue slots than it saves: with eight B8 T2048 D1024
-        // forward 21.6 -> 23.0, B1 T65536 D4096 274 / 476.
+        // bound of problems with few columns: forward / backward B1 T65536 bf16 D128 28.6 / 29.8 -> 22.6 / 24.4 us, D512 57.0 /
+        // 67.4 -> 45.8 / 64.0, D1024 91 / 124 -> 78 / 119, D4096 274 / 423 -> 255 / 417; B2 T1024 D768 7.8 / 9.1 -> 7.4 / 8.6.
+        // More per trip costs the passes more issue slots than it saves: with eight B8 T2048 D1024 forward 21.6 -> 23.0, B1
+        // T65536 D4096 274 / 476.
         constexpr int kLooks = kWindow > kSp ? kWindow / kSp : 1;
         constexpr int kTrip = kLooks * kSp;            // predecessors the warp reads per round trip
+        // Rolled where a lane has one look: unrolled, the loops over a trip made the kernels long enough to cost a gated
+        // forward and backward in turn 2 to 4 % (B4 T512 D2048 bf16 35.5 -> 34.8 us, B4 T700 D1536 fp32 50.6 -> 48.7).
+        constexpr int kUnroll = kLooks > 1 ? kTrip : 1;
         using AggPk = PacketGroup<2 * V, LPG>;         // (P, C) of the tile scanned from zero
         using IncPk = PacketGroup<NI, LPG>;                 // state after the tile (and product up to it)
         constexpr int kTilePackets = (AggPk::kPackets + IncPk::kPackets) * LPG;
@@ -929,6 +932,7 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                             ag_ok[j] = AggPk::load(pk, ag[j], tag_agg);
                         }
                     }
+                    auto look_of = [](int w) { return kLooks > 1 ? w / kSp : 0; };
                     auto of = [&](const float &x, int w) {       // what the lane group of window position w has
                         return kSp > 1 ? __shfl_sync(0xffffffffu, x, (w % kSp) * LPG + cl) : x;
                     };
@@ -972,18 +976,18 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                         if (from <= at) {
 #pragma unroll
                             for (int j = 0; j < kLooks; ++j) {
-                                if (from / kSp == j) {
+                                if (look_of(from) == j) {
 #pragma unroll
                                     for (int v = 0; v < V; ++v) state[v] = of(inc[j][v], from);
                                 }
                             }
                         }
-#pragma unroll
-                        for (int w = kTrip - 1; w >= 0; --w) {
+#pragma unroll (kUnroll)
+                        for (int w = kUnroll > 1 ? kTrip - 1 : from - 1; w >= 0; --w) {
                             if (w < from) {
 #pragma unroll
                                 for (int v = 0; v < V; ++v)
-                                    state[v] = fmaf(of(ag[w / kSp][v], w), state[v], of(ag[w / kSp][V + v], w));
+                                    state[v] = fmaf(of(ag[look_of(w)][v], w), state[v], of(ag[look_of(w)][V + v], w));
                             }
                         }
 #pragma unroll
@@ -991,13 +995,13 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
                         break;
                     }
                     if (p.deterministic) adv = 0;       // summaries are not folded ahead of the state they carry
-#pragma unroll
-                    for (int w = 0; w < kTrip; ++w) {
+#pragma unroll (kUnroll)
+                    for (int w = 0; w < (kUnroll > 1 ? kTrip : adv); ++w) {
                         if (w < adv) {
 #pragma unroll
                             for (int v = 0; v < V; ++v) {
-                                Ca[v] = fmaf(Pa[v], of(ag[w / kSp][V + v], w), Ca[v]);
-                                Pa[v] *= of(ag[w / kSp][v], w);
+                                Ca[v] = fmaf(Pa[v], of(ag[look_of(w)][V + v], w), Ca[v]);
+                                Pa[v] *= of(ag[look_of(w)][v], w);
                             }
                         }
                     }

@@ -57,6 +57,7 @@ class Workspace:
         self.device = device
         self.stream_handle = stream_handle
         self.buf = None
+        self.replaced = []       # smaller buffers of before: CUDA graphs that were captured with them still write there
         self.contexts = {}       # what the library is handed, per (algo, flags); never changed once made (by the caller)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._flag = self.status.numpy()      # same memory, read without going through torch
@@ -69,9 +70,13 @@ class Workspace:
     def ensure(self, nbytes: int) -> None:
         if self.buf is not None and self.buf.numel() >= nbytes:
             return
-        # grow geometrically; a fresh buffer has to be zeroed before its first launch
+        # grow geometrically (all that was replaced is together less than what is in use); a fresh buffer has to be
+        # zeroed before its first launch
         size = max(nbytes, 2 * (self.buf.numel() if self.buf is not None else 0), 1 << 16)
-        self.buf = torch.empty(size, dtype=torch.uint8, device=self.device)
+        buf = torch.empty(size, dtype=torch.uint8, device=self.device)
+        if self.buf is not None:
+            self.replaced.append(self.buf)
+        self.buf = buf
         self.contexts = {}
         _lib.check(_lib.lib().fss_workspace_init(self.buf.data_ptr(), size, self.stream_handle),
                    "fss_workspace_init")
@@ -80,8 +85,8 @@ class Workspace:
         code = int(self._flag[0])
         if code:
             self._flag[0] = 0
-            if self.buf is not None:   # descriptors of the failed launch are not trustworthy
-                _lib.check(_lib.lib().fss_workspace_init(self.buf.data_ptr(), self.buf.numel(),
+            for buf in [*self.replaced, self.buf] if self.buf is not None else []:      # descriptors of the failed launch
+                _lib.check(_lib.lib().fss_workspace_init(buf.data_ptr(), buf.numel(),        # are not trustworthy
                                                          self.stream_handle), "fss_workspace_init")
             raise RuntimeError("fss_b200 kernel reported: " + _lib.STATUS_TEXT.get(code, f"status {code}"))
 

@@ -4,6 +4,7 @@ What has to hold: the context that a native call reads is its own, and a launch 
 the launch before it, so that it can wait for that launch's end (two single-pass grids that overlap on a device can wait
 for one another)."""
 import threading
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -135,3 +136,32 @@ def test_a_call_that_fails_gives_the_device_back(fake, monkeypatch):
     thread = _second_thread(lambda: _scan(fake, 1))
     thread.join(LIMIT)
     assert not thread.is_alive() and fake.log[-1] == ("launch", 1, 0)
+
+
+def test_a_replaced_buffer_outlives_the_graphs_that_may_write_to_it(monkeypatch):
+    """A captured launch keeps the address of its workspace.  Growing replaces the buffer, and must not free the old one."""
+    cleared = []
+
+    def init(address, nbytes, stream):
+        cleared.append((address, nbytes))
+        return 0
+    monkeypatch.setattr(_lib, "lib", lambda: SimpleNamespace(fss_workspace_init=init))
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self: self)
+    monkeypatch.setattr(workspace, "_devices", {})
+    ws = workspace.Workspace(SimpleNamespace(type="cpu", index=0), 1)
+    monkeypatch.setattr(ws, "device", torch.device("cpu"))
+    made = []
+    for nbytes in (1000, 1 << 16, (1 << 16) + 1, 1 << 20, 5000, 1 << 21):
+        if ws.buf is None or ws.buf.numel() < nbytes:
+            ws.ensure(nbytes)
+            made.append(weakref.ref(ws.buf))
+    buffers = [ref() for ref in made]
+    assert len(buffers) == 4 and all(t is not None for t in buffers)
+    assert sum(t.numel() for t in buffers[:-1]) < buffers[-1].numel()
+    assert cleared == [(t.data_ptr(), t.numel()) for t in buffers]
+    # a launch that reported a failure may have been any of theirs: all are cleared
+    cleared.clear()
+    ws._flag[0] = 1
+    with pytest.raises(RuntimeError):
+        ws.raise_if_flagged()
+    assert sorted(cleared) == sorted((t.data_ptr(), t.numel()) for t in buffers)

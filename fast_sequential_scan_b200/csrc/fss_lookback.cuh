@@ -852,9 +852,11 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         // without: kSp = 1 B16 T4096 D2560 bf16 173 / 178 us, kSp = 2 B1 T7084 D9472 fp32 151 / 154, kSp = 4 B1 T1024 D3584 fp32
         // 11.8 / 12.0.  From 12 tiles per CTA on it gains nothing at kSp = 4 and loses on large tensors (B1 T10951 D6128 fp32
         // 149 / 143), and with fewer columns, where the chain of carries is the bound, it is a round trip lost (B1 T65536
-        // D64 bf16 36.3 / 35.9).  Narrow backward scans are indifferent (B4 T4096 D2048 bf16 60.7 / 61.0).
-        const bool look_again =
-            p.ncols >= p.grid && (kSp == 1 || (!kBackward && (kSp == 2 || p.ntiles <= 12 * p.grid)));
+        // D64 bf16 36.3 / 35.9).  Narrow backward scans are indifferent (B4 T4096 D2048 bf16 60.7 / 61.0).  Narrow gated scans
+        // go without its instructions, which cost a forward and a backward that take turns more than it gave (B4 T512
+        // D2048 bf16 34.4 -> 34.0 us, B4 T700 D1536 fp32 49.2 -> 48.6).
+        constexpr bool kMayLookAgain = kSp == 1 || !(kBackward || kGate);
+        const bool look_again = kMayLookAgain && p.ncols >= p.grid && (kSp < 4 || p.ntiles <= 12 * p.grid);
 
 #pragma unroll 1
         for (int i = lb;; i += kLookbackWarps) {

@@ -1515,3 +1515,44 @@ def test_carries_in_every_channel(dtype, B, T, D, rows, reverse):
     _, _, _lib = _mods()
     assert _lib.lib().fss_tile_rows(int(dtype == "f32"), 0, B, T, D, _lib.FLAG_REVERSE if reverse else 0) == rows
     _every_channel(dtype, B, T, D, reverse)
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("dtype, B, T, D, rows", [
+    ("f32", 1, 6000, 56, 64), ("bf16", 2, 4000, 120, 64), ("f32", 5, 400, 4100, 64),      # full-width tiles, two looks per lane
+    ("bf16", 1, 500, 18944, 128), ("f32", 3, 400, 4100, 128),      # lane groups of 16, short sequences
+    ("f32", 3, 2731, 2064, 128),      # the same in many row blocks (forward; the last column of 128 bytes half there)
+    ("f32", 1, 9000, 256, 256), ("bf16", 2, 3000, 1032, 256)])      # lane groups of 8
+def test_deterministic_bits_in_every_tile_shape(dtype, B, T, D, rows, reverse):
+    """FSS_FLAG_DETERMINISTIC: a tile starts from whichever final state of its window is published, carried forward through
+    the summaries between as the tiles between do it, so which one it was cannot be told from the bits."""
+    pkg, native, _lib = _mods()
+    assert _lib.lib().fss_tile_rows(int(dtype == "f32"), 0, B, T, D, _lib.FLAG_REVERSE if reverse else 0) == rows
+    dt = torch.float32 if dtype == "f32" else torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    a = torch.rand((B, T, D), generator=gen, device="cuda").mul_(0.099).add_(0.9).to(dt)       # a state is felt many rows later
+    b, g = (torch.randn((B, T, D), generator=gen, device="cuda").to(dt) for _ in range(2))
+    previous = native.set_deterministic(True)
+    try:
+        first = None
+        for it in range(10):
+            outs = [torch.full_like(a, float("nan")) for _ in range(3)]
+            native.forward_into(a, b, outs[0], algo=_lib.ALGO_LOOKBACK, reverse=reverse)
+            native.backward_into(a, outs[0], g, outs[1], outs[2], algo=_lib.ALGO_LOOKBACK, reverse=reverse)
+            first = first or outs
+            for x, y, what in zip(outs, first, ("h", "dalpha", "dbeta")):
+                assert torch.equal(x, y), f"launch {it}: {what} differs from launch 0"
+        pkg.check_status()
+    finally:
+        native.set_deterministic(previous)
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("dtype, B, T, D, rows", [
+    ("f32", 3, 2731, 2064, 128), ("bf16", 12, 2731, 1032, 128), ("f32", 3, 2729, 2048, 256), ("f32", 2, 3200, 2624, 256)])
+def test_large_scans_in_every_channel(dtype, B, T, D, rows, reverse):
+    """Both sides of the line (64 MiB a tensor, 384 columns of 64 bytes) from which tiles are 128 rows x 128 bytes, the last
+    column half there, with entering and returned states."""
+    _, _, _lib = _mods()
+    assert _lib.lib().fss_tile_rows(int(dtype == "f32"), 0, B, T, D, _lib.FLAG_REVERSE if reverse else 0) == rows
+    _every_channel(dtype, B, T, D, reverse)

@@ -815,8 +815,8 @@ scan_kernel(const __grid_constant__ Maps<Kind<kBackward, kGate>::kIn, Kind<kBack
         constexpr int NI = V;                          // floats of an inclusive descriptor
         // Predecessors a lane reads per round trip.  In narrow tiles the lane groups, which hold the same channels, look at
         // different ones: four in one trip at kSp = 4.  With every group at the same two the chain of carries was the
-        // bound of problems with few columns: forward / backward B1 T65536 bf16 D128 28.6 / 29.8 -> 22.6 / 24.4 us, D512 57.0 /
-        // 67.4 -> 45.8 / 64.0, D1024 91 / 124 -> 78 / 119, D4096 274 / 423 -> 255 / 417; B2 T1024 D768 7.8 / 9.1 -> 7.4 / 8.6.
+        // bound of problems with few columns: forward / backward B1 T65536 bf16 D128 28.8 / 29.9 -> 22.9 / 24.7 us, D512 57.5 /
+        // 67.2 -> 46.4 / 64.5, D1024 91 / 124 -> 78 / 119, D4096 274 / 423 -> 255 / 417; B2 T1024 D768 7.8 / 9.1 -> 7.4 / 8.6.
         // More per trip costs the passes more issue slots than it saves: with eight B8 T2048 D1024 forward 21.6 -> 23.0, B1
         // T65536 D4096 274 / 476.
         constexpr int kLooks = kWindow > kSp ? kWindow / kSp : 1;
@@ -1501,12 +1501,19 @@ inline int launch_tail(int dtype, bool backward, bool gated, bool reverse, int64
 // Tile shape of a plain scan whose row blocks no caller asks for.  From 384 of the narrowest columns on (a wave of CTAs takes
 // 148) a row block's columns span several waves, nothing holds the CTAs together any more, and in the fixed order the
 // ones that the memory system serves slowly finish late (the CTAs of B4 T4096 D2048 fp32 ended between 59 and 72 us).  Large
-// tensors make that dearer than the second halving of the columns is worth: 128 rows x 128 bytes against 256 x 64,
-// forward: 64 MiB a tensor 37.1 -> 35.8 us (B4 T2048 D2048 fp32) and 39.4 -> 37.8 (B16 T2048 D1024 bf16), 128 MiB 76.8 -> 67.4 and
-// 81.6 -> 70.2 (twice the rows), 176 MiB 105 -> 90 (B3 T6000 D2560 fp32), 256 MiB 195 -> 138 (B32 T8192 D512
-// bf16).  Below 64 MiB or 384 columns it is the other way round: 31 MiB 20.3 / 20.2, B16 T512 D1024 bf16 13.1 / 13.8, 320
-// columns 79.4 / 81.0 (B2 T8192 D2560 fp32).  The backward gains 2 to 3 % in the fixed order (61.1 -> 59.8) and loses as much with
-// tickets, which balance the CTAs themselves (105 / 107).
+// tensors make that dearer than the second halving of the columns is worth.  Forward, 128 rows x 128 bytes against
+// 256 x 64, in per cent (fp32 / bf16; columns of 64 bytes down, MiB a tensor across; a spread of 1 to 2):
+//               32           48           64           96          128          256          512         1024
+//   160   +4.4 / +9.0  +2.7 / +5.6  +4.5 / +7.7  +3.6 / +5.8  +3.7 / +5.4  +2.2 / +6.0  +1.7 / +6.5  +1.0 / +8.0
+//   256   +2.7 / +3.9  +3.1 / +4.4  +1.4 / +4.4  +1.8 / +3.7  +3.1 / +3.3  +0.9 / +3.4  -0.9 / +4.6  -7.8 / +0.6
+//   320   -1.1 / -0.9  +0.7 / +4.3  +0.8 / +2.9  +0.0 / +1.5  +0.0 / +2.4  -0.5 / +1.8  -3.5 / +0.5  -4.8 / -3.3
+//   352   -0.3 / +2.6  +0.1 / +3.1  +0.5 / +2.5  -1.9 / +1.2  -1.9 / +0.6  -1.4 / -0.1  -6.4 / -3.9  -9.3 / -9.9
+//   384   -4.3 / -3.9  -0.2 / +2.0  -1.1 / +0.5  -2.9 / -2.0  -2.9 / -0.2  -8.0 / -0.9  -4.9 / -4.4  -8.0 / -8.1
+//   448   -1.7 / -1.4  -2.1 / -0.1  -6.2 / -5.5  -2.8 / -2.4  -6.2 / -4.7  -18 / -13    -8.2 / -7.3  -6.4 / -7.9
+//   512   -1.2 / +1.1  -2.2 / -1.0  -2.7 / -1.7  -4.4 / -2.7  -7.8 / -4.5  -13 / -14    -7.0 / -6.2  -9.4 / -7.5
+// Nothing inside 64 MiB and 384 columns is slower by more than the spread.  Outside, below 64 MiB the shapes are mostly level, and
+// from 512 MiB on 128 x 128 would pay from 320 or 352 columns on (fp32: from 256 at 1 GiB).  The backward gains 2 % in the
+// fixed order (B4 T2048 D2048 fp32 61.9 -> 60.0 us) and loses as much with tickets, which balance the CTAs themselves (105 / 107).
 inline int choose_split_freely(int dtype, int64_t B, int64_t T, int64_t D, bool tickets) {
     const int s = choose_split(dtype, B, T, D);
     const int64_t esize = dtype == FSS_DTYPE_BF16 ? 2 : 4;
